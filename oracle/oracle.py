@@ -22,8 +22,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 REF_LIB = os.path.join(HERE, "_ref", "libref_oracle.so")
 ADAPTER_CHECK = os.path.join(HERE, "_ref", "adapter_check")
 ORC_LIB = os.path.join(HERE, "libdipl_oracle.so")
-# where the reference tree is compiled from (the reference harness is built only where it exists)
+# where the reference tree is compiled from: "" where there is none, or an empty folder in its place (the reference
+# harness and the adapter are built only where the sources are)
 REFERENCE_TREE = os.environ.get("DIPL_REFERENCE_TREE", "/root/reference")
+if not os.path.isfile(os.path.join(REFERENCE_TREE, "src", "acceleration", "sbvh.cc")):
+    REFERENCE_TREE = ""
 
 _f32p = np.ctypeslib.ndpointer(np.float32, flags="C_CONTIGUOUS")
 _f64p = np.ctypeslib.ndpointer(np.float64, flags="C_CONTIGUOUS")
