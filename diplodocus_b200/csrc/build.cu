@@ -1817,6 +1817,168 @@ __global__ void node_write_kernel(LayoutParams P, const float4* __restrict__ tbo
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// 4-wide nodes of the traversal: one for every binary inner node f, at the same index, holding what lies two levels
+// below f. Every binary node gets one, so no traversal of the tree is needed to choose and number the ones a ray can
+// reach (about half of them), a reference means the same node in both layouts, and the kernel is one pass over the
+// finished BNodes: bound by the gathers of the two children's 64-byte records (reached nodes are L2 hits, the
+// numbering keeps children near each other).
+//
+// Children: both children of f, each replaced by its own two if it is an inner node; slots still free (a child was
+// a leaf) are filled by opening the child of largest area again, an inner node into its children or a leaf of several
+// triangles into two ranges of them, so that fewer triangles are tested. A ray going down passes at least two binary
+// levels per node unless it reaches a leaf, which bounds the traversal stack by 3 entries per two levels.
+// ------------------------------------------------------------------------------------------------
+struct QChild {
+    float3 lo, hi;
+    int ref;
+};
+
+__device__ __forceinline__ float half_area(const QChild& c) {
+    const float dx = c.hi.x - c.lo.x, dy = c.hi.y - c.lo.y, dz = c.hi.z - c.lo.z;
+    return dx * dy + dy * dz + dz * dx;
+}
+
+__device__ __forceinline__ void bnode_children(const BNode* __restrict__ nodes, int f, QChild& l, QChild& r) {
+    const float4* p = reinterpret_cast<const float4*>(nodes + f);
+    const float4 a = p[0], b = p[1], c = p[2];
+    const int4 d = *reinterpret_cast<const int4*>(p + 3);
+    l.lo = make_float3(a.x, a.z, c.x), l.hi = make_float3(a.y, a.w, c.y), l.ref = d.x;
+    r.lo = make_float3(b.x, b.z, c.z), r.hi = make_float3(b.y, b.w, c.w), r.ref = d.y;
+}
+
+// The leaf's triangles [first, first + count) as one child: their padded box within the leaf's box (a pre-split
+// reference's box holds the part of its triangle that the leaf stands for).
+__device__ __forceinline__ QChild leaf_part(const float4* __restrict__ tris, const QChild& leaf, int first, int count) {
+    const float inf = __int_as_float(0x7F800000);
+    QChild c;
+    c.lo = make_float3(inf, inf, inf), c.hi = make_float3(-inf, -inf, -inf);
+    for (int k = first; k < first + count; ++k) {
+        const float4 a = tris[3 * (long long)k], b = tris[3 * (long long)k + 1], d = tris[3 * (long long)k + 2];
+        const Tri t{make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z), make_float3(d.x, d.y, d.z)};
+        float3 lo, hi;
+        tri_box(t, lo, hi);
+        c.lo = make_float3(fminf(c.lo.x, lo.x), fminf(c.lo.y, lo.y), fminf(c.lo.z, lo.z));
+        c.hi = make_float3(fmaxf(c.hi.x, hi.x), fmaxf(c.hi.y, hi.y), fmaxf(c.hi.z, hi.z));
+    }
+    const float3 lo = c.lo, hi = c.hi;
+    c.lo = make_float3(fmaxf(pad_down(lo.x, hi.x), leaf.lo.x), fmaxf(pad_down(lo.y, hi.y), leaf.lo.y),
+                       fmaxf(pad_down(lo.z, hi.z), leaf.lo.z));
+    c.hi = make_float3(fminf(pad_up(lo.x, hi.x), leaf.hi.x), fminf(pad_up(lo.y, hi.y), leaf.hi.y),
+                       fminf(pad_up(lo.z, hi.z), leaf.hi.z));
+    c.ref = lo.x <= hi.x ? make_leaf_ref(first, count) : make_leaf_ref(0, 0);  // no finite triangle: never hit
+    return c;
+}
+
+// Frame and bytes of one axis. The bytes are chosen in FP64, where the distance of a plane from p in steps is off by
+// less than 2^-36 of a step (the boxes are padded by far more): every child's interval lies within its planes.
+__device__ __forceinline__ void quad_axis(const float* lo, const float* hi, uint32_t valid, float& p, uint32_t& ebias,
+                                          uint32_t& qlo, uint32_t& qhi) {
+    float mn = __int_as_float(0x7F800000), mx = __int_as_float(0xFF800000);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if ((valid >> k) & 1u) mn = fminf(mn, lo[k]), mx = fmaxf(mx, hi[k]);
+    // the first scale to try: the least 2^e with 254 steps over the extent (p is rounded down by up to one)
+    const float step = __fdiv_ru(__fsub_ru(mx, mn), 254.0f);
+    uint32_t eb = min(max(__float_as_uint(step) >> 23, 1u) + 1u, 238u);
+    if (eb > 1u && __uint_as_float((eb - 1u) << 23) >= step) --eb;
+    for (;; ++eb) {
+        const double s = (double)__uint_as_float(eb << 23), inv = 1.0 / s;
+        p = __double2float_rd((double)mn - 32768.0 * s);
+        qlo = qhi = 0u;
+        bool ok = true;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (!((valid >> k) & 1u)) {
+                qlo |= 255u << (8 * k);
+                continue;
+            }
+            const double a = floor(((double)lo[k] - (double)p) * inv) - 32768.0;
+            const double b = ceil(((double)hi[k] - (double)p) * inv) - 32768.0;
+            ok = ok && a >= 0.0 && b <= 255.0;
+            qlo |= (uint32_t)fmin(fmax(a, 0.0), 255.0) << (8 * k);
+            qhi |= (uint32_t)fmin(fmax(b, 0.0), 255.0) << (8 * k);
+        }
+        if (ok || eb >= 238u) break;
+    }
+    ebias = eb;
+}
+
+__global__ void __launch_bounds__(128) quad_write_kernel(const BNode* __restrict__ nodes,
+                                                         const float4* __restrict__ tris,
+                                                         const uint32_t* __restrict__ num_inner,
+                                                         QNode* __restrict__ quads, const uint32_t* err) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= (int)*num_inner || *err != 0u) return;
+    QChild c[4];
+    const int none = make_leaf_ref(0, 0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k].lo = c[k].hi = make_float3(0.f, 0.f, 0.f), c[k].ref = none;
+    {
+        QChild l, r;
+        bnode_children(nodes, f, l, r);
+        c[0] = l, c[2] = r;
+        if (l.ref >= 0) bnode_children(nodes, l.ref, c[0], c[1]);
+        if (r.ref >= 0) bnode_children(nodes, r.ref, c[2], c[3]);
+    }
+    for (int round = 0; round < 2; ++round) {
+        int free_k = -1, best = -1;
+        float area = -1.0f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (c[k].ref == none) {
+                free_k = k;
+            } else if (c[k].ref >= 0 || leaf_count(c[k].ref) > 1) {
+                const float a = half_area(c[k]);
+                if (a > area) area = a, best = k;
+            }
+        }
+        if (free_k < 0 || best < 0) break;
+        QChild x = c[0], l, r;
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+            if (k == best) x = c[k];
+        if (x.ref >= 0) {
+            bnode_children(nodes, x.ref, l, r);
+        } else {
+            const int first = leaf_first(x.ref), cnt = leaf_count(x.ref), n0 = cnt >> 1;
+            l = leaf_part(tris, x, first, n0);
+            r = leaf_part(tris, x, first + n0, cnt - n0);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k == best) c[k] = l;
+            if (k == free_k) c[k] = r;
+        }
+    }
+    uint32_t valid = 0u;
+    float lo[3][4], hi[3][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        lo[0][k] = c[k].lo.x, lo[1][k] = c[k].lo.y, lo[2][k] = c[k].lo.z;
+        hi[0][k] = c[k].hi.x, hi[1][k] = c[k].hi.y, hi[2][k] = c[k].hi.z;
+        // a box of triangles that can never be hit is empty (its padded planes are NaN): no child
+        const bool box = lo[0][k] <= hi[0][k] && lo[1][k] <= hi[1][k] && lo[2][k] <= hi[2][k];
+        if (c[k].ref != none && box) valid |= 1u << k;
+    }
+    QNode q;
+    q.pad[0] = q.pad[1] = 0u;
+    if (valid == 0u) {
+        q.px = q.py = q.pz = 0.0f;
+        q.exps = 0x010101u;
+        q.qlox = q.qloy = q.qloz = 0xFFFFFFFFu, q.qhix = q.qhiy = q.qhiz = 0u;
+    } else {
+        uint32_t ex, ey, ez;
+        quad_axis(lo[0], hi[0], valid, q.px, ex, q.qlox, q.qhix);
+        quad_axis(lo[1], hi[1], valid, q.py, ey, q.qloy, q.qhiy);
+        quad_axis(lo[2], hi[2], valid, q.pz, ez, q.qloz, q.qhiz);
+        q.exps = ex | (ey << 8) | (ez << 16);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q.ref[k] = ((valid >> k) & 1u) ? c[k].ref : none;
+    quads[f] = q;
+}
+
 // Roots of every mesh: the final clusters (one per mesh, in mesh order).
 struct RootInfo {
     int root_ref;
@@ -2044,6 +2206,7 @@ struct BuildPlan {
     int* slot_pos = nullptr;  // pre-split SOBB builds: per slot of the leaf triangle array, its sorted position
     unsigned char* scan_scratch = nullptr;
     BNode* nodes = nullptr;
+    QNode* quads = nullptr;  // binary AABB layout only
     float4* tris = nullptr;
     double* d_sah = nullptr;
     RootInfo* d_roots = nullptr;
@@ -2202,6 +2365,9 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
         (st = W.alloc(&P.d_counts, 4)) != DIPL_OK || (st = O.alloc(&P.nodes, Kalloc)) != DIPL_OK ||
         (st = O.alloc(&P.tris, 3 * N)) != DIPL_OK || (st = W.alloc(&P.d_sah, 2 * m)) != DIPL_OK ||
         (st = W.alloc(&P.d_roots, m)) != DIPL_OK)
+        return st;
+    if (d0.bv_type == DIPL_BV_AABB && d0.layout == DIPL_LAYOUT_BINARY &&
+        (st = O.alloc(&P.quads, Kalloc)) != DIPL_OK)
         return st;
     if (d0.bv_type == DIPL_BV_SOBB) {
         if ((st = sobb_prepare(N, K, W, O, &P.sobb, &P.snodes)) != DIPL_OK) return st;
@@ -2385,6 +2551,10 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
         node_write_kernel<<<blocks_for(K, 256), 256, 0, stream>>>(LP, P.tbox, P.d_coffsets, m, P.perm, P.rev_flags,
                                                                    P.leaf_start_of, P.nodes, P.d_sah, P.d_err);
         note_launches();
+        if (P.quads) {
+            quad_write_kernel<<<blocks_for(K, 128), 128, 0, stream>>>(P.nodes, P.tris, P.d_counts, P.quads, P.d_err);
+            note_launches();
+        }
     }
     roots_kernel<<<blocks_for(m, 64), 64, 0, stream>>>(LP, P.c_lo[0], P.c_hi[0], P.c_lo[1], P.c_hi[1], P.d_ctrl, m,
                                                        P.rev_flags, P.leaf_start_of, P.d_roots, P.d_err);
@@ -2462,6 +2632,7 @@ static dipl_status plan_finish(BuildPlan& P, dipl_bvh** out, bool allow_wide) {
     for (int i = 0; i < P.count; ++i) {
         dipl_bvh* h = make_handle(i);
         h->nodes = d0.bv_type == DIPL_BV_SOBB ? static_cast<void*>(P.snodes) : static_cast<void*>(P.nodes);
+        h->quads = P.quads;
         h->tris = P.tris;
         h->perm = reinterpret_cast<int32_t*>(P.perm);
         h->children = P.child;

@@ -46,6 +46,20 @@ struct __align__(16) BNode {
 };
 static_assert(sizeof(BNode) == 64, "BNode must be 64 bytes");
 
+// 4-wide traversal node (64 bytes, two 32-byte loads): a binary inner node's grandchildren, their boxes in 8-bit
+// steps of a frame of their own. Plane q of axis a lies at p[a] + (32768 + q) * 2^(e[a] - 127): the offset makes
+// "32768 + q" a float whose bits are the byte q shifted by 8 under a constant exponent, so the traversal decodes a
+// byte with one byte permute and no integer-to-float conversion. An unused slot has planes in the wrong order
+// (255 .. 0) and a leaf reference of no triangles.
+struct __align__(64) QNode {
+    float px, py, pz;
+    uint32_t exps;          // biased exponents: x | y << 8 | z << 16
+    int ref[4];             // as in BNode: >= 0 the binary inner node of that index (and its QNode), < 0 a leaf range
+    uint32_t qlox, qhix, qloy, qhiy, qloz, qhiz;  // byte k: child k
+    uint32_t pad[2];
+};
+static_assert(sizeof(QNode) == 64, "QNode must be 64 bytes");
+
 // Binary SOBB node (64 bytes): per child three slab directions (indices into the direction table)
 // and the slab intervals along them.
 struct __align__(16) SNode {

@@ -118,6 +118,7 @@ struct dipl_bvh {
     // traced arrays (device)
     void* nodes = nullptr;      // BNode / SNode / WNode
     int64_t node_size = 64;     // bytes per node of the traced layout
+    dipl::QNode* quads = nullptr;  // binary AABB layout: the 4-wide node of every binary node, same indices
     float4* tris = nullptr;     // 3 float4 per triangle in leaf order (v0.w = primitive id bits)
     // clustering result (device), for downloads
     int32_t* perm = nullptr;    // triangle id per sorted position (of this mesh, local ids)
