@@ -1320,28 +1320,41 @@ __global__ void __launch_bounds__(kTailThreads) ploc_tail_kernel(PlocParams P) {
 // (keys[s] ^ keys[s+1], s ^ (s+1), s), lexicographic; a node [l, r] joins the neighbour across the split with the
 // smaller key (split r if l is its mesh's first position or r is not its mesh's last and key(r) < key(l-1), else
 // split l-1). Mesh bits above the code make every split between meshes larger than any split inside one, so a
-// mesh is a subtree. One thread starts at each leaf; at a split, the first child to arrive leaves its far boundary
+// mesh is a subtree. A thread climbs from each leaf; at a split, the first child to arrive leaves its far boundary
 // (atomic exchange) and stops, the second goes on with the union.
 //
 // Each node holds a list of clusters in position order, stored at its first position: a node of at most T
 // positions (T = kHplocThreshold) is its leaves, untouched; a larger one is processed by the whole warp of the
 // thread that reached it: the left child's list then the right child's, one cluster per lane, and PLOC
-// iterations (nearest neighbour by the key of ploc_kernel over list indices within the radius, by warp shuffles;
-// mutual pairs merge into the lower index; ballot compaction) until at most T clusters are left, or one at a
+// iterations (nearest neighbour by the key of ploc_kernel over list indices within the radius; mutual pairs merge
+// into the lower index; compaction) until at most T clusters are left, or one at a
 // mesh's root. Node ids are deterministic: split s of mesh k owns id N + s - k; a list of c clusters carries
 // c - 1 ids not yet used, a node's pool is the left list's unused ids, its own split's id, the right list's;
 // merges take ids from the front of the pool (iteration, then position order) and the rest go up with the list.
 // oracle/dipl_oracle.c orc_hploc restates the whole procedure sequentially.
+//
+// What bounds it: the latency of one warp's chain of node iterations (0.28 iterations a leaf on the pre-split 16M
+// soup; the last ones, up to the root, run alone) and issue slots; DRAM is at a few percent. So an iteration reads its
+// candidates from the warp's copy of the list in shared memory (two loads a candidate at constant offsets, four gaps
+// in flight, no bounds tests: what lies past the list is a box of infinite extent) and compacts through it: 2200
+// cycles against 5200 with every box word, partner record and compaction by shuffles. And a block first builds the
+// nodes that lie within its own 512 positions with lists, arrivals and fences in shared memory (three in five nodes,
+// and nearly all arrivals), lanes taking the next leaf as soon as they stop, so that only the nodes across block
+// borders go through L2; it gathers the leaf boxes itself. Pre-split 16M soup (20.3M leaves): 14.2 ms with the gather
+// kernel before -> 7.4 ms; 1M sphere 0.76 -> 0.43 ms; 3,978 triangles 155 -> 85 us. On the way: iterations through
+// shared memory 10.9 ms at 128 leaves and threads a block; lanes refilled, 512 leaves on 128 threads 8.3 ms; one-word
+// list records, so that 6 blocks share an SM instead of 4, 7.4 ms (256 leaves 8.8, 512 on 256 threads 8.6 ms).
 // ------------------------------------------------------------------------------------------------
 constexpr int kHplocThreshold = 16;
-constexpr int kHplocThreads = 256;
 constexpr int kHplocMaxSteps = 192;  // tree levels: key bits (<= 64) + index bits (<= 32), with room to spare
 
 struct HplocParams {
     const void* keys;           // sorted keys (uint32 or uint64)
+    const uint32_t* perm;       // reference or triangle at each sorted position
+    const float4* tbox;         // its box: two float4
     const long long* offsets;   // first sorted position of each mesh (+ the total)
     float4* lo;                 // cluster records by sorted position: min xyz, node id bits
-    float4* hi;                 //                                     max xyz, mesh index bits
+    float4* hi;                 //                                     max xyz
     int4* info;                 //                                     triangle count, first position, height, 0
     int4* child;                // internal node k: left, right, height, 0
     float4* node_lo;            // internal node k: min xyz, triangle count bits
@@ -1367,33 +1380,59 @@ __device__ __forceinline__ int atomic_exch_acq_rel(int* p, int v) {
     return old;
 }
 
-template <typename K>
-__device__ __forceinline__ bool split_before(const K* __restrict__ keys, int a, int b) {
-    const K xa = __ldg(keys + a) ^ __ldg(keys + a + 1), xb = __ldg(keys + b) ^ __ldg(keys + b + 1);
-    if (xa != xb) return xa < xb;
-    const unsigned ia = (unsigned)a ^ (unsigned)(a + 1), ib = (unsigned)b ^ (unsigned)(b + 1);
-    if (ia != ib) return ia < ib;
-    return a < b;
+// The value of the lane `by` below, or `none` where there is none.
+__device__ __forceinline__ float shfl_up_or(float v, int by, float none) {
+    float r;
+    asm volatile("{\n\t.reg .pred p;\n\tshfl.sync.up.b32 %0|p, %1, %2, 0, 0xffffffff;\n\tselp.f32 %0, %0, %3, p;\n\t}"
+                 : "=f"(r)
+                 : "f"(v), "r"(by), "f"(none));
+    return r;
 }
 
-__device__ __forceinline__ float4 shfl4(float4 v, int src) {
-    return make_float4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
-                       __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
+// The lists of a block's own nodes, by position - first position of the block. What a list needs of a cluster besides
+// its box and id fits one word while the cluster lies within the block: triangles (10 bits), first position - the
+// block's (9), height (9); ids and positions relative to the block fit 16 bits. 51 bytes a leaf with 64-bit keys.
+template <typename K, int LEAVES>
+struct HplocBlock {
+    static_assert(LEAVES <= 512, "fields relative to the block");
+    float4 lo[LEAVES];              // min xyz, node id
+    float4 hi[LEAVES];              // max xyz, triangles | (first position - b0) << 10 | height << 19
+    K delta[LEAVES + 1];            // keys[p] ^ keys[p + 1] of splits p = first position - 1 + index
+    int other[LEAVES];
+    unsigned exits[LEAVES];         // per warp: the nodes whose parents reach beyond the block (both ends relative)
+    unsigned mine[LEAVES / 32];     // bit per split: its node lies within the block
+    int edge[2][LEAVES / 32];
+    unsigned short fid[LEAVES];     // unused node ids - the id of the block's first split
+    unsigned char cnt[LEAVES];
+};
+__device__ __forceinline__ int4 unpack_info(float w, int b0) {
+    const unsigned v = __float_as_uint(w);
+    return make_int4((int)(v & 1023u), b0 + (int)((v >> 10) & 511u), (int)(v >> 19), 0);
 }
-__device__ __forceinline__ int4 shfl4(int4 v, int src) {
-    return make_int4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
-                     __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
+__device__ __forceinline__ float pack_info(const int4& i, int b0) {
+    return __uint_as_float((unsigned)i.x | ((unsigned)(i.y - b0) << 10) | ((unsigned)i.z << 19));
 }
 
-// One node [nl, nr] with split nm, processed by the whole warp (every lane calls this with the same arguments).
-// Returns the PLOC iterations it ran.
-__device__ __forceinline__ int hploc_node(const HplocParams& P, int nl, int nr, int nm, int id_base, bool whole) {
+// A warp's clusters while it processes a node. The entries past the last cluster are boxes of infinite extent: every
+// distance to them is +inf, so the search needs no bounds.
+struct HplocWarp {
+    float4 box[64];   // lo.xyz, hi.x
+    float2 yz[64];    // hi.y, hi.z
+    int4 rec[32];          // node id, triangle count, first position, height
+};
+
+// One node [nl, nr] with split nm, processed by the whole warp (every lane calls this with the same arguments); `own`:
+// its lists are the block's, `b0` the block's first position. Returns the PLOC iterations it ran.
+template <typename K, int LEAVES>
+__device__ __forceinline__ int hploc_node(const HplocParams& P, HplocBlock<K, LEAVES>& S, HplocWarp& W, int b0, bool own, int nl, int nr, int nm,
+                                          int id_base, bool whole) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int T = kHplocThreshold;
     const int lsize = nm - nl + 1, rsize = nr - nm;
-    int cl = lsize > T ? __ldcg(P.cnt + nl) : lsize;
-    int cr = rsize > T ? __ldcg(P.cnt + nm + 1) : rsize;
+    int cl = lsize, cr = rsize;
+    if (lsize > T) cl = own ? S.cnt[nl - b0] : __ldcg(P.cnt + nl);
+    if (rsize > T) cr = own ? S.cnt[nm + 1 - b0] : __ldcg(P.cnt + nm + 1);
     if (cl < 1 || cl > T || cr < 1 || cr > T) {  // a processed child left 1..T clusters; never read past a list
         if (lane == 0) atomicOr(P.err, kErrIterations);
         cl = min(max(cl, 1), min(lsize, T));
@@ -1404,146 +1443,328 @@ __device__ __forceinline__ int hploc_node(const HplocParams& P, int nl, int nr, 
     const int p = lane < cl ? nl + lane : nm + 1 + (lane - cl);
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
     int4 inf = make_int4(0, 0, 0, 0);
-    if (have) {
-        a = __ldcg(P.lo + p);
-        b = __ldcg(P.hi + p);
-        inf = __ldcg(P.info + p);
-    }
-    int pool = -1;  // lane q holds the pool's entry q (c - 1 entries)
-    if (lane < cl - 1) pool = lsize > T ? __ldcg(P.fid + nl + lane) : id_base + nl + lane;
-    else if (lane == cl - 1) pool = id_base + nm;
-    else if (lane < c - 1) {
-        const int j = lane - cl;
-        pool = rsize > T ? __ldcg(P.fid + nm + 1 + j) : id_base + nm + 1 + j;
+    int pool = -1;  // lane q holds the pool's entry q (c - 1 entries): by default its position's split
+    if (lane < c - 1) pool = id_base + (lane == cl - 1 ? nm : p);
+    const bool listed = (lane < cl - 1 && lsize > T) || (lane >= cl && lane < c - 1 && rsize > T);
+    if (own) {
+        if (have) a = S.lo[p - b0], b = S.hi[p - b0], inf = unpack_info(b.w, b0);
+        if (listed) pool = id_base + b0 + S.fid[p - b0];
+    } else {
+        if (have) a = __ldcg(P.lo + p), b = __ldcg(P.hi + p), inf = __ldcg(P.info + p);
+        if (listed) pool = __ldcg(P.fid + p);
     }
     const int target = whole ? 1 : T;
     const int R = min(P.radius, 31);
+    const float inf_f = __int_as_float(0x7F800000);
+    const float4 no_box = make_float4(-inf_f, -inf_f, -inf_f, inf_f);
+    const float2 no_yz = make_float2(inf_f, inf_f);
+    W.box[lane] = have ? make_float4(a.x, a.y, a.z, b.x) : no_box;
+    W.yz[lane] = have ? make_float2(b.y, b.z) : no_yz;
+    W.rec[lane] = make_int4(__float_as_int(a.w), inf.x, inf.y, inf.z);
+    W.box[32 + lane] = no_box, W.yz[32 + lane] = no_yz;
+    __syncwarp();
+    const unsigned lt = (1u << lane) - 1u;
     int used = 0, iters = 0;
     while (c > target) {
         if (iters >= P.max_node_iterations) {
             if (lane == 0) atomicOr(P.err, kErrIterations);
             break;
         }
-        float bestd = __int_as_float(0x7F800000);
-        int bestj = -1;
-        // candidates in the order of the key: gap d ascending; at one gap, the candidate with the even lower index
-        // first, then the one below (the key's tie fields after the gap: parity of the lower index, side)
-        auto consider = [&](int d, float df, float db, bool fwd_ok, bool back_ok) {
-            if (((lane - d) & 1) <= (lane & 1)) {
-                if (back_ok && (db < bestd || bestj < 0)) bestd = db, bestj = lane - d;
-                if (fwd_ok && (df < bestd || bestj < 0)) bestd = df, bestj = lane + d;
-            } else {
-                if (fwd_ok && (df < bestd || bestj < 0)) bestd = df, bestj = lane + d;
-                if (back_ok && (db < bestd || bestj < 0)) bestd = db, bestj = lane - d;
-            }
-        };
+        const float4 x = W.box[lane];
+        const float2 xy = W.yz[lane];
+        const int4 rec = W.rec[lane];
+        // Nearest neighbour by the key (distance, gap, parity of the lower index, side): gaps in ascending order with a
+        // strict "<"; at one gap the pair with the even lower index first, then the one below. The pair (lane, lane + g)
+        // is evaluated by its lower lane, which hands the distance up. The search starts from the first candidate of
+        // that order, which wins when every distance is infinite.
+        float bestd = inf_f;
+        int bestg = lane + 1 < c && ((lane & 1) == 0 || lane == 0) ? 1 : -1;
         const int dmax = min(R, c - 1);
-        // two gaps per pass (independent shuffles and distances in flight together), folded in gap order
-        for (int d = 1; d <= dmax; d += 2) {
-            const int e = d + 1;  // the second gap (only when e <= dmax; e <= 32, and a shuffle by 32 is harmless)
-            const float fx = __shfl_down_sync(full, a.x, d), fy = __shfl_down_sync(full, a.y, d);
-            const float fz = __shfl_down_sync(full, a.z, d), gx = __shfl_down_sync(full, b.x, d);
-            const float gy = __shfl_down_sync(full, b.y, d), gz = __shfl_down_sync(full, b.z, d);
-            const float hx = __shfl_down_sync(full, a.x, e), hy = __shfl_down_sync(full, a.y, e);
-            const float hz = __shfl_down_sync(full, a.z, e), kx = __shfl_down_sync(full, b.x, e);
-            const float ky = __shfl_down_sync(full, b.y, e), kz = __shfl_down_sync(full, b.z, e);
-            const bool fwd_d = lane + d < c, fwd_e = e <= dmax && lane + e < c;
-            const float df = fwd_d ? ploc_distance(a.x, a.y, a.z, b.x, b.y, b.z, fx, fy, fz, gx, gy, gz)
-                                   : __int_as_float(0x7F800000);
-            const float de = fwd_e ? ploc_distance(a.x, a.y, a.z, b.x, b.y, b.z, hx, hy, hz, kx, ky, kz)
-                                   : __int_as_float(0x7F800000);
-            const float db = __shfl_up_sync(full, df, d);  // the pair (lane - d, lane), evaluated by lane - d
-            const float dbe = __shfl_up_sync(full, de, e);
-            consider(d, df, db, fwd_d, lane >= d && lane < c);
-            if (e <= dmax) consider(e, de, dbe, fwd_e, lane >= e && lane < c);
+        for (int g0 = 1; g0 <= dmax; g0 += 4) {
+            float up[4], dn[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float4 y = W.box[lane + g0 + k];
+                const float2 yy = W.yz[lane + g0 + k];
+                const float dx = __fsub_rn(fmaxf(x.w, y.w), fminf(x.x, y.x));
+                const float dy = __fsub_rn(fmaxf(xy.x, yy.x), fminf(x.y, y.y));
+                const float dz = __fsub_rn(fmaxf(xy.y, yy.y), fminf(x.z, y.z));
+                up[k] = fminf(__fmaf_rn(dx, dy, __fmaf_rn(dy, dz, __fmul_rn(dz, dx))), inf_f);  // NaN counts as +inf
+                dn[k] = shfl_up_or(up[k], g0 + k, inf_f);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (g0 + k > dmax) break;
+                const bool below = (k & 1) == 0 && (lane & 1) == 0 ? dn[k] < up[k] : dn[k] <= up[k];  // g0 is odd
+                const float m = fminf(dn[k], up[k]);
+                if (m < bestd) bestg = below ? -(g0 + k) : g0 + k;
+                bestd = fminf(bestd, m);
+            }
         }
-        const int partner = bestj >= 0 ? bestj : lane;
-        const int nn_of_partner = __shfl_sync(full, bestj, partner);
         const bool valid = lane < c;
-        const bool mutual = valid && bestj >= 0 && nn_of_partner == lane;
-        const bool creator = mutual && lane < bestj;
-        const float4 pa = shfl4(a, partner), pb = shfl4(b, partner);
-        const int4 pi = shfl4(inf, partner);
+        const int partner = valid ? lane + bestg : lane;
+        const int partner_g = __shfl_sync(full, bestg, partner);
+        const bool mutual = valid && partner_g == -bestg;
+        const bool creator = mutual && bestg > 0;
         const unsigned cm = __ballot_sync(full, creator);
-        const int t = __popc(cm & ((1u << lane) - 1u));
-        const int id = __shfl_sync(full, pool, (used + t) & 31);
-        const int k = id - P.num_leaves;
-        const int left = __float_as_int(a.w), right = __float_as_int(pa.w);
-        const bool in_range = k >= 0 && k < P.num_inner && left >= 0 && left < P.num_leaves + P.num_inner &&
-                              right >= 0 && right < P.num_leaves + P.num_inner;
-        if (creator && !in_range) atomicOr(P.err, kErrIterations);  // never write outside the node arrays
-        if (creator && in_range) {
-            const float3 lo = make_float3(fminf(a.x, pa.x), fminf(a.y, pa.y), fminf(a.z, pa.z));
-            const float3 hi = make_float3(fmaxf(b.x, pb.x), fmaxf(b.y, pb.y), fmaxf(b.z, pb.z));
-            const int count = inf.x + pi.x, pmin = min(inf.y, pi.y), height = max(inf.z, pi.z) + 1;
-            P.child[k] = make_int4(left, right, height, 0);
-            P.node_lo[k] = make_float4(lo.x, lo.y, lo.z, __int_as_float(count));
-            P.node_hi[k] = make_float4(hi.x, hi.y, hi.z, __int_as_float(pmin));
-            P.parent[left] = id;
-            P.parent[right] = id;
-            a = make_float4(lo.x, lo.y, lo.z, __int_as_float(id));
-            b = make_float4(hi.x, hi.y, hi.z, b.w);
-            inf = make_int4(count, pmin, height, 0);
+        const unsigned km = __ballot_sync(full, valid && !(mutual && bestg < 0));
+        const int id = __shfl_sync(full, pool, (used + __popc(cm & lt)) & 31);
+        const float4 y = W.box[partner];
+        const float2 yy = W.yz[partner];
+        const int4 yr = W.rec[partner];
+        float4 nb = x;
+        float2 nyz = xy;
+        int4 nrec = rec;
+        if (creator) {
+            const int k = id - P.num_leaves;
+            const int left = rec.x, right = yr.x;
+            const bool in_range = k >= 0 && k < P.num_inner && left >= 0 && left < P.num_leaves + P.num_inner &&
+                                  right >= 0 && right < P.num_leaves + P.num_inner;
+            if (!in_range) {
+                atomicOr(P.err, kErrIterations);  // never write outside the node arrays
+            } else {
+                nb = make_float4(fminf(x.x, y.x), fminf(x.y, y.y), fminf(x.z, y.z), fmaxf(x.w, y.w));
+                nyz = make_float2(fmaxf(xy.x, yy.x), fmaxf(xy.y, yy.y));
+                nrec = make_int4(id, rec.y + yr.y, min(rec.z, yr.z), max(rec.w, yr.w) + 1);
+                P.child[k] = make_int4(left, right, nrec.w, 0);
+                P.node_lo[k] = make_float4(nb.x, nb.y, nb.z, __int_as_float(nrec.y));
+                P.node_hi[k] = make_float4(nb.w, nyz.x, nyz.y, __int_as_float(nrec.z));
+                P.parent[left] = id;
+                P.parent[right] = id;
+            }
         }
         used += __popc(cm);
-        const bool keep = valid && !(mutual && lane > bestj);
-        const unsigned km = __ballot_sync(full, keep);
         const int nc = __popc(km);
         ++iters;
         if (nc == c) {  // no pair merged: impossible under a strict order on pairs
             if (lane == 0) atomicOr(P.err, kErrIterations);
             break;
         }
-        const int src = lane < nc ? (int)__fns(km, 0, lane + 1) : lane;
-        a = shfl4(a, src);
-        b = shfl4(b, src);
-        inf = shfl4(inf, src);
+        __syncwarp();  // every lane has read its own and its partner's entries
+        if ((km >> lane) & 1u) {
+            const int to = __popc(km & lt);
+            W.box[to] = nb, W.yz[to] = nyz, W.rec[to] = nrec;
+        }
+        if (lane >= nc && lane < c) W.box[lane] = no_box, W.yz[lane] = no_yz;
+        __syncwarp();
         c = nc;
     }
-    if (lane < c) {
-        __stcg(P.lo + nl + lane, a);
-        __stcg(P.hi + nl + lane, b);
-        __stcg(P.info + nl + lane, inf);
+    {
+        const float4 x = W.box[lane];
+        const float2 xy = W.yz[lane];
+        const int4 rec = W.rec[lane];
+        a = make_float4(x.x, x.y, x.z, __int_as_float(rec.x));
+        b = make_float4(x.w, xy.x, xy.y, 0.0f);
+        inf = make_int4(rec.y, rec.z, rec.w, 0);
     }
     const int f = __shfl_sync(full, pool, (used + lane) & 31);
-    if (lane < c - 1) __stcg(P.fid + nl + lane, f);
-    if (lane == 0) __stcg(P.cnt + nl, c);
+    if (own) {
+        b.w = pack_info(inf, b0);
+        if (lane < c) S.lo[nl - b0 + lane] = a, S.hi[nl - b0 + lane] = b;
+        if (lane < c - 1) S.fid[nl - b0 + lane] = (unsigned short)(f - id_base - b0);
+        if (lane == 0) S.cnt[nl - b0] = (unsigned char)c;
+    } else {
+        if (lane < c) __stcg(P.lo + nl + lane, a), __stcg(P.hi + nl + lane, b), __stcg(P.info + nl + lane, inf);
+        if (lane < c - 1) __stcg(P.fid + nl + lane, f);
+        if (lane == 0) __stcg(P.cnt + nl, c);
+    }
     return iters;
 }
 
-template <typename K>
-__global__ void __launch_bounds__(kHplocThreads) hploc_kernel(HplocParams P) {
+template <typename K, int LEAVES, int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS) hploc_kernel(HplocParams P) {
+    __shared__ HplocBlock<K, LEAVES> S;
+    __shared__ HplocWarp s_warp[THREADS / 32];
+    constexpr int kChunks = LEAVES / 32, kWarps = THREADS / 32;
     const unsigned full = 0xffffffffu;
     const K* __restrict__ keys = static_cast<const K*>(P.keys);
     const int N = P.num_leaves;
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    bool active = pos < N;
-    int l = pos, r = pos, mesh = 0, mstart = 0, mend = N - 1;
-    if (active && P.num_meshes > 1) {
-        mesh = find_mesh(P.offsets, P.num_meshes, pos);
-        mstart = (int)__ldg(P.offsets + mesh);
-        mend = (int)__ldg(P.offsets + mesh + 1) - 1;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int b0 = blockIdx.x * LEAVES;
+    const int count = min(LEAVES, N - b0);
+    // ---- the block's leaves and the orders of its splits --------------------------------------------------------------
+    for (int i = tid; i < count; i += THREADS) {
+        const long long g = __ldg(P.perm + b0 + i);
+        const float4 lo = __ldg(P.tbox + 2 * g), hi = __ldg(P.tbox + 2 * g + 1);
+        S.lo[i] = make_float4(lo.x, lo.y, lo.z, __int_as_float(b0 + i));
+        S.hi[i] = make_float4(hi.x, hi.y, hi.z, pack_info(make_int4(1, b0 + i, 0, 0), b0));
+        S.other[i] = -1;
     }
-    const int id_base = N - mesh;
-    int iters = 0;
-    for (int step = 0;; ++step) {
-        bool todo = false;
+    for (int i = tid; i <= count; i += THREADS) {
+        const int p = b0 - 1 + i;
+        S.delta[i] = p >= 0 && p < N - 1 ? __ldg(keys + p) ^ __ldg(keys + p + 1) : K(0);
+    }
+    __syncthreads();
+    auto ties = [](int a, int b) {  // the order of splits a and b whose keys differ alike
+        const unsigned ia = (unsigned)a ^ (unsigned)(a + 1), ib = (unsigned)b ^ (unsigned)(b + 1);
+        return ia != ib ? ia < ib : a < b;
+    };
+    auto before_own = [&](int a, int b) {  // the order of splits a and b of b0 - 1 .. b0 + count - 1
+        const K xa = S.delta[a - b0 + 1], xb = S.delta[b - b0 + 1];
+        return xa != xb ? xa < xb : ties(a, b);
+    };
+    // The node of split s reaches left and right to the nearest splits after s in the order. It lies within the block
+    // when there are such splits among b0 - 1 .. s - 1 and s + 1 .. last (a split before the first or after the last
+    // leaf counts: no node reaches beyond it). Greatest split of a run of splits by a scan, kNoSplit = beyond the leaves.
+    constexpr int kNoSplit = -2;
+    auto later = [&](int a, int b) { return a == kNoSplit || b == kNoSplit ? kNoSplit : (before_own(a, b) ? b : a); };
+    const int last = b0 + count - 1;  // the block's last position; its split is shared with the next block
+    const int left_edge = b0 > 0 ? b0 - 1 : kNoSplit, right_edge = last < N - 1 ? last : kNoSplit;
+    int below[(kChunks + kWarps - 1) / kWarps], above[(kChunks + kWarps - 1) / kWarps];
+#pragma unroll
+    for (int q = 0; q < (kChunks + kWarps - 1) / kWarps; ++q) {
+        const int c = q * kWarps + warp;
+        const int s = min(b0 + 32 * c + lane, last);      // lanes beyond the leaves repeat the last
+        int up = s == last ? right_edge : s, down = up;   // greatest of the chunk's splits up to / from this one
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(full, up, o), d = __shfl_down_sync(full, down, o);
+            if (lane >= o) up = later(up, u);
+            if (lane + o < 32) down = later(down, d);
+        }
+        if (lane == 31) S.edge[0][c] = up;
+        if (lane == 0) S.edge[1][c] = down;
+        below[q] = __shfl_up_sync(full, up, 1), above[q] = __shfl_down_sync(full, down, 1);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < (kChunks + kWarps - 1) / kWarps; ++q) {
+        const int c = q * kWarps + warp;
+        const int s = b0 + 32 * c + lane;
+        int lmax = left_edge, rmax = right_edge;
+        for (int w = 0; w < c; ++w) lmax = later(lmax, S.edge[0][w]);
+        for (int w = c + 1; w < kChunks; ++w) rmax = later(rmax, S.edge[1][w]);
+        if (lane > 0) lmax = later(lmax, below[q]);
+        if (lane < 31) rmax = later(rmax, above[q]);
+        const bool mine = s < last && (lmax == kNoSplit || before_own(s, lmax)) && (rmax == kNoSplit || before_own(s, rmax));
+        const unsigned m = __ballot_sync(full, mine);
+        if (lane == 0) S.mine[c] = m;
+    }
+    __syncthreads();
+
+    // ---- the block's own nodes: arrivals and lists in shared memory ----------------------------------------------------
+    int l = 0, r = 0, mesh = 0, mstart = 0, mend = N - 1, climbs = 0, iters = 0, exits = 0;
+    bool active = false;
+    auto enter = [&](int nl, int nr) {
+        l = nl, r = nr, climbs = 0, active = true;
+        if (P.num_meshes > 1) {
+            mesh = find_mesh(P.offsets, P.num_meshes, nl);
+            mstart = (int)__ldg(P.offsets + mesh);
+            mend = (int)__ldg(P.offsets + mesh + 1) - 1;
+        }
+    };
+    auto process = [&](bool todo, bool own, int split) {
+        unsigned pending = __ballot_sync(full, todo);
+        while (pending) {
+            const int src = __ffs(pending) - 1;
+            pending &= pending - 1u;
+            const int nl = __shfl_sync(full, l, src), nr = __shfl_sync(full, r, src);
+            const int nm = __shfl_sync(full, split, src), nbase = N - __shfl_sync(full, mesh, src);
+            const bool whole = __shfl_sync(full, (int)(l == mstart && r == mend), src) != 0;
+            iters += hploc_node(P, S, s_warp[warp], b0, own, nl, nr, nm, nbase, whole);
+        }
+        __syncwarp();  // every lane's part of the lists and nodes, before any lane's next (releasing) arrival
+    };
+    constexpr int kShare = LEAVES / kWarps;  // leaves per warp; a lane that stops climbing takes the next
+    const int first = b0 + warp * kShare, end = min(first + kShare, b0 + count);
+    for (int next = first;;) {
+        const unsigned idle = __ballot_sync(full, !active);
+        if (next < end && idle) {
+            const int k = next + __popc(idle & lt);
+            if (!active && k < end) enter(k, k);
+            next += __popc(idle);
+        }
+        if (!__any_sync(full, active)) break;
+        bool todo = false, leaves = false;
         int split = -1;
         if (active) {
             if (l == mstart && r == mend) {
                 // this mesh's root, processed by this warp in the previous step (its list is one cluster), or a
                 // one-triangle mesh's leaf: the root goes to the second cluster buffer, where the layout reads it
-                P.root_lo[mesh] = __ldcg(P.lo + mstart);
-                P.root_hi[mesh] = __ldcg(P.hi + mstart);
+                P.root_lo[mesh] = S.lo[mstart - b0];
+                P.root_hi[mesh] = S.hi[mstart - b0];
                 active = false;
-            } else if (step >= kHplocMaxSteps) {
+            } else if (++climbs > kHplocMaxSteps) {
                 active = false;
                 atomicOr(P.err, kErrIterations);
             } else {
-                const bool left_child = l == mstart || (r != mend && split_before(keys, r, l - 1));
+                const bool left_child = l == mstart || (r != mend && before_own(r, l - 1));
                 split = left_child ? r : l - 1;
-                // release: this node's list, written by the lanes of this warp before the warp barrier that ended
-                // the previous step, is visible before the arrival; acquire: so is the sibling's when we are second
+                const unsigned i = (unsigned)(split - b0);
+                if (i < (unsigned)LEAVES && ((S.mine[i >> 5] >> (i & 31u)) & 1u)) {
+                    __threadfence_block();  // the lists written before this arrival, and those read after it
+                    const int prev = atomicExch(&S.other[i], left_child ? l : r);
+                    __threadfence_block();
+                    if (prev < 0) {
+                        active = false;  // first to arrive: the sibling's thread goes on
+                    } else {
+                        if (left_child) r = prev;
+                        else l = prev;
+                        todo = (r - l + 1 > kHplocThreshold) || (l == mstart && r == mend);
+                    }
+                } else {
+                    leaves = true;
+                    active = false;
+                }
+            }
+        }
+        const unsigned lm = __ballot_sync(full, leaves);
+        if (leaves) S.exits[warp * kShare + exits + __popc(lm & lt)] = (unsigned)(l - b0) | ((unsigned)(r - b0) << 16);
+        exits += __popc(lm);
+        process(todo, true, split);
+    }
+    __syncwarp();
+
+    // ---- the nodes that reach beyond the block: arrivals and lists in global memory ---------------------------------------
+    for (int next = 0;;) {
+        const unsigned idle = __ballot_sync(full, !active);
+        if (next < exits && idle) {
+            const int k = next + __popc(idle & lt);
+            const bool takes = !active && k < exits;
+            if (takes) {
+                const unsigned e = S.exits[warp * kShare + k];
+                enter(b0 + (int)(e & 0xFFFFu), b0 + (int)(e >> 16));
+            }
+            next += __popc(idle);
+            unsigned moves = __ballot_sync(full, takes);  // its list goes to global memory
+            while (moves) {
+                const int src = __ffs(moves) - 1;
+                moves &= moves - 1u;
+                const int nl = __shfl_sync(full, l, src), nr = __shfl_sync(full, r, src);
+                const int nbase = N - __shfl_sync(full, mesh, src);
+                const bool merged = nr - nl + 1 > kHplocThreshold;
+                const int c = merged ? S.cnt[nl - b0] : nr - nl + 1;
+                if (lane < c) {
+                    const float4 hi = S.hi[nl - b0 + lane];
+                    __stcg(P.lo + nl + lane, S.lo[nl - b0 + lane]);
+                    __stcg(P.hi + nl + lane, hi);
+                    __stcg(P.info + nl + lane, unpack_info(hi.w, b0));
+                    if (merged && lane < c - 1) __stcg(P.fid + nl + lane, nbase + b0 + (int)S.fid[nl - b0 + lane]);
+                }
+                if (merged && lane == 0) __stcg(P.cnt + nl, c);
+            }
+            __syncwarp();
+        }
+        if (!__any_sync(full, active)) break;
+        bool todo = false;
+        int split = -1;
+        if (active) {
+            if (l == mstart && r == mend) {
+                P.root_lo[mesh] = __ldcg(P.lo + mstart);
+                P.root_hi[mesh] = __ldcg(P.hi + mstart);
+                active = false;
+            } else if (++climbs > kHplocMaxSteps) {
+                active = false;
+                atomicOr(P.err, kErrIterations);
+            } else {
+                bool left_child = l == mstart;
+                if (!left_child && r != mend) {
+                    const K xr = __ldg(keys + r) ^ __ldg(keys + r + 1), xl = __ldg(keys + l - 1) ^ __ldg(keys + l);
+                    left_child = xr != xl ? xr < xl : ties(r, l - 1);
+                }
+                split = left_child ? r : l - 1;
+                // release: this node's list, written by the lanes of this warp before the warp barrier, is visible
+                // before the arrival; acquire: so is the sibling's when we are second
                 const int prev = atomic_exch_acq_rel(P.other + split, left_child ? l : r);
                 if (prev < 0) {
                     active = false;  // first to arrive: the sibling's thread goes on
@@ -1555,20 +1776,10 @@ __global__ void __launch_bounds__(kHplocThreads) hploc_kernel(HplocParams P) {
             }
         }
         __syncwarp();  // every lane's acquire before any lane of the warp loads a list
-        unsigned pending = __ballot_sync(full, todo);
-        while (pending) {
-            const int src = __ffs(pending) - 1;
-            pending &= pending - 1u;
-            const int nl = __shfl_sync(full, l, src), nr = __shfl_sync(full, r, src);
-            const int nm = __shfl_sync(full, split, src), nbase = __shfl_sync(full, id_base, src);
-            const bool whole = __shfl_sync(full, (int)(l == mstart && r == mend), src) != 0;
-            iters += hploc_node(P, nl, nr, nm, nbase, whole);
-        }
-        __syncwarp();  // every lane's part of the lists and nodes, before any lane's next (releasing) arrival
-        if (!__any_sync(full, active)) break;
+        process(todo, false, split);
     }
     // every lane ran the same node iterations: one count per warp
-    if ((threadIdx.x & 31) == 0 && iters) atomicAdd(&P.ctrl->iterations, (uint32_t)iters);
+    if (lane == 0 && iters) atomicAdd(&P.ctrl->iterations, (uint32_t)iters);
 }
 
 __global__ void ploc_init_kernel(const MeshDesc* __restrict__ meshes, const long long* __restrict__ offsets, int m,
@@ -2128,6 +2339,14 @@ dipl_status launch_ploc_tail(const PlocParams& P, cudaStream_t stream) {
 
 inline unsigned blocks_for(long long n, int threads) { return (unsigned)std::max<long long>(1, (n + threads - 1) / threads); }
 
+// Small builds take small blocks, which spread the leaves over more SMs: 3,978 triangles 85 us against 118 us with the
+// large ones, 60k 116 against 144; at 250k the large blocks are ahead (202 against 212 us), at 1M by a third.
+template <typename K>
+void launch_hploc(const HplocParams& P, cudaStream_t stream) {
+    if (P.num_leaves < (1 << 17)) hploc_kernel<K, 64, 64, 12><<<blocks_for(P.num_leaves, 64), 64, 0, stream>>>(P);
+    else hploc_kernel<K, 512, 128, 6><<<blocks_for(P.num_leaves, 512), 128, 0, stream>>>(P);
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------------------------------------
@@ -2471,14 +2690,16 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
         DIPL_CUDA(cudaMemsetAsync(P.status, 0, sizeof(unsigned long long) * (2 * P.tiles_max + 2), stream));
     fill_int_kernel<<<blocks_for(N + K, 256), 256, 0, stream>>>(P.parent, N + K, -1);
     note_launches();
-    ploc_init_kernel<<<blocks_for(N, 256), 256, 0, stream>>>(P.d_meshes, P.d_coffsets, m, N, P.perm, P.tbox,
-                                                             P.c_lo[0], P.c_hi[0], P.c_in[0], P.parent);
-    note_launches();
+    if (!hier) {
+        ploc_init_kernel<<<blocks_for(N, 256), 256, 0, stream>>>(P.d_meshes, P.d_coffsets, m, N, P.perm, P.tbox,
+                                                                 P.c_lo[0], P.c_hi[0], P.c_in[0], P.parent);
+        note_launches();
+    }
     DIPL_CUDA(cudaGetLastError());
     if (hier) {
         DIPL_CUDA(cudaMemsetAsync(P.hp_other, 0xFF, sizeof(int) * N, stream));
         HplocParams hp{};
-        hp.keys = P.keys_sorted, hp.offsets = P.d_coffsets;
+        hp.keys = P.keys_sorted, hp.perm = P.perm, hp.tbox = P.tbox, hp.offsets = P.d_coffsets;
         hp.lo = P.c_lo[0], hp.hi = P.c_hi[0], hp.info = P.c_in[0];
         hp.child = P.child, hp.node_lo = P.nlo, hp.node_hi = P.nhi, hp.parent = P.parent;
         hp.other = P.hp_other, hp.cnt = P.hp_cnt, hp.fid = P.hp_fid;
@@ -2486,9 +2707,8 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
         hp.ctrl = P.d_ctrl, hp.err = P.d_err;
         hp.num_leaves = (int)N, hp.num_inner = (int)K, hp.num_meshes = m, hp.radius = d0.nn_search_radius;
         hp.max_node_iterations = clustering_iteration_limit() ? (int)clustering_iteration_limit() : 64;
-        const unsigned grid = blocks_for(N, kHplocThreads);
-        if (P.key_bytes == 4) hploc_kernel<uint32_t><<<grid, kHplocThreads, 0, stream>>>(hp);
-        else hploc_kernel<unsigned long long><<<grid, kHplocThreads, 0, stream>>>(hp);
+        if (P.key_bytes == 4) launch_hploc<uint32_t>(hp, stream);
+        else launch_hploc<unsigned long long>(hp, stream);
         note_launches();
         DIPL_CUDA(cudaGetLastError());
     }

@@ -115,6 +115,20 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
+// Position of the n-th set bit of m (n from 0; m has more than n bits set), by halving: 5 popcounts.
+__device__ __forceinline__ int nth_set_bit(uint32_t m, int n) {
+    int pos = 0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const int c = __popc(m & ((1u << w) - 1u));
+        const bool above = n >= c;
+        n -= above ? c : 0;
+        pos += above ? w : 0;
+        m = above ? m >> w : m;
+    }
+    return pos;
+}
+
 // Grid-wide barrier for co-resident (cooperatively launched) blocks: sense by generation count,
 // bounded spin. Returns false (and sets *err) if it gave up.
 struct GridBarrier {

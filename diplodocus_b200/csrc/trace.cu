@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(kTraceThreads) tail_kernel(const BNode* __rest
                 }
                 const int rank = __popc(hm & lt_mask);
                 const bool receive = hungry && rank < nd;
-                const int src = receive ? (int)__fns(dm, 0, rank + 1) : lane;
+                const int src = receive ? nth_set_bit(dm, rank) : lane;
                 const int rref = __shfl_sync(full, gref, src);
                 const float rt = __shfl_sync(full, gt, src);
                 if (receive && rref != kNone && rt <= lim) cur = rref;
@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(kTraceThreads, PERSIST ? 8 : 9) quad_trace_ker
         if (idle && givers) {
             const int rank = __popc(idle & lt_mask);
             const bool take = !working && rank < __popc(givers);
-            const int src = take ? (int)__fns(givers, 0, rank + 1) : lane;
+            const int src = take ? nth_set_bit(givers, rank) : lane;
             const int sbot = __shfl_sync(full, bot, src), sowner = __shfl_sync(full, owner, src);
             QRay q;
             q.o.x = __shfl_sync(full, r.o.x, src), q.o.y = __shfl_sync(full, r.o.y, src);
