@@ -36,8 +36,38 @@ uint32_t clustering_iteration_limit() { return g_clustering_iterations.load(std:
 uint32_t trace_step_limit() { return g_trace_steps.load(std::memory_order_relaxed); }
 
 static DeviceProbe g_pool_configured;  // per device: each device has its own default pool
+static DeviceProbe g_kept_probe;
+static cudaMemPool_t g_kept_pool[kMaxProbeDevices];  // written under g_kept_probe's lock, once per device
 
-dipl_status device_alloc(void** ptr, size_t bytes, cudaStream_t stream) {
+// Keep freed blocks for reuse: builds allocate the same sizes repeatedly.
+static void keep_blocks(cudaMemPool_t pool) {
+    uint64_t threshold = ~0ull;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
+}
+
+// The pool of the arrays that handles keep, nullptr where there is none (they then come from the default pool). A pool
+// hands out the block freed last, whatever its size: with one pool a build's scratch took the block of the handle just
+// destroyed, and the new handle's arrays then had to be mapped anew (16M soup: 7 to 200 ms).
+static cudaMemPool_t kept_pool() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxProbeDevices) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    const int ok = probe_per_device(g_kept_probe, [dev] {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        const bool made = cudaMemPoolCreate(&g_kept_pool[dev], &props) == cudaSuccess;
+        if (made) keep_blocks(g_kept_pool[dev]);
+        (void)cudaGetLastError();
+        return made ? 1 : 0;
+    });
+    return ok ? g_kept_pool[dev] : nullptr;
+}
+
+dipl_status device_alloc(void** ptr, size_t bytes, cudaStream_t stream, bool kept) {
     {
         std::lock_guard<std::mutex> lock(g_mem_mu);
         const uint64_t limit = g_mem_limit.load(std::memory_order_relaxed);
@@ -53,14 +83,23 @@ dipl_status device_alloc(void** ptr, size_t bytes, cudaStream_t stream) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess) return 0;
         cudaMemPool_t pool;
-        if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-            uint64_t threshold = ~0ull;  // keep freed blocks for reuse: builds allocate the same sizes repeatedly
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
-        }
+        if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) keep_blocks(pool);
         (void)cudaGetLastError();
         return 1;
     });
-    cudaError_t e = cudaMallocAsync(ptr, bytes, stream);
+    cudaMemPool_t own = kept ? kept_pool() : nullptr;
+    cudaError_t e = own ? cudaMallocFromPoolAsync(ptr, bytes, own, stream) : cudaMallocAsync(ptr, bytes, stream);
+    if (e == cudaErrorMemoryAllocation) {
+        // the other pool may hold free blocks: give them back and try once more
+        (void)cudaGetLastError();
+        int dev = 0;
+        cudaMemPool_t pool;
+        cudaStreamSynchronize(stream);
+        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+            cudaMemPoolTrimTo(pool, 0);
+        if (cudaMemPool_t k = kept_pool()) cudaMemPoolTrimTo(k, 0);
+        e = own ? cudaMallocFromPoolAsync(ptr, bytes, own, stream) : cudaMallocAsync(ptr, bytes, stream);
+    }
     std::lock_guard<std::mutex> lock(g_mem_mu);
     if (e != cudaSuccess) {
         g_mem_in_use -= bytes;

@@ -42,7 +42,6 @@ struct PlocCtrl {
     uint32_t n[2];       // cluster count at the start of an iteration (by parity)
     uint32_t merges[2];  // internal nodes created before an iteration (by parity)
     uint32_t iterations;
-    uint32_t roots_second;    // 1: the roots are in the second cluster buffer (hierarchical clustering)
     uint32_t tiles_taken[2];  // tiles claimed in an iteration (by parity)
     GridBarrier barrier;
 };
@@ -1782,30 +1781,19 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) hploc_kernel(HplocParams P) {
     if (lane == 0 && iters) atomicAdd(&P.ctrl->iterations, (uint32_t)iters);
 }
 
-__global__ void ploc_init_kernel(const MeshDesc* __restrict__ meshes, const long long* __restrict__ offsets, int m,
-                                 long long n, const uint32_t* __restrict__ perm, const float4* __restrict__ tbox,
+__global__ void ploc_init_kernel(const long long* __restrict__ offsets, int m, long long n,
+                                 const uint32_t* __restrict__ perm, const float4* __restrict__ tbox,
                                  float4* __restrict__ lo, float4* __restrict__ hi, int4* __restrict__ info,
-                                 int* __restrict__ parent) {
+                                 PlocCtrl* __restrict__ ctrl) {
     long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (p == 0) ctrl->n[0] = (uint32_t)n;  // the rest starts at zero
     if (p >= n) return;
     long long g = perm[p];
-    int k = find_mesh(offsets, m, g);
-    (void)meshes;
+    int k = find_mesh(offsets, m, p);
     const float4 a = __ldg(tbox + 2 * g), b = __ldg(tbox + 2 * g + 1);
     lo[p] = make_float4(a.x, a.y, a.z, __int_as_float((int)p));
     hi[p] = make_float4(b.x, b.y, b.z, __int_as_float(k));
     info[p] = make_int4(1, (int)p, 0, 0);
-    parent[p] = -1;
-}
-
-__global__ void ploc_ctrl_init_kernel(PlocCtrl* ctrl, uint32_t n, uint32_t roots_second) {
-    ctrl->n[0] = n;  // the rest was cleared by a memset
-    ctrl->roots_second = roots_second;
-}
-
-__global__ void fill_int_kernel(int* p, long long n, int v) {
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -2202,16 +2190,21 @@ struct RootInfo {
 
 __global__ void roots_kernel(LayoutParams P, const float4* __restrict__ lo0, const float4* __restrict__ hi0,
                              const float4* __restrict__ lo1, const float4* __restrict__ hi1, const PlocCtrl* ctrl,
-                             int m, const uint32_t* __restrict__ rev_index, const int* __restrict__ leaf_start_of,
-                             RootInfo* __restrict__ roots, const uint32_t* err) {
+                             bool hier, int m, const uint32_t* __restrict__ rev_index,
+                             const int* __restrict__ leaf_start_of, RootInfo* __restrict__ roots,
+                             uint32_t* __restrict__ counts, const uint32_t* err) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0) {
+        counts[1] = ctrl->iterations;
+        counts[2] = *err;
+    }
     if (k >= m) return;
     RootInfo ri{};
     if (*err != 0u) {
         roots[k] = ri;
         return;
     }
-    const bool odd = ctrl->roots_second != 0u || (ctrl->iterations & 1u) != 0u;
+    const bool odd = hier || (ctrl->iterations & 1u) != 0u;
     const float4* final_lo = odd ? lo1 : lo0;
     const float4* final_hi = odd ? hi1 : hi0;
     int id = __float_as_int(final_lo[k].w);
@@ -2405,6 +2398,8 @@ struct BuildPlan {
     long long* d_coffsets = nullptr;  // = d_offsets without pre-splitting
     uint32_t *pieces = nullptr, *piece_first = nullptr;  // per triangle: references, first reference
     unsigned long long* mesh_wsum = nullptr;
+    uint32_t *d_total = nullptr, *d_split_err = nullptr;
+    unsigned char* piece_scan = nullptr;
     int* ref_tri = nullptr;           // per reference: its triangle (global index); NULL without pre-splitting
     Bounds* d_bounds = nullptr;
     CodeParams* d_params = nullptr;
@@ -2423,7 +2418,10 @@ struct BuildPlan {
     uint32_t *rev_flags = nullptr, *contrib = nullptr, *d_counts = nullptr;
     int *owner_leaf = nullptr, *leaf_start_of = nullptr;
     int* slot_pos = nullptr;  // pre-split SOBB builds: per slot of the leaf triangle array, its sorted position
-    unsigned char* scan_scratch = nullptr;
+    unsigned char *height_scratch = nullptr, *scan_scratch[2] = {nullptr, nullptr};
+    unsigned char* zero = nullptr;       // the summary, the controls and the scratch that start at zero
+    unsigned char* d_summary = nullptr;  // roots, SAH sums, counts: read back as one
+    size_t zero_bytes = 0, ones_bytes = 0;
     BNode* nodes = nullptr;
     QNode* quads = nullptr;  // binary AABB layout only
     float4* tris = nullptr;
@@ -2431,6 +2429,7 @@ struct BuildPlan {
     RootInfo* d_roots = nullptr;
     SobbScratch sobb{};
     SNode* snodes = nullptr;
+    WideScratch wide{};
     unsigned char* h_summary = nullptr;  // pinned
     bool owns_summary = false;
     size_t summary_bytes = 0;
@@ -2445,6 +2444,49 @@ struct BuildPlan {
 };
 
 static dipl_status enqueue_bounds_and_params(BuildPlan& P, cudaStream_t stream);
+
+// Pre-splitting: bounds and code parameters (they are the triangles'), the piece counts, their scan and every mesh's
+// first reference; the reference count sizes what the handles keep, so it is read back here.
+static dipl_status count_references(BuildPlan& P, cudaStream_t stream) {
+    const long long T = P.T;
+    const int m = P.m;
+    dipl_status st;
+    P.d_err = P.d_split_err;
+    if ((st = enqueue_bounds_and_params(P, stream)) != DIPL_OK) return st;
+    DIPL_CUDA(cudaMemsetAsync(P.mesh_wsum, 0, sizeof(unsigned long long) * m, stream));
+    split_weight_kernel<<<blocks_for(T, 256), 256, 0, stream>>>(P.d_meshes, P.d_offsets, m, T, P.d_bounds, P.mesh_wsum);
+    note_launches();
+    split_count_kernel<<<blocks_for(T, 256), 256, 0, stream>>>(P.d_meshes, P.d_offsets, m, T, P.d_bounds, P.mesh_wsum,
+                                                               P.d0.split_budget, P.pieces);
+    note_launches();
+    DIPL_CUDA(cudaGetLastError());
+    if ((st = exclusive_scan_u32(P.pieces, P.piece_first, T, P.d_total, P.piece_scan, stream, P.d_err)) != DIPL_OK)
+        return st;
+    mesh_ref_offsets_kernel<<<blocks_for(m + 1, 64), 64, 0, stream>>>(P.d_offsets, m, P.piece_first, P.d_total,
+                                                                      P.d_coffsets);
+    note_launches();
+    DIPL_CUDA(cudaGetLastError());
+    P.coffsets.assign(m + 1, 0);
+    DIPL_CUDA(cudaMemcpyAsync(P.coffsets.data(), P.d_coffsets, sizeof(long long) * (m + 1), cudaMemcpyDeviceToHost,
+                              stream));
+    uint32_t err = 0;
+    DIPL_CUDA(cudaMemcpyAsync(&err, P.d_err, 4, cudaMemcpyDeviceToHost, stream));
+    DIPL_CUDA(cudaStreamSynchronize(stream));
+    if (err != 0u) {
+        set_last_error("build: a bounded device wait timed out while counting the pieces of large triangles");
+        return DIPL_ERR_TIMEOUT;
+    }
+    const long long bound = T + T * P.d0.split_budget / 100;
+    P.N = P.coffsets[m];
+    DIPL_CHECK_ARG(P.N < (1ll << 27), "references of a build (triangles and their pieces) must be < 2^27");
+    if (P.N > bound) {
+        set_last_error("build: more references than the budget allows (internal)");
+        return DIPL_ERR_INTERNAL;
+    }
+    P.K = P.N - m;
+    P.Kalloc = std::max<long long>(P.K, 1);
+    return DIPL_OK;
+}
 
 static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int count, cudaStream_t stream,
                                 bool own_summary) {
@@ -2486,66 +2528,40 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
     P.L = d0.max_triangles_per_leaf;
     P.out = std::make_shared<Storage>();
     P.out->stream = stream;
+    P.out->kept = true;
     P.work = std::make_shared<Storage>();
     P.work->stream = stream;
     dipl_status st;
-    if ((st = P.out->alloc(&P.d_err, 4)) != DIPL_OK) return st;
     P.K = P.N - P.m;
     P.Kalloc = std::max<long long>(P.K, 1);
-    if (P.m == 0) return DIPL_OK;
+    if (P.m == 0) {
+        P.out->reserve(&P.d_err, 4);
+        return P.out->commit();
+    }
     const int m = P.m;
     Storage& W = *P.work;
     Storage& O = *P.out;
-    if ((st = W.alloc(&P.d_meshes, m)) != DIPL_OK || (st = W.alloc(&P.d_offsets, m + 1)) != DIPL_OK ||
-        (st = W.alloc(&P.d_bounds, m)) != DIPL_OK || (st = W.alloc(&P.d_params, m)) != DIPL_OK)
-        return st;
-    DIPL_CUDA(cudaMemcpyAsync(P.d_meshes, P.meshes.data(), sizeof(MeshDesc) * m, cudaMemcpyHostToDevice, stream));
-    DIPL_CUDA(cudaMemcpyAsync(P.d_offsets, P.offsets.data(), sizeof(long long) * (m + 1), cudaMemcpyHostToDevice,
-                              stream));
-    P.d_coffsets = P.d_offsets;
+    // meshes and offsets in one block: one upload
+    const size_t mesh_bytes = sizeof(MeshDesc) * m, table_bytes = mesh_bytes + sizeof(long long) * (m + 1);
+    std::vector<unsigned char> table(table_bytes);
+    std::memcpy(table.data(), P.meshes.data(), mesh_bytes);
+    std::memcpy(table.data() + mesh_bytes, P.offsets.data(), table_bytes - mesh_bytes);
+    unsigned char* d_table = nullptr;
+    W.reserve(&d_table, table_bytes);
+    W.reserve(&P.d_bounds, m);
+    W.reserve(&P.d_params, m);
+    // Scratch is sized by a bound on the references, at most split_budget percent more than the triangles, so that it is
+    // one block taken before they are counted; what the handles keep is taken after, by the count.
+    const long long N = P.split ? P.T + P.T * d0.split_budget / 100 : P.T, K = N - m, Kalloc = std::max<long long>(K, 1);
     if (P.split) {
-        // bounds and code parameters first (they are the triangles'), then the piece counts, their scan and every
-        // mesh's first reference; the reference count sizes everything after, so it is read back here
-        const long long T = P.T;
-        uint32_t* d_total = nullptr;
-        if ((st = W.alloc(&P.pieces, T)) != DIPL_OK || (st = W.alloc(&P.piece_first, T)) != DIPL_OK ||
-            (st = W.alloc(&P.mesh_wsum, m)) != DIPL_OK || (st = W.alloc(&P.d_coffsets, m + 1)) != DIPL_OK ||
-            (st = W.alloc(&d_total, 4)) != DIPL_OK)
-            return st;
-        unsigned char* scan_tmp = nullptr;
-        if ((st = W.alloc(&scan_tmp, scan_scratch_bytes(T))) != DIPL_OK) return st;
-        if ((st = enqueue_bounds_and_params(P, stream)) != DIPL_OK) return st;
-        DIPL_CUDA(cudaMemsetAsync(P.mesh_wsum, 0, sizeof(unsigned long long) * m, stream));
-        split_weight_kernel<<<blocks_for(T, 256), 256, 0, stream>>>(P.d_meshes, P.d_offsets, m, T, P.d_bounds,
-                                                                    P.mesh_wsum);
-        note_launches();
-        split_count_kernel<<<blocks_for(T, 256), 256, 0, stream>>>(P.d_meshes, P.d_offsets, m, T, P.d_bounds,
-                                                                   P.mesh_wsum, d0.split_budget, P.pieces);
-        note_launches();
-        DIPL_CUDA(cudaGetLastError());
-        if ((st = exclusive_scan_u32(P.pieces, P.piece_first, T, d_total, scan_tmp, stream, P.d_err)) != DIPL_OK)
-            return st;
-        mesh_ref_offsets_kernel<<<blocks_for(m + 1, 64), 64, 0, stream>>>(P.d_offsets, m, P.piece_first, d_total,
-                                                                          P.d_coffsets);
-        note_launches();
-        DIPL_CUDA(cudaGetLastError());
-        P.coffsets.assign(m + 1, 0);
-        DIPL_CUDA(cudaMemcpyAsync(P.coffsets.data(), P.d_coffsets, sizeof(long long) * (m + 1), cudaMemcpyDeviceToHost,
-                                  stream));
-        uint32_t err = 0;
-        DIPL_CUDA(cudaMemcpyAsync(&err, P.d_err, 4, cudaMemcpyDeviceToHost, stream));
-        DIPL_CUDA(cudaStreamSynchronize(stream));
-        if (err != 0u) {
-            set_last_error("build: a bounded device wait timed out while counting the pieces of large triangles");
-            return DIPL_ERR_TIMEOUT;
-        }
-        P.N = P.coffsets[m];
-        DIPL_CHECK_ARG(P.N < (1ll << 27), "references of a build (triangles and their pieces) must be < 2^27");
-        P.K = P.N - m;
-        P.Kalloc = std::max<long long>(P.K, 1);
-        if ((st = O.alloc(&P.ref_tri, P.N)) != DIPL_OK) return st;
+        W.reserve(&P.pieces, P.T);
+        W.reserve(&P.piece_first, P.T);
+        W.reserve(&P.mesh_wsum, m);
+        W.reserve(&P.d_coffsets, m + 1);
+        W.reserve(&P.d_total, 4);
+        W.reserve(&P.piece_scan, scan_scratch_bytes(P.T));
+        W.reserve(&P.d_split_err, 4);
     }
-    const long long N = P.N, K = P.K, Kalloc = P.Kalloc;
     P.code_bits = d0.code_type == DIPL_CODE_MORTON30 ? 30 : 60;
     while ((1ll << P.mesh_bits) < m) ++P.mesh_bits;
     P.key_bits = P.code_bits + P.mesh_bits;
@@ -2556,43 +2572,95 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
     P.mesh_shift = P.mesh_bits > 0 ? P.code_bits - P.code_shift : 0;
     P.key_bytes = P.key_bits <= 32 ? 4 : 8;
     P.digit_bits = d0.sort_digit_bits > 0 ? d0.sort_digit_bits : 8;
-    if ((st = W.alloc((unsigned char**)&P.keys, N * P.key_bytes)) != DIPL_OK ||
-        (st = W.alloc((unsigned char**)&P.keys_sorted, N * P.key_bytes)) != DIPL_OK ||
-        (st = W.alloc((unsigned char**)&P.keys_alt, N * P.key_bytes)) != DIPL_OK ||
-        (st = O.alloc(&P.perm, N)) != DIPL_OK || (st = W.alloc(&P.perm_alt, N)) != DIPL_OK ||
-        (st = W.alloc(&P.tbox, 2 * N)) != DIPL_OK ||
-        (st = W.alloc(&P.sort_scratch, radix_sort_scratch_bytes(N, 0, P.key_bits, P.digit_bits))) != DIPL_OK)
-        return st;
-    P.B = ploc_block_for(d0.ploc_block_size, (int64_t)N);
-    P.tiles0 = (int)((N + P.B * ploc_ipt_max(P.B) - 1) / (P.B * ploc_ipt_max(P.B)));
-    P.tiles_max = (int)((N + P.B - 1) / P.B);
-    if ((st = W.alloc(&P.d_ctrl, 1)) != DIPL_OK || (st = O.alloc(&P.child, Kalloc)) != DIPL_OK ||
-        (st = O.alloc(&P.nlo, Kalloc)) != DIPL_OK || (st = O.alloc(&P.nhi, Kalloc)) != DIPL_OK ||
-        (st = W.alloc(&P.parent, N + Kalloc)) != DIPL_OK || (st = W.alloc(&P.status, 2 * P.tiles_max + 2)) != DIPL_OK)
-        return st;
-    for (int k = 0; k < 2; ++k)
-        if ((st = W.alloc(&P.c_lo[k], N)) != DIPL_OK || (st = W.alloc(&P.c_hi[k], N)) != DIPL_OK ||
-            (st = W.alloc(&P.c_in[k], N)) != DIPL_OK)
-            return st;
-    if (d0.clustering == DIPL_CLUSTER_HPLOC &&
-        ((st = W.alloc(&P.hp_other, N)) != DIPL_OK || (st = W.alloc(&P.hp_cnt, N)) != DIPL_OK ||
-         (st = W.alloc(&P.hp_fid, N)) != DIPL_OK))
-        return st;
-    if ((st = W.alloc(&P.rev_flags, Kalloc)) != DIPL_OK || (st = W.alloc(&P.contrib, N)) != DIPL_OK ||
-        (st = W.alloc(&P.owner_leaf, N)) != DIPL_OK || (st = W.alloc(&P.leaf_start_of, N + Kalloc)) != DIPL_OK ||
-        (st = W.alloc(&P.scan_scratch, scan_scratch_bytes(std::max(N, Kalloc)))) != DIPL_OK ||
-        (st = W.alloc(&P.d_counts, 4)) != DIPL_OK || (st = O.alloc(&P.nodes, Kalloc)) != DIPL_OK ||
-        (st = O.alloc(&P.tris, 3 * N)) != DIPL_OK || (st = W.alloc(&P.d_sah, 2 * m)) != DIPL_OK ||
-        (st = W.alloc(&P.d_roots, m)) != DIPL_OK)
-        return st;
-    if (d0.bv_type == DIPL_BV_AABB && d0.layout == DIPL_LAYOUT_BINARY &&
-        (st = O.alloc(&P.quads, Kalloc)) != DIPL_OK)
-        return st;
-    if (d0.bv_type == DIPL_BV_SOBB) {
-        if ((st = sobb_prepare(N, K, W, O, &P.sobb, &P.snodes)) != DIPL_OK) return st;
-        if (P.split && (st = W.alloc(&P.slot_pos, N)) != DIPL_OK) return st;
+    const bool hier = d0.clustering == DIPL_CLUSTER_HPLOC;
+    auto set_tiles = [&P](long long n) {
+        P.B = ploc_block_for(P.d0.ploc_block_size, (int64_t)n);
+        P.tiles0 = (int)((n + P.B * ploc_ipt_max(P.B) - 1) / (P.B * ploc_ipt_max(P.B)));
+        P.tiles_max = (int)((n + P.B - 1) / P.B);
+    };
+    set_tiles(N);
+    W.reserve((unsigned char**)&P.keys, N * P.key_bytes);
+    W.reserve((unsigned char**)&P.keys_sorted, N * P.key_bytes);
+    W.reserve((unsigned char**)&P.keys_alt, N * P.key_bytes);
+    W.reserve(&P.perm_alt, N);
+    W.reserve(&P.tbox, 2 * N);
+    for (int k = 0; k < 2; ++k) {  // the hierarchical clustering keeps only the roots in the second buffer
+        W.reserve(&P.c_lo[k], hier && k ? m : N);
+        W.reserve(&P.c_hi[k], hier && k ? m : N);
+        W.reserve(&P.c_in[k], hier && k ? m : N);
     }
+    if (hier) {
+        W.reserve(&P.hp_cnt, N);
+        W.reserve(&P.hp_fid, N);
+    }
+    W.reserve(&P.rev_flags, Kalloc);
+    W.reserve(&P.contrib, N);
+    W.reserve(&P.owner_leaf, N);
+    W.reserve(&P.leaf_start_of, N + Kalloc);
+    // what a build starts from all ones (parents, arrivals) and from zero, each in one block: one memset
+    P.ones_bytes = sizeof(int) * (size_t)(N + Kalloc + (hier ? N : 0));
+    W.reserve(&P.parent, P.ones_bytes / sizeof(int));
     P.summary_bytes = sizeof(RootInfo) * m + sizeof(double) * 2 * m + 16;
+    auto pad = [](size_t b) { return (b + 255) & ~size_t(255); };
+    const size_t sort_bytes = pad(radix_sort_scratch_bytes(N, 0, P.key_bits, P.digit_bits));
+    const size_t height_bytes = hier ? pad(radix_sort_scratch_bytes(Kalloc, 0, 8, 8)) : 0;
+    const size_t scan_bytes = pad(scan_scratch_bytes(std::max(N, Kalloc)));
+    const size_t status_bytes = hier ? 0 : pad(sizeof(unsigned long long) * (2 * P.tiles_max + 2));
+    P.zero_bytes = pad(P.summary_bytes) + pad(sizeof(PlocCtrl)) + sort_bytes + height_bytes + 2 * scan_bytes + status_bytes;
+    W.reserve(&P.zero, P.zero_bytes);
+    const bool wide = d0.layout == DIPL_LAYOUT_WIDE8_Q8, sobb = d0.bv_type == DIPL_BV_SOBB;
+    if (wide) {  // the binary layout is only a step towards the kept one
+        W.reserve(&P.nodes, Kalloc);
+        W.reserve(&P.tris, 3 * N);
+        wide_reserve(P.wide, W, Kalloc);
+    }
+    if (sobb) {
+        if ((st = sobb_prepare(N, K, W, &P.sobb)) != DIPL_OK) return st;
+        if (P.split) W.reserve(&P.slot_pos, N);
+    }
+    if ((st = W.commit()) != DIPL_OK) return st;
+    P.d_meshes = reinterpret_cast<MeshDesc*>(d_table);
+    P.d_offsets = reinterpret_cast<long long*>(d_table + mesh_bytes);
+    if (!P.split) P.d_coffsets = P.d_offsets;
+    DIPL_CUDA(cudaMemcpyAsync(d_table, table.data(), table_bytes, cudaMemcpyHostToDevice, stream));
+    if (P.split) {
+        if ((st = count_references(P, stream)) != DIPL_OK) return st;
+        O.reserve(&P.ref_tri, P.N);
+    }
+    O.reserve(&P.d_err, 4);
+    O.reserve(&P.perm, P.N);
+    O.reserve(&P.child, P.Kalloc);
+    O.reserve(&P.nlo, P.Kalloc);
+    O.reserve(&P.nhi, P.Kalloc);
+    if (wide) {
+        O.reserve(&P.wide.nodes, P.Kalloc);
+        O.reserve(&P.wide.tris, 3 * P.N);
+    } else {
+        O.reserve(&P.nodes, P.Kalloc);
+        O.reserve(&P.tris, 3 * P.N);
+        if (sobb) O.reserve(&P.snodes, P.Kalloc);
+        else O.reserve(&P.quads, P.Kalloc);
+    }
+    if ((st = O.commit()) != DIPL_OK) return st;
+    if (P.split) DIPL_CUDA(cudaMemsetAsync(P.d_err, 0, 4, stream));
+    if (hier) P.hp_other = P.parent + N + Kalloc;
+    unsigned char* z = P.zero;
+    auto carve = [&](size_t bytes) {
+        unsigned char* at = z;
+        z += bytes;
+        return at;
+    };
+    P.d_summary = carve(pad(P.summary_bytes));
+    P.d_roots = reinterpret_cast<RootInfo*>(P.d_summary);
+    P.d_sah = reinterpret_cast<double*>(P.d_summary + sizeof(RootInfo) * m);
+    P.d_counts = reinterpret_cast<uint32_t*>(P.d_summary + sizeof(RootInfo) * m + sizeof(double) * 2 * m);
+    P.d_ctrl = reinterpret_cast<PlocCtrl*>(carve(pad(sizeof(PlocCtrl))));
+    P.sort_scratch = carve(sort_bytes);
+    P.height_scratch = carve(height_bytes);
+    P.scan_scratch[0] = carve(scan_bytes);
+    P.scan_scratch[1] = carve(scan_bytes);
+    P.status = reinterpret_cast<unsigned long long*>(carve(status_bytes));
+    set_tiles(P.N);  // at most as many as the status was sized for
     if (own_summary) {  // a plan replays into its own pinned buffer
         if (cudaMallocHost(&P.h_summary, P.summary_bytes) != cudaSuccess) {
             P.h_summary = nullptr;
@@ -2676,28 +2744,22 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
         note_launches();
     }
     DIPL_CUDA(cudaGetLastError());
+    DIPL_CUDA(cudaMemsetAsync(P.zero, 0, P.zero_bytes, stream));
+    DIPL_CUDA(cudaMemsetAsync(P.parent, 0xFF, P.ones_bytes, stream));
     st = radix_sort_pairs(P.keys, nullptr, P.keys_sorted, P.perm, P.keys_alt, P.perm_alt, N, P.key_bytes, 0,
-                          P.key_bits, P.digit_bits, P.sort_scratch, stream, P.d_err);
+                          P.key_bits, P.digit_bits, P.sort_scratch, stream, P.d_err, true);
     if (st != DIPL_OK) return st;
 
     // ---- PLOC ------------------------------------------------------------------------------------------
     PlocParams pp{};
-    DIPL_CUDA(cudaMemsetAsync(P.d_ctrl, 0, sizeof(PlocCtrl), stream));
     const bool hier = d0.clustering == DIPL_CLUSTER_HPLOC;
-    ploc_ctrl_init_kernel<<<1, 1, 0, stream>>>(P.d_ctrl, (uint32_t)N, hier ? 1u : 0u);
-    note_launches();
-    if (!hier)
-        DIPL_CUDA(cudaMemsetAsync(P.status, 0, sizeof(unsigned long long) * (2 * P.tiles_max + 2), stream));
-    fill_int_kernel<<<blocks_for(N + K, 256), 256, 0, stream>>>(P.parent, N + K, -1);
-    note_launches();
     if (!hier) {
-        ploc_init_kernel<<<blocks_for(N, 256), 256, 0, stream>>>(P.d_meshes, P.d_coffsets, m, N, P.perm, P.tbox,
-                                                                 P.c_lo[0], P.c_hi[0], P.c_in[0], P.parent);
+        ploc_init_kernel<<<blocks_for(N, 256), 256, 0, stream>>>(P.d_coffsets, m, N, P.perm, P.tbox, P.c_lo[0],
+                                                                 P.c_hi[0], P.c_in[0], P.d_ctrl);
         note_launches();
     }
     DIPL_CUDA(cudaGetLastError());
     if (hier) {
-        DIPL_CUDA(cudaMemsetAsync(P.hp_other, 0xFF, sizeof(int) * N, stream));
         HplocParams hp{};
         hp.keys = P.keys_sorted, hp.perm = P.perm, hp.tbox = P.tbox, hp.offsets = P.d_coffsets;
         hp.lo = P.c_lo[0], hp.hi = P.c_hi[0], hp.info = P.c_in[0];
@@ -2735,12 +2797,11 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
 
     // ---- layout -------------------------------------------------------------------------------------
     LayoutParams LP{P.child, P.nlo, P.nhi, P.parent, (int)N, (int)K, P.L};
-    DIPL_CUDA(cudaMemsetAsync(P.d_sah, 0, sizeof(double) * 2 * m, stream));
-    DIPL_CUDA(cudaMemsetAsync(P.d_counts, 0, 16, stream));
     if (K > 0) {
         inner_flags_kernel<<<blocks_for(K, 256), 256, 0, stream>>>(LP, P.rev_flags, P.d_err);
         note_launches();
-        if ((st = exclusive_scan_u32(P.rev_flags, P.rev_flags, K, P.d_counts, P.scan_scratch, stream, P.d_err)) !=
+        if ((st = exclusive_scan_u32(P.rev_flags, P.rev_flags, K, P.d_counts, P.scan_scratch[0], stream, P.d_err,
+                                     true)) !=
             DIPL_OK)
             return st;
         if (hier) {
@@ -2754,7 +2815,7 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
             note_launches();
             DIPL_CUDA(cudaGetLastError());
             if ((st = radix_sort_pairs(hkeys, nullptr, hsorted, P.perm_alt, P.keys_alt, P.contrib, K, 4, 0, 8, 8,
-                                       P.sort_scratch, stream, P.d_err)) != DIPL_OK)
+                                       P.height_scratch, stream, P.d_err, true)) != DIPL_OK)
                 return st;
             height_index_kernel<<<blocks_for(K, 256), 256, 0, stream>>>(LP, P.perm_alt, P.rev_flags, P.d_err);
             note_launches();
@@ -2762,7 +2823,8 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
     }
     leaf_owner_kernel<<<blocks_for(N, 256), 256, 0, stream>>>(LP, P.contrib, P.owner_leaf, P.d_err);
     note_launches();
-    if ((st = exclusive_scan_u32(P.contrib, P.contrib, N, nullptr, P.scan_scratch, stream, P.d_err)) != DIPL_OK)
+    if ((st = exclusive_scan_u32(P.contrib, P.contrib, N, nullptr, P.scan_scratch[1], stream, P.d_err, true)) !=
+        DIPL_OK)
         return st;
     leaf_write_kernel<<<blocks_for(N, 256), 256, 0, stream>>>(LP, P.d_meshes, P.d_offsets, m, P.perm, P.ref_tri,
                                                                P.contrib, P.leaf_start_of, P.tris, P.slot_pos, P.d_err);
@@ -2776,9 +2838,6 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
             note_launches();
         }
     }
-    roots_kernel<<<blocks_for(m, 64), 64, 0, stream>>>(LP, P.c_lo[0], P.c_hi[0], P.c_lo[1], P.c_hi[1], P.d_ctrl, m,
-                                                       P.rev_flags, P.leaf_start_of, P.d_roots, P.d_err);
-    note_launches();
     DIPL_CUDA(cudaGetLastError());
     if (d0.bv_type == DIPL_BV_SOBB) {
         SobbRefs refs;
@@ -2787,15 +2846,12 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
                           (int)N, (int)K, P.L, d0.kdop_size, P.sobb, refs, P.snodes, stream, P.d_err);
         if (st != DIPL_OK) return st;
     }
-    // ---- the per-mesh summary to pinned host memory --------------------------------------------------
-    RootInfo* h_roots = reinterpret_cast<RootInfo*>(P.h_summary);
-    double* h_sah = reinterpret_cast<double*>(P.h_summary + sizeof(RootInfo) * m);
-    uint32_t* h_tail = reinterpret_cast<uint32_t*>(P.h_summary + sizeof(RootInfo) * m + sizeof(double) * 2 * m);
-    DIPL_CUDA(cudaMemcpyAsync(h_roots, P.d_roots, sizeof(RootInfo) * m, cudaMemcpyDeviceToHost, stream));
-    DIPL_CUDA(cudaMemcpyAsync(h_sah, P.d_sah, sizeof(double) * 2 * m, cudaMemcpyDeviceToHost, stream));
-    DIPL_CUDA(cudaMemcpyAsync(h_tail, P.d_counts, 4, cudaMemcpyDeviceToHost, stream));
-    DIPL_CUDA(cudaMemcpyAsync(h_tail + 1, &P.d_ctrl->iterations, 4, cudaMemcpyDeviceToHost, stream));
-    DIPL_CUDA(cudaMemcpyAsync(h_tail + 2, P.d_err, 4, cudaMemcpyDeviceToHost, stream));
+    // ---- the per-mesh summary, last (it holds the error word), to pinned host memory ------------------------------
+    roots_kernel<<<blocks_for(m, 64), 64, 0, stream>>>(LP, P.c_lo[0], P.c_hi[0], P.c_lo[1], P.c_hi[1], P.d_ctrl, hier, m,
+                                                       P.rev_flags, P.leaf_start_of, P.d_roots, P.d_counts, P.d_err);
+    note_launches();
+    DIPL_CUDA(cudaGetLastError());
+    DIPL_CUDA(cudaMemcpyAsync(P.h_summary, P.d_summary, P.summary_bytes, cudaMemcpyDeviceToHost, stream));
     return DIPL_OK;
 }
 
@@ -2834,8 +2890,6 @@ static dipl_status plan_finish(BuildPlan& P, dipl_bvh** out, bool allow_wide) {
     }
     const int64_t inner_total = (int64_t)h_tail[0];
     const int iterations = (int)h_tail[1];
-    WNode* wnodes = nullptr;
-    float4* wtris = nullptr;
     int64_t wcount = 0;
     std::vector<int> wroots, wlevels;
     if (d0.layout == DIPL_LAYOUT_WIDE8_Q8) {
@@ -2846,7 +2900,7 @@ static dipl_status plan_finish(BuildPlan& P, dipl_bvh** out, bool allow_wide) {
         std::vector<int> root_ids(m), root_counts(m);
         for (int k = 0; k < m; ++k) root_ids[k] = h_roots[k].root_id, root_counts[k] = h_roots[k].num_leaves;
         dipl_status st = build_wide(P.child, P.nlo, P.nhi, P.leaf_start_of, P.tris, (int)P.N, P.L, root_ids,
-                                    root_counts, *P.out, P.stream, P.d_err, &wnodes, &wtris, &wcount, wroots, wlevels);
+                                    root_counts, P.wide, P.stream, P.d_err, &wcount, wroots, wlevels);
         if (st != DIPL_OK) return st;
     }
     for (int i = 0; i < P.count; ++i) {
@@ -2879,8 +2933,8 @@ static dipl_status plan_finish(BuildPlan& P, dipl_bvh** out, bool allow_wide) {
             }
         }
         if (d0.layout == DIPL_LAYOUT_WIDE8_Q8) {
-            h->nodes = wnodes;
-            h->tris = wtris;
+            h->nodes = P.wide.nodes;
+            h->tris = P.wide.tris;
             h->node_size = sizeof(WNode);
             h->node_capacity = wcount;
             h->num_nodes = wcount;

@@ -2,8 +2,10 @@
 #pragma once
 
 #include <algorithm>
+#include <cstring>
 #include <memory>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -39,23 +41,26 @@ int probe_per_device(DeviceProbe& p, F&& probe) {
 // ---- sort ----------------------------------------------------------------------------------------
 size_t radix_sort_scratch_bytes(int64_t n, int begin_bit, int end_bit, int digit_bits);
 bool radix_sort_bits_ok(int begin_bit, int end_bit, int digit_bits);
+// `cleared`: the scratch is zero already (all radix_sort_scratch_bytes of it).
 dipl_status radix_sort_pairs(const void* kin, const uint32_t* vin, void* kout, uint32_t* vout, void* kalt,
                              uint32_t* valt, int64_t n, int key_bytes, int begin_bit, int end_bit, int digit_bits,
-                             void* scratch, cudaStream_t stream, uint32_t* d_err);
+                             void* scratch, cudaStream_t stream, uint32_t* d_err, bool cleared = false);
 
 // ---- scan ----------------------------------------------------------------------------------------
 size_t scan_scratch_bytes(int64_t n);
 // Exclusive prefix sum of n uint32 values (in and out may alias); optional total written to d_total.
+// `cleared`: the scratch is zero already.
 dipl_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* d_total, void* scratch,
-                               cudaStream_t stream, uint32_t* d_err);
+                               cudaStream_t stream, uint32_t* d_err, bool cleared = false);
 
 // ---- device memory -------------------------------------------------------------------------------
-// Stream-ordered allocation from the device's default pool (kept warm: release threshold raised once).
+// Stream-ordered allocation from the device's default pool (kept warm: release threshold raised once), or with `kept`
+// from the library's pool of the arrays that handles keep.
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
 };
-dipl_status device_alloc(void** ptr, size_t bytes, cudaStream_t stream);
+dipl_status device_alloc(void** ptr, size_t bytes, cudaStream_t stream, bool kept = false);
 void device_free(void* ptr, cudaStream_t stream);
 
 // Process-wide limits set by dipl_set_limits (0 = the built-in bound).
@@ -85,22 +90,44 @@ class ScratchArena {
 };
 
 // ---- the BVH handle ------------------------------------------------------------------------------
-// Device memory of one build; shared by the handles of a batched build.
+// Device memory of one build; shared by the handles of a batched build. Arrays are asked for with reserve() and made by
+// commit() in one allocation, so a build takes two blocks (what the handles keep, scratch) instead of about forty: 40 us
+// of a small build's 380. Block sizes are rounded up to a sixteenth of their power of two, so that builds of nearly the
+// same size reuse each other's blocks. With blocks of many sizes in one pool, three 16M-triangle handles rebuilt in turn
+// took 30 to 62 ms a build and trace, half of it mapping memory; two blocks from two pools: 20 ms.
 struct Storage {
     std::vector<void*> ptrs;
     cudaStream_t stream = nullptr;
+    bool kept = false;  // what a handle keeps: from the pool of those
     ~Storage() {
         for (void* p : ptrs) device_free(p, stream);
     }
     template <typename T>
-    dipl_status alloc(T** out, size_t count) {
-        void* p = nullptr;
-        dipl_status st = device_alloc(&p, std::max<size_t>(count * sizeof(T), 16), stream);
-        if (st != DIPL_OK) return st;
-        ptrs.push_back(p);
-        *out = static_cast<T*>(p);
-        return DIPL_OK;
+    void reserve(T** out, size_t count) {
+        want_.push_back({static_cast<void*>(out), total_});
+        total_ += (std::max<size_t>(count * sizeof(T), 16) + 255) & ~size_t(255);
     }
+    dipl_status commit() {
+        if (want_.empty()) return DIPL_OK;
+        size_t unit = 256;
+        while (unit * 32 <= total_) unit *= 2;  // total_ / 32 < unit: at most 16 to 32 units
+        void* p = nullptr;
+        dipl_status st = device_alloc(&p, (total_ + unit - 1) / unit * unit, stream, kept);
+        if (st == DIPL_OK) {
+            ptrs.push_back(p);
+            for (const auto& w : want_) {
+                void* at = static_cast<char*>(p) + w.second;
+                std::memcpy(w.first, &at, sizeof(at));
+            }
+        }
+        want_.clear();
+        total_ = 0;
+        return st;
+    }
+
+   private:
+    std::vector<std::pair<void*, size_t>> want_;  // where each pointer goes, its offset
+    size_t total_ = 0;
 };
 
 }  // namespace dipl
@@ -176,12 +203,20 @@ dipl_status trace_adjoint(const float* v0, const float* v1, const float* v2, con
                           const dipl_hit* hits, const float* dtuv, int64_t n, float* dv0, float* dv1, float* dv2,
                           float* dorig, float* ddir, cudaStream_t stream);
 
-// Precision form (wide.cu): 8-wide quantised layout built from the binary clustering, and its traversal.
+// Precision form (wide.cu): 8-wide quantised layout built from the binary clustering, and its traversal. Arrays of one
+// layout build: the kept nodes and triangles, and scratch for `capacity` nodes.
+struct WideScratch {
+    WNode* nodes = nullptr;
+    float4* tris = nullptr;
+    int *front[2] = {nullptr, nullptr}, *kids = nullptr;
+    uint32_t *ninner = nullptr, *ntris = nullptr, *totals = nullptr;
+    unsigned char* scan = nullptr;
+};
+void wide_reserve(WideScratch& w, Storage& work, int64_t capacity);
 dipl_status build_wide(const int4* child, const float4* node_lo, const float4* node_hi, const int* leaf_start_of,
                        const float4* btris, int N, int L, const std::vector<int>& root_ids,
-                       const std::vector<int>& root_counts, Storage& storage, cudaStream_t s, uint32_t* d_err,
-                       WNode** out_nodes, float4** out_tris, int64_t* out_num_nodes, std::vector<int>& out_root_refs,
-                       std::vector<int>& out_levels);
+                       const std::vector<int>& root_counts, const WideScratch& w, cudaStream_t s, uint32_t* d_err,
+                       int64_t* out_num_nodes, std::vector<int>& out_root_refs, std::vector<int>& out_levels);
 dipl_status trace_wide(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ, int leaf_test,
                        uint32_t flags, unsigned long long* counters, bool any, cudaStream_t s);
 
@@ -199,7 +234,7 @@ struct SobbRefs {
     const uint32_t* perm = nullptr;
     const float4* rbox = nullptr;
 };
-dipl_status sobb_prepare(long long N, long long K, Storage& work, Storage& out, SobbScratch* sc, SNode** snodes);
+dipl_status sobb_prepare(long long N, long long K, Storage& work, SobbScratch* sc);
 dipl_status sobb_enqueue(const int4* child, const float4* node_lo, const float4* node_hi, const int* parent,
                          const int* leaf_start_of, const int* owner_leaf, const float4* btris, const BNode* bnodes,
                          const uint32_t* rev_index, int N, int K, int L, int kdop_size, const SobbScratch& sc,

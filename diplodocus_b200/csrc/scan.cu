@@ -78,7 +78,7 @@ size_t scan_scratch_bytes(int64_t n) {
 }
 
 dipl_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* d_total, void* scratch,
-                               cudaStream_t stream, uint32_t* d_err) {
+                               cudaStream_t stream, uint32_t* d_err, bool cleared) {
     if (n <= 0) {
         if (d_total) DIPL_CUDA(cudaMemsetAsync(d_total, 0, 4, stream));
         return DIPL_OK;
@@ -86,7 +86,7 @@ dipl_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uin
     int64_t tiles = (n + kScanTile - 1) / kScanTile;
     auto* counter = static_cast<uint32_t*>(scratch);
     auto* status = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(scratch) + 64);
-    DIPL_CUDA(cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), stream));
+    if (!cleared) DIPL_CUDA(cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), stream));
     scan_kernel<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, out, n, status, counter, d_total, d_err); note_launches();
     DIPL_CUDA(cudaGetLastError());
     return DIPL_OK;

@@ -702,19 +702,15 @@ dipl_status upload_triples() {
 }  // namespace
 
 // Allocations of the SOBB refit (and the one-time upload of the direction triples).
-dipl_status sobb_prepare(long long N, long long K, Storage& work, Storage& out, SobbScratch* sc, SNode** snodes) {
-    dipl_status st = DIPL_OK;
+dipl_status sobb_prepare(long long N, long long K, Storage& work, SobbScratch* sc) {
     if (!probe_per_device(g_triples_uploaded, [] { return upload_triples() == DIPL_OK ? 1 : 0; })) {
         set_last_error("SOBB: upload of the direction-triple table failed");
         return DIPL_ERR_CUDA;
     }
     const long long Kalloc = std::max<long long>(K, 1);
-    Kdop* kdop;
-    if ((st = work.alloc(&kdop, (size_t)(N + Kalloc))) != DIPL_OK ||
-        (st = work.alloc(&sc->mag, (size_t)(N + Kalloc))) != DIPL_OK ||
-        (st = work.alloc(&sc->arrivals, (size_t)Kalloc)) != DIPL_OK || (st = out.alloc(snodes, (size_t)Kalloc)) != DIPL_OK)
-        return st;
-    sc->kdop = kdop;
+    work.reserve(reinterpret_cast<Kdop**>(&sc->kdop), (size_t)(N + Kalloc));
+    work.reserve(&sc->mag, (size_t)(N + Kalloc));
+    work.reserve(&sc->arrivals, (size_t)Kalloc);
     sc->triples = g_triples;
     return DIPL_OK;
 }

@@ -224,7 +224,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) onesweep_kernel(
 
 template <typename K, int BITS>
 dipl_status sort_impl(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, K* kalt, uint32_t* valt, int64_t n,
-                      int begin_bit, int end_bit, unsigned char* scratch, cudaStream_t stream, uint32_t* d_err) {
+                      int begin_bit, int end_bit, unsigned char* scratch, cudaStream_t stream, uint32_t* d_err,
+                      bool cleared) {
     constexpr int BINS = 1 << BITS;
     const int passes = (end_bit - begin_bit + BITS - 1) / BITS;
     const int64_t tiles = (n + kSortTile - 1) / kSortTile;
@@ -232,7 +233,7 @@ dipl_status sort_impl(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout
     uint32_t* counters = hist + kMaxPasses * 1024;
     uint32_t* lookback = counters + 64;
     size_t clear = (size_t)(kMaxPasses * 1024 + 64) * 4 + (size_t)passes * tiles * BINS * 4;
-    DIPL_CUDA(cudaMemsetAsync(scratch, 0, clear, stream));
+    if (!cleared) DIPL_CUDA(cudaMemsetAsync(scratch, 0, clear, stream));
 
     const size_t hsmem = (size_t)passes * BINS * 4;
     int hblocks = (int)std::min<int64_t>((n + 255) / 256, 148 * 8);
@@ -267,12 +268,12 @@ dipl_status sort_impl(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout
 template <typename K>
 dipl_status sort_dispatch(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, K* kalt, uint32_t* valt,
                           int64_t n, int begin_bit, int end_bit, int bits, unsigned char* scratch, cudaStream_t s,
-                          uint32_t* err) {
+                          uint32_t* err, bool cleared) {
     switch (bits) {
-        case 6: return sort_impl<K, 6>(kin, vin, kout, vout, kalt, valt, n, begin_bit, end_bit, scratch, s, err);
-        case 7: return sort_impl<K, 7>(kin, vin, kout, vout, kalt, valt, n, begin_bit, end_bit, scratch, s, err);
-        case 8: return sort_impl<K, 8>(kin, vin, kout, vout, kalt, valt, n, begin_bit, end_bit, scratch, s, err);
-        case 10: return sort_impl<K, 10>(kin, vin, kout, vout, kalt, valt, n, begin_bit, end_bit, scratch, s, err);
+        case 6: return sort_impl<K, 6>(kin, vin, kout, vout, kalt, valt, n, begin_bit, end_bit, scratch, s, err, cleared);
+        case 7: return sort_impl<K, 7>(kin, vin, kout, vout, kalt, valt, n, begin_bit, end_bit, scratch, s, err, cleared);
+        case 8: return sort_impl<K, 8>(kin, vin, kout, vout, kalt, valt, n, begin_bit, end_bit, scratch, s, err, cleared);
+        case 10: return sort_impl<K, 10>(kin, vin, kout, vout, kalt, valt, n, begin_bit, end_bit, scratch, s, err, cleared);
         default: set_last_error("sort digit width must be 6, 7, 8 or 10"); return DIPL_ERR_INVALID_ARGUMENT;
     }
 }
@@ -295,18 +296,18 @@ bool radix_sort_bits_ok(int begin_bit, int end_bit, int digit_bits) {
 
 dipl_status radix_sort_pairs(const void* kin, const uint32_t* vin, void* kout, uint32_t* vout, void* kalt,
                              uint32_t* valt, int64_t n, int key_bytes, int begin_bit, int end_bit, int digit_bits,
-                             void* scratch, cudaStream_t stream, uint32_t* d_err) {
+                             void* scratch, cudaStream_t stream, uint32_t* d_err, bool cleared) {
     if (n <= 0) return DIPL_OK;
     int bits = digit_bits > 0 ? digit_bits : 8;
     auto* sc = static_cast<unsigned char*>(scratch);
     if (key_bytes == 4)
         return sort_dispatch<uint32_t>(static_cast<const uint32_t*>(kin), vin, static_cast<uint32_t*>(kout), vout,
                                        static_cast<uint32_t*>(kalt), valt, n, begin_bit, end_bit, bits, sc, stream,
-                                       d_err);
+                                       d_err, cleared);
     return sort_dispatch<unsigned long long>(static_cast<const unsigned long long*>(kin), vin,
                                              static_cast<unsigned long long*>(kout), vout,
                                              static_cast<unsigned long long*>(kalt), valt, n, begin_bit, end_bit,
-                                             bits, sc, stream, d_err);
+                                             bits, sc, stream, d_err, cleared);
 }
 
 }  // namespace dipl

@@ -670,30 +670,31 @@ dipl_status launch_wide_stack(const dipl_bvh* b, const dipl_ray* rays, int64_t n
 
 }  // namespace
 
+void wide_reserve(WideScratch& w, Storage& work, int64_t capacity) {
+    work.reserve(&w.front[0], capacity);
+    work.reserve(&w.front[1], capacity);
+    work.reserve(&w.kids, 8 * (size_t)capacity);
+    work.reserve(&w.ninner, capacity);
+    work.reserve(&w.ntris, capacity);
+    work.reserve(&w.totals, 4);
+    work.reserve(&w.scan, scan_scratch_bytes(capacity));
+}
+
 // Builds the wide layout of every mesh of a batch from the binary PLOC tree. root_ids[k] = PLOC node id of
-// mesh k's root, root_counts[k] its triangle count. Outputs the wide nodes/triangles (in `storage`), each
-// mesh's root reference (wide node index or leaf reference), the number of wide levels per mesh, and the
-// node count.
+// mesh k's root, root_counts[k] its triangle count. Fills w.nodes and w.tris; outputs each mesh's root reference (wide
+// node index or leaf reference), the number of wide levels per mesh, and the node count.
 dipl_status build_wide(const int4* child, const float4* node_lo, const float4* node_hi, const int* leaf_start_of,
                        const float4* btris, int N, int L, const std::vector<int>& root_ids,
-                       const std::vector<int>& root_counts, Storage& storage, cudaStream_t s, uint32_t* d_err,
-                       WNode** out_nodes, float4** out_tris, int64_t* out_num_nodes, std::vector<int>& out_root_refs,
-                       std::vector<int>& out_levels) {
+                       const std::vector<int>& root_counts, const WideScratch& w, cudaStream_t s, uint32_t* d_err,
+                       int64_t* out_num_nodes, std::vector<int>& out_root_refs, std::vector<int>& out_levels) {
     const int m = (int)root_ids.size();
     const int K = std::max(N - m, 1);
-    ScratchArena scratch(s);
-    WNode* nodes;
-    float4* tris;
-    int *front0, *front1, *kids;
-    uint32_t *ninner, *ntris, *totals;
-    unsigned char* scan_scratch;
+    WNode* const nodes = w.nodes;
+    float4* const tris = w.tris;
+    int *const front0 = w.front[0], *const front1 = w.front[1], *const kids = w.kids;
+    uint32_t *const ninner = w.ninner, *const ntris = w.ntris, *const totals = w.totals;
+    unsigned char* const scan_scratch = w.scan;
     dipl_status st;
-    if ((st = storage.alloc(&nodes, K)) != DIPL_OK || (st = storage.alloc(&tris, 3 * (size_t)std::max(N, 1))) != DIPL_OK ||
-        (st = scratch.alloc(&front0, K)) != DIPL_OK || (st = scratch.alloc(&front1, K)) != DIPL_OK ||
-        (st = scratch.alloc(&kids, 8 * (size_t)K)) != DIPL_OK || (st = scratch.alloc(&ninner, K)) != DIPL_OK ||
-        (st = scratch.alloc(&ntris, K)) != DIPL_OK || (st = scratch.alloc(&totals, 4)) != DIPL_OK ||
-        (st = scratch.alloc(&scan_scratch, scan_scratch_bytes(K))) != DIPL_OK)
-        return st;
     WideIn W{child, node_lo, node_hi, leaf_start_of, btris, N, L};
     out_root_refs.assign(m, 0);
     out_levels.assign(m, 0);
@@ -751,8 +752,6 @@ dipl_status build_wide(const int4* child, const float4* node_lo, const float4* n
         }
     }
     for (int k = 0; k < m; ++k) out_levels[k] = levels;
-    *out_nodes = nodes;
-    *out_tris = tris;
     *out_num_nodes = base;
     return DIPL_OK;
 }
