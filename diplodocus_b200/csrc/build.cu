@@ -31,7 +31,6 @@ struct CodeParams {
     float lo[4];
     float s[4];
     unsigned long long top[4];
-    unsigned long long mask[4];
     int bits[4];
     // EMC60: dep[a][c][v] = the bits of nibble v of dimension a's cell index, chunk c (bits 4c..4c+3),
     // deposited at their code positions, so a code is an OR of table entries instead of a bit loop.
@@ -222,69 +221,68 @@ __device__ __forceinline__ unsigned long long deposit_bits(unsigned long long va
     return out;
 }
 
-// One thread per mesh: Morton30 scales, or the EMC60 bit plan (60 positions MSB first, each to the
-// dimension x, y, z, size with the largest remaining extent, which is then halved).
-__global__ void code_params_kernel(const Bounds* __restrict__ bounds, int m, int code_type, CodeParams* out) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m) return;
-    float cmin[3], cmax[3], bmin[3], bmax[3];
-    for (int a = 0; a < 3; ++a) {
-        cmin[a] = ordered_to_float(bounds[k].v[a]);
-        cmax[a] = ordered_to_float(bounds[k].v[3 + a]);
-        bmin[a] = ordered_to_float(bounds[k].v[6 + a]);
-        bmax[a] = ordered_to_float(bounds[k].v[9 + a]);
-    }
-    CodeParams p;  // scalar fields only; the deposit tables are written to out[k] directly
-    if (code_type == DIPL_CODE_MORTON30) {
+// One block per mesh: Morton30 scales, or the EMC60 bit plan (60 positions MSB first, each to the dimension x, y, z, size
+// with the largest remaining extent, which is then halved) and its deposit tables, an entry per (dimension, chunk, nibble).
+// The plan is a serial chain of 60 steps, kept in registers (indexed arrays took 11 us of it).
+__global__ void __launch_bounds__(256) code_params_kernel(const Bounds* __restrict__ bounds, int code_type,
+                                                          CodeParams* __restrict__ out) {
+    CodeParams& p = out[blockIdx.x];
+    __shared__ unsigned long long s_mask[4];
+    if (threadIdx.x == 0) {
+        const Bounds& b = bounds[blockIdx.x];
+        float cmin[3], cmax[3], bmin[3], bmax[3];
+#pragma unroll
         for (int a = 0; a < 3; ++a) {
-            float ext = __fsub_rn(cmax[a], cmin[a]);
-            p.lo[a] = cmin[a];
-            p.s[a] = ext > 0.0f ? __fdiv_rn(1024.0f, ext) : 0.0f;
-            p.bits[a] = 10;
-            p.top[a] = 1023;
-            p.mask[a] = 0;
+            cmin[a] = ordered_to_float(b.v[a]);
+            cmax[a] = ordered_to_float(b.v[3 + a]);
+            bmin[a] = ordered_to_float(b.v[6 + a]);
+            bmax[a] = ordered_to_float(b.v[9 + a]);
         }
-        p.lo[3] = 0.0f, p.s[3] = 0.0f, p.bits[3] = 0, p.top[3] = 0, p.mask[3] = 0;
-    } else {
-        float dx = __fsub_rn(bmax[0], bmin[0]), dy = __fsub_rn(bmax[1], bmin[1]), dz = __fsub_rn(bmax[2], bmin[2]);
-        float diag = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
-        float ext[4] = {__fsub_rn(cmax[0], cmin[0]), __fsub_rn(cmax[1], cmin[1]), __fsub_rn(cmax[2], cmin[2]), diag};
-        float e[4];
-        for (int a = 0; a < 4; ++a) {
-            e[a] = ext[a] > 0.0f ? ext[a] : 0.0f;
-            p.bits[a] = 0;
-            p.mask[a] = 0;
-        }
-        for (int pos = 59; pos >= 0; --pos) {
-            int best = 0;
-            for (int a = 1; a < 4; ++a)
-                if (e[a] > e[best]) best = a;
-            p.bits[best] += 1;
-            p.mask[best] |= 1ull << pos;
-            e[best] = __fmul_rn(e[best], 0.5f);
-        }
-        for (int a = 0; a < 4; ++a) {
-            float cells = ldexpf(1.0f, p.bits[a]);
-            p.lo[a] = a < 3 ? cmin[a] : 0.0f;
-            p.s[a] = (ext[a] > 0.0f && p.bits[a] > 0) ? __fdiv_rn(cells, ext[a]) : 0.0f;
-            p.top[a] = p.bits[a] >= 64 ? ~0ull : ((1ull << p.bits[a]) - 1ull);
+        if (code_type == DIPL_CODE_MORTON30) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float ext = __fsub_rn(cmax[a], cmin[a]);
+                p.lo[a] = cmin[a];
+                p.s[a] = ext > 0.0f ? __fdiv_rn(1024.0f, ext) : 0.0f;
+                p.bits[a] = 10;
+                p.top[a] = 1023;
+            }
+            p.lo[3] = 0.0f, p.s[3] = 0.0f, p.bits[3] = 0, p.top[3] = 0;
+        } else {
+            const float dx = __fsub_rn(bmax[0], bmin[0]), dy = __fsub_rn(bmax[1], bmin[1]), dz = __fsub_rn(bmax[2], bmin[2]);
+            const float diag = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+            const float ext[4] = {__fsub_rn(cmax[0], cmin[0]), __fsub_rn(cmax[1], cmin[1]), __fsub_rn(cmax[2], cmin[2]), diag};
+            float e[4];
+            unsigned long long mask[4] = {0ull, 0ull, 0ull, 0ull};
+            int bits[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int a = 0; a < 4; ++a) e[a] = ext[a] > 0.0f ? ext[a] : 0.0f;
+            for (unsigned long long bit = 1ull << 59; bit != 0ull; bit >>= 1) {
+                int best = 0;
+                float eb = e[0];
+#pragma unroll
+                for (int a = 1; a < 4; ++a)
+                    if (e[a] > eb) best = a, eb = e[a];
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+                    if (a == best) bits[a] += 1, mask[a] |= bit, e[a] = __fmul_rn(e[a], 0.5f);
+            }
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const float cells = ldexpf(1.0f, bits[a]);
+                p.lo[a] = a < 3 ? cmin[a] : 0.0f;
+                p.s[a] = (ext[a] > 0.0f && bits[a] > 0) ? __fdiv_rn(cells, ext[a]) : 0.0f;
+                p.top[a] = (1ull << bits[a]) - 1ull;
+                p.bits[a] = bits[a];
+                s_mask[a] = mask[a];
+            }
         }
     }
-    for (int a = 0; a < 4; ++a) {
-        out[k].lo[a] = p.lo[a];
-        out[k].s[a] = p.s[a];
-        out[k].top[a] = p.top[a];
-        out[k].mask[a] = p.mask[a];
-        out[k].bits[a] = p.bits[a];
-    }
-}
-
-// EMC60 deposit tables of every mesh: one block per mesh, one thread per (dimension, chunk, nibble) entry.
-__global__ void __launch_bounds__(256) emc_tables_kernel(CodeParams* params) {
-    CodeParams& p = params[blockIdx.x];
+    if (code_type == DIPL_CODE_MORTON30) return;
+    __syncthreads();
     for (int e = threadIdx.x; e < 4 * 16 * 16; e += blockDim.x) {
         const int a = e >> 8, c = (e >> 4) & 15, v = e & 15;
-        p.dep[a][c][v] = deposit_bits((unsigned long long)v << (4 * c), p.mask[a]);
+        p.dep[a][c][v] = deposit_bits((unsigned long long)v << (4 * c), s_mask[a]);
     }
 }
 
@@ -381,24 +379,37 @@ __device__ __forceinline__ float mesh_diag(const Bounds& b) {
     return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(e[0], e[0]), __fmul_rn(e[1], e[1])), __fmul_rn(e[2], e[2])));
 }
 
+// Integer sums are exact in any order. A block walks a contiguous run of triangles: one atomic per block while the run
+// lies in one mesh (one per warp of 32 triangles took 413 us for 16M, all on one address; 100 us now), else one per thread and mesh.
 __global__ void __launch_bounds__(256) split_weight_kernel(const MeshDesc* __restrict__ meshes,
                                                            const long long* __restrict__ offsets, int m, long long n,
-                                                           const Bounds* __restrict__ bounds,
+                                                           long long chunk, const Bounds* __restrict__ bounds,
                                                            unsigned long long* __restrict__ mesh_sum) {
-    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long beg = blockIdx.x * chunk, end = min(n, beg + chunk);
+    if (beg >= end) return;
+    const int m_first = find_mesh(offsets, m, beg), m_last = find_mesh(offsets, m, end - 1);
     unsigned long long q = 0ull;
-    int k = 0;
-    if (g < n) {
-        k = find_mesh(offsets, m, g);
-        q = split_weight(load_tri(meshes[k], g - meshes[k].first), mesh_diag(bounds[k]));
+    int cur = m_first;
+    float diag = mesh_diag(bounds[cur]);
+    for (long long g = beg + threadIdx.x; g < end; g += blockDim.x) {
+        const int k = m_first == m_last ? m_first : find_mesh(offsets, m, g);
+        if (k != cur) {
+            if (q) atomicAdd(mesh_sum + cur, q);
+            q = 0ull, cur = k, diag = mesh_diag(bounds[k]);
+        }
+        q += split_weight(load_tri(meshes[k], g - meshes[k].first), diag);
     }
-    // integer sums are exact in any order: one atomic per warp when the warp lies in one mesh, else one per thread
-    const int k0 = __shfl_sync(0xffffffffu, k, 0);
-    if (__all_sync(0xffffffffu, k == k0)) {
-        for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-        if ((threadIdx.x & 31) == 0 && q) atomicAdd(mesh_sum + k0, q);
-    } else if (q) {
-        atomicAdd(mesh_sum + k, q);
+    if (m_first != m_last) {
+        if (q) atomicAdd(mesh_sum + cur, q);
+        return;
+    }
+    __shared__ unsigned long long s_q[8];
+    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    if ((threadIdx.x & 31) == 0) s_q[threadIdx.x >> 5] = q;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) q += s_q[w];
+        if (q) atomicAdd(mesh_sum + m_first, q);
     }
 }
 
@@ -499,13 +510,18 @@ __global__ void __launch_bounds__(256) ref_tri_kernel(long long n, const uint32_
     for (uint32_t i = 0; i < c; ++i) ref_tri[r + i] = (int)g;
 }
 
-// One thread per reference: its box and its code. An unsplit triangle's reference takes the triangle's box and
-// codes exactly as codes_kernel; piece j of a triangle split into c pieces follows its own path of halvings from
-// the triangle's box: a box of c pieces is cut at the midpoint of its longest axis, the lower half takes the
-// first ceil(c/2) pieces and the upper half the rest, and each half's box comes from split_half. The
-// pieces of one triangle are the leaves of that binary recursion in depth-first order (lower half first), and
-// every box is computed with the same operations whichever thread computes it. A piece codes by the centre and
-// the diagonal of its box.
+// Every reference's box and code. An unsplit triangle's reference takes the triangle's box and codes exactly as
+// codes_kernel; piece j of a triangle split into c pieces follows its own path of halvings from the triangle's box: a
+// box of c pieces is cut at the midpoint of its longest axis, the lower half takes the first ceil(c/2) pieces and the
+// upper half the rest, and each half's box comes from split_half. The pieces of one triangle are the leaves of that
+// binary recursion in depth-first order (lower half first), and every box is computed with the same operations
+// whichever thread computes it. A piece codes by the centre and the diagonal of its box.
+//
+// A block takes kSplitRefs references: first the unsplit ones (and the list of pieces), then the pieces, one per
+// thread, so that a warp's lanes all clip. With one thread per reference in order nearly every warp held a piece and
+// waited for its halvings with most lanes idle: 1.46 ms for the 16M soup's 20.3M references, 1.07 ms now.
+constexpr int kSplitRefs = 1024;
+
 template <typename K>
 __global__ void __launch_bounds__(kSplitThreads) split_refs_kernel(const MeshDesc* __restrict__ meshes,
                                                                    const long long* __restrict__ offsets, int m,
@@ -516,18 +532,47 @@ __global__ void __launch_bounds__(kSplitThreads) split_refs_kernel(const MeshDes
                                                                    int code_type, int code_shift, int mesh_shift,
                                                                    float4* __restrict__ rbox, K* __restrict__ keys) {
     __shared__ float s_poly[2 * kPolyMax * 3 * kSplitThreads];
-    const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (r >= n_refs) return;
-    const long long g = ref_tri[r];
-    const int k = find_mesh(offsets, m, g);
-    const Tri t = load_tri(meshes[k], g - meshes[k].first);
-    int c = (int)pieces[g];
-    float3 blo, bhi;
-    tri_box(t, blo, bhi);
-    unsigned long long code;
-    if (c == 1) {
-        code = tri_code(t, params[k], code_type);
-    } else {
+    __shared__ unsigned short s_list[kSplitRefs];
+    __shared__ int s_count;
+    const long long r0 = blockIdx.x * (long long)kSplitRefs;
+    auto write = [&](long long r, int k, const float3& lo, const float3& hi, unsigned long long code) {
+        rbox[2 * r] = make_float4(lo.x, lo.y, lo.z, 0.0f);
+        rbox[2 * r + 1] = make_float4(hi.x, hi.y, hi.z, 0.0f);
+        code >>= code_shift;
+        if (mesh_shift > 0) code |= (unsigned long long)k << mesh_shift;
+        keys[r] = static_cast<K>(code);
+    };
+    if (threadIdx.x == 0) s_count = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < kSplitRefs; i += kSplitThreads) {
+        const long long r = r0 + i;
+        bool piece = false;
+        if (r < n_refs) {
+            const long long g = ref_tri[r];
+            piece = pieces[g] > 1u;
+            if (!piece) {
+                const int k = find_mesh(offsets, m, g);
+                const Tri t = load_tri(meshes[k], g - meshes[k].first);
+                float3 lo, hi;
+                tri_box(t, lo, hi);
+                write(r, k, lo, hi, tri_code(t, params[k], code_type));
+            }
+        }
+        const unsigned pm = __ballot_sync(0xffffffffu, piece);
+        int base = 0;
+        if ((threadIdx.x & 31) == 0 && pm) base = atomicAdd(&s_count, __popc(pm));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (piece) s_list[base + __popc(pm & lanemask_lt())] = (unsigned short)i;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < s_count; q += kSplitThreads) {
+        const long long r = r0 + s_list[q];
+        const long long g = ref_tri[r];
+        const int k = find_mesh(offsets, m, g);
+        const Tri t = load_tri(meshes[k], g - meshes[k].first);
+        int c = (int)pieces[g];
+        float3 blo, bhi;
+        tri_box(t, blo, bhi);
         Poly P{s_poly + threadIdx.x}, Q{s_poly + kPolyMax * 3 * kSplitThreads + threadIdx.x};
         P.at(0, 0) = t.a.x, P.at(0, 1) = t.a.y, P.at(0, 2) = t.a.z;
         P.at(1, 0) = t.b.x, P.at(1, 1) = t.b.y, P.at(1, 2) = t.b.z;
@@ -554,14 +599,10 @@ __global__ void __launch_bounds__(kSplitThreads) split_refs_kernel(const MeshDes
         }
         const float3 ctr = make_float3(__fmul_rn(__fadd_rn(blo.x, bhi.x), 0.5f), __fmul_rn(__fadd_rn(blo.y, bhi.y), 0.5f),
                                        __fmul_rn(__fadd_rn(blo.z, bhi.z), 0.5f));
-        code = point_code(ctr, __fsub_rn(bhi.x, blo.x), __fsub_rn(bhi.y, blo.y), __fsub_rn(bhi.z, blo.z), params[k],
-                          code_type);
+        write(r, k, blo, bhi,
+              point_code(ctr, __fsub_rn(bhi.x, blo.x), __fsub_rn(bhi.y, blo.y), __fsub_rn(bhi.z, blo.z), params[k],
+                         code_type));
     }
-    rbox[2 * r] = make_float4(blo.x, blo.y, blo.z, 0.0f);
-    rbox[2 * r + 1] = make_float4(bhi.x, bhi.y, bhi.z, 0.0f);
-    code >>= code_shift;
-    if (mesh_shift > 0) code |= (unsigned long long)k << mesh_shift;
-    keys[r] = static_cast<K>(code);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1825,21 +1866,30 @@ __global__ void inner_flags_kernel(LayoutParams P, uint32_t* __restrict__ rev_fl
     rev_flags[P.num_inner - 1 - k] = f;
 }
 
-// Inner-node numbering by height (hierarchical clustering): sort keys, then each inner node's traced index is its
-// rank, stored where the reverse-order consumers read it (rev_index[num_inner - 1 - k]).
-__global__ void height_keys_kernel(LayoutParams P, uint32_t* __restrict__ keys, const uint32_t* err) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= P.num_inner) return;
-    const bool inner = (*err == 0u) && __float_as_int(P.node_lo[k].w) >= P.L;
-    keys[k] = inner ? 254u - (uint32_t)min(max(P.child[k].z, 0), 254) : 255u;
-}
-
-__global__ void height_index_kernel(LayoutParams P, const uint32_t* __restrict__ order, uint32_t* __restrict__ rev_index,
-                                    const uint32_t* err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.num_inner || *err != 0u) return;
-    const int k = (int)order[i];
-    if (__float_as_int(P.node_lo[k].w) >= P.L) rev_index[P.num_inner - 1 - k] = (uint32_t)i;  // inner nodes sort first
+// Inner-node numbering by height (hierarchical clustering): the byte keys, their histogram and the number of inner
+// nodes; each inner node's traced index is its key's rank, written where the reverse-order consumers read it
+// (rev_index[num_inner - 1 - k]). Inner nodes sort first.
+__global__ void __launch_bounds__(256) height_keys_kernel(LayoutParams P, unsigned char* __restrict__ keys,
+                                                          uint32_t* __restrict__ hist, uint32_t* __restrict__ inner,
+                                                          const uint32_t* err) {
+    __shared__ uint32_t s_hist[256];
+    s_hist[threadIdx.x] = 0u;
+    __syncthreads();
+    const bool ok = *err == 0u;
+    for (long long k = blockIdx.x * 256ll + threadIdx.x; k < P.num_inner; k += gridDim.x * 256ll) {
+        const bool in = ok && __float_as_int(P.node_lo[k].w) >= P.L;
+        const uint32_t key = in ? 254u - (uint32_t)min(max(P.child[k].z, 0), 254) : 255u;
+        keys[k] = (unsigned char)key;
+        // most nodes share a few heights: one shared atomic per height of a warp
+        const uint32_t peers = __match_any_sync(__activemask(), key);
+        if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&s_hist[key], (uint32_t)__popc(peers));
+    }
+    __syncthreads();
+    const uint32_t c = s_hist[threadIdx.x];
+    if (c) atomicAdd(&hist[threadIdx.x], c);
+    uint32_t sum = threadIdx.x < 255u ? c : 0u;
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(inner, sum);
 }
 
 __global__ void leaf_owner_kernel(LayoutParams P, uint32_t* __restrict__ contrib, int* __restrict__ owner_leaf,
@@ -2454,7 +2504,9 @@ static dipl_status count_references(BuildPlan& P, cudaStream_t stream) {
     P.d_err = P.d_split_err;
     if ((st = enqueue_bounds_and_params(P, stream)) != DIPL_OK) return st;
     DIPL_CUDA(cudaMemsetAsync(P.mesh_wsum, 0, sizeof(unsigned long long) * m, stream));
-    split_weight_kernel<<<blocks_for(T, 256), 256, 0, stream>>>(P.d_meshes, P.d_offsets, m, T, P.d_bounds, P.mesh_wsum);
+    const long long grid = std::max<long long>(1, std::min<long long>((T + 1023) / 1024, 148 * 16));
+    split_weight_kernel<<<(unsigned)grid, 256, 0, stream>>>(P.d_meshes, P.d_offsets, m, T, (T + grid - 1) / grid,
+                                                            P.d_bounds, P.mesh_wsum);
     note_launches();
     split_count_kernel<<<blocks_for(T, 256), 256, 0, stream>>>(P.d_meshes, P.d_offsets, m, T, P.d_bounds, P.mesh_wsum,
                                                                P.d0.split_budget, P.pieces);
@@ -2697,12 +2749,8 @@ static dipl_status enqueue_bounds_and_params(BuildPlan& P, cudaStream_t stream) 
         bounds_kernel<<<(unsigned)grid, 256, 0, stream>>>(P.d_meshes, P.d_offsets, m, T, chunk, P.d_bounds);
         note_launches();
     }
-    code_params_kernel<<<blocks_for(m, 64), 64, 0, stream>>>(P.d_bounds, m, P.d0.code_type, P.d_params);
+    code_params_kernel<<<(unsigned)m, 256, 0, stream>>>(P.d_bounds, P.d0.code_type, P.d_params);
     note_launches();
-    if (P.d0.code_type == DIPL_CODE_EMC60) {
-        emc_tables_kernel<<<(unsigned)m, 256, 0, stream>>>(P.d_params);
-        note_launches();
-    }
     DIPL_CUDA(cudaGetLastError());
     return DIPL_OK;
 }
@@ -2721,11 +2769,11 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
         ref_tri_kernel<<<blocks_for(P.T, 256), 256, 0, stream>>>(P.T, P.pieces, P.piece_first, P.ref_tri);
         note_launches();
         if (P.key_bytes == 4)
-            split_refs_kernel<uint32_t><<<blocks_for(N, kSplitThreads), kSplitThreads, 0, stream>>>(
+            split_refs_kernel<uint32_t><<<blocks_for(N, kSplitRefs), kSplitThreads, 0, stream>>>(
                 P.d_meshes, P.d_offsets, m, N, P.ref_tri, P.pieces, P.piece_first, P.d_params, d0.code_type,
                 P.code_shift, P.mesh_shift, P.tbox, (uint32_t*)P.keys);
         else
-            split_refs_kernel<unsigned long long><<<blocks_for(N, kSplitThreads), kSplitThreads, 0, stream>>>(
+            split_refs_kernel<unsigned long long><<<blocks_for(N, kSplitRefs), kSplitThreads, 0, stream>>>(
                 P.d_meshes, P.d_offsets, m, N, P.ref_tri, P.pieces, P.piece_first, P.d_params, d0.code_type,
                 P.code_shift, P.mesh_shift, P.tbox, (unsigned long long*)P.keys);
         note_launches();
@@ -2798,27 +2846,23 @@ static dipl_status plan_enqueue(BuildPlan& P, cudaStream_t stream) {
     // ---- layout -------------------------------------------------------------------------------------
     LayoutParams LP{P.child, P.nlo, P.nhi, P.parent, (int)N, (int)K, P.L};
     if (K > 0) {
-        inner_flags_kernel<<<blocks_for(K, 256), 256, 0, stream>>>(LP, P.rev_flags, P.d_err);
-        note_launches();
-        if ((st = exclusive_scan_u32(P.rev_flags, P.rev_flags, K, P.d_counts, P.scan_scratch[0], stream, P.d_err,
-                                     true)) !=
-            DIPL_OK)
-            return st;
         if (hier) {
             // Hierarchical ids follow split positions, so reverse id order would scatter the tree's top levels over
             // the whole node array. Number the inner nodes by height instead, the tallest (the roots) first, ties
             // by id: the top levels every ray visits sit together at the front, as with the global loop's reverse
-            // creation order. A one-pass stable sort of 8-bit keys (255 - height; 255 for nodes inside leaves).
-            uint32_t* hkeys = reinterpret_cast<uint32_t*>(P.keys);
-            uint32_t* hsorted = reinterpret_cast<uint32_t*>(P.keys_sorted);
-            height_keys_kernel<<<blocks_for(K, 256), 256, 0, stream>>>(LP, hkeys, P.d_err);
+            // creation order. Stable ranks of byte keys (254 - height; 255 for nodes inside leaves).
+            unsigned char* hkeys = static_cast<unsigned char*>(P.keys);
+            height_keys_kernel<<<(unsigned)std::min<long long>((K + 255) / 256, 148 * 8), 256, 0, stream>>>(
+                LP, hkeys, byte_rank_histogram(P.height_scratch), P.d_counts, P.d_err);
             note_launches();
             DIPL_CUDA(cudaGetLastError());
-            if ((st = radix_sort_pairs(hkeys, nullptr, hsorted, P.perm_alt, P.keys_alt, P.contrib, K, 4, 0, 8, 8,
-                                       P.height_scratch, stream, P.d_err, true)) != DIPL_OK)
-                return st;
-            height_index_kernel<<<blocks_for(K, 256), 256, 0, stream>>>(LP, P.perm_alt, P.rev_flags, P.d_err);
+            if ((st = byte_ranks_reversed(hkeys, P.rev_flags, K, P.height_scratch, stream, P.d_err)) != DIPL_OK) return st;
+        } else {
+            inner_flags_kernel<<<blocks_for(K, 256), 256, 0, stream>>>(LP, P.rev_flags, P.d_err);
             note_launches();
+            if ((st = exclusive_scan_u32(P.rev_flags, P.rev_flags, K, P.d_counts, P.scan_scratch[0], stream, P.d_err,
+                                         true)) != DIPL_OK)
+                return st;
         }
     }
     leaf_owner_kernel<<<blocks_for(N, 256), 256, 0, stream>>>(LP, P.contrib, P.owner_leaf, P.d_err);
@@ -3061,11 +3105,8 @@ dipl_status compute_codes(const dipl_build_desc* desc, void* d_codes, cudaStream
     long long grid = std::max<long long>(1, std::min<long long>((N + 1023) / 1024, 148 * 16));
     long long chunk = (N + grid - 1) / grid;
     bounds_kernel<<<(unsigned)grid, 256, 0, stream>>>(d_meshes, d_offsets, 1, N, chunk, d_bounds); note_launches();
-    code_params_kernel<<<1, 32, 0, stream>>>(d_bounds, 1, desc->code_type, d_params); note_launches();
-    if (desc->code_type == DIPL_CODE_EMC60) {
-        emc_tables_kernel<<<1, 256, 0, stream>>>(d_params);
-        note_launches();
-    }
+    code_params_kernel<<<1, 256, 0, stream>>>(d_bounds, desc->code_type, d_params);
+    note_launches();
     if (desc->code_type == DIPL_CODE_MORTON30)
         codes_kernel<uint32_t><<<blocks_for(N, 256), 256, 0, stream>>>(d_meshes, d_offsets, 1, N, d_params,
                                                                        desc->code_type, 0, 0, (uint32_t*)d_codes,

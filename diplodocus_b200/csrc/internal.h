@@ -46,6 +46,12 @@ dipl_status radix_sort_pairs(const void* kin, const uint32_t* vin, void* kout, u
                              uint32_t* valt, int64_t n, int key_bytes, int begin_bit, int end_bit, int digit_bits,
                              void* scratch, cudaStream_t stream, uint32_t* d_err, bool cleared = false);
 
+// Stable ranks of byte keys, last key first: ranks[n - 1 - i] = position of keys[i] in the sorted order. The scratch
+// (radix_sort_scratch_bytes(n, 0, 8, 8), zero before) must hold the histogram of the keys at byte_rank_histogram.
+uint32_t* byte_rank_histogram(void* scratch);
+dipl_status byte_ranks_reversed(const unsigned char* keys, uint32_t* ranks, int64_t n, void* scratch, cudaStream_t stream,
+                                uint32_t* d_err);
+
 // ---- scan ----------------------------------------------------------------------------------------
 size_t scan_scratch_bytes(int64_t n);
 // Exclusive prefix sum of n uint32 values (in and out may alias); optional total written to d_total.

