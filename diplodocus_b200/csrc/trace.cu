@@ -13,53 +13,15 @@
 // the best t by more than 1e-5 relative, so a node can never be skipped for rounding of its own box.
 #include <limits>
 
-#include "internal.h"
-#include "intersect.cuh"
+#include "traverse.cuh"
 
 namespace dipl {
 namespace {
 
-constexpr int kTraceThreads = 128;
 // Resident blocks per SM the kernel is compiled for: 9 x 128 threads at <= 56 registers. Builds with more
 // registers and 8 blocks per SM measured up to 1.5x slower on the 16M-triangle soup.
 constexpr int kTraceMinBlocks = 9;
 constexpr float kSlabWiden = 1e-6f;
-constexpr float kPruneSlack = 1e-5f;
-
-struct RayState {
-    float3 o, d, inv;
-    float tmin, tmax;
-};
-
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// One 32-byte read-only load (p must be 32-byte aligned): a 64-byte node in two loads instead of four.
-__device__ __forceinline__ void ldg_v8(const void* p, float4& x, float4& y) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w), "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w)
-        : "l"(p));
-}
-
-__device__ __forceinline__ RayState load_ray(const dipl_ray* rays, int64_t i) {
-    const float4* r4 = reinterpret_cast<const float4*>(rays) + 2 * i;
-    const float4 a = __ldg(r4), b = __ldg(r4 + 1);
-    RayState r;
-    r.o = make_float3(a.x, a.y, a.z);
-    r.d = make_float3(b.x, b.y, b.z);
-    r.tmin = a.w;
-    r.tmax = b.w;
-    // Directions below 1e-20 in magnitude are treated as +-1e-20 so that 1/d stays finite and a ray lying
-    // on a slab plane is still inside it (0 * inf would be NaN). 1/d only feeds the slab tests, which widen
-    // their interval by 1e-6 relative: the hardware reciprocal (relative error below 2^-22) is well inside
-    // that margin.
-    auto safe = [](float x) { return fabsf(x) < 1e-20f ? copysignf(1e-20f, x) : x; };
-    r.inv = make_float3(rcp_approx(safe(r.d.x)), rcp_approx(safe(r.d.y)), rcp_approx(safe(r.d.z)));
-    return r;
-}
 
 // Conservative ray/box interval; returns entry t (or +inf when the box is missed or out of range).
 __device__ __forceinline__ float box_entry(const RayState& r, float lx, float hx, float ly, float hy, float lz, float hz,
@@ -74,8 +36,6 @@ __device__ __forceinline__ float box_entry(const RayState& r, float lx, float hx
     const bool hit = tn <= tf && tf >= r.tmin && tn <= t_limit;
     return hit ? tn : __int_as_float(0x7F800000);
 }
-
-__device__ __forceinline__ float prune_limit(float best_t) { return best_t + fabsf(best_t) * kPruneSlack; }
 
 // Traversal stack of (node reference, entry t). Entries [0, SHORT) live in shared memory, one column per
 // thread (entry k of thread j at sh[k * kTraceThreads + j], so a warp's accesses never share a bank), the rest
@@ -126,15 +86,6 @@ struct TailQueue {
     int max_lanes;
     uint32_t step_limit; // steps one ray may take (both kernels), beyond which it is given up and flagged
 };
-
-// Float bits in an order that compares like the floats (for warp minima).
-__device__ __forceinline__ unsigned ordered_bits(float f) {
-    const unsigned b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float from_ordered_bits(unsigned k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
 
 // Leaf test dispatch: ref_mt or watertight.
 template <int LEAF>
@@ -485,74 +436,24 @@ __global__ void __launch_bounds__(kTraceThreads) tail_kernel(const BNode* __rest
 // all lanes of the warp when few are left. Measured against the binary traversal it replaces (node visits of the
 // pre-split soup 359 -> 192 a ray, L1 cycles 1474 -> 760): 4M-triangle soup, 2M rays in the coherent order 15.2 ->
 // 11.2 ms; 16M soup, 16M rays 127 -> 90 ms; 1M sphere, 4M rays 0.52 -> 0.38 ms; 4096 rays of a small frame 60 -> 28 us.
-constexpr int kQPop = -0x7FFFFFFF - 1;   // next: pop the stack
-constexpr int kQIdle = 0x7FFFFFFF;       // no node
-constexpr float kQMiss = 3.40282346638528859812e+38f;  // entry distance of a child that is not entered
-constexpr int kQShort = 32;              // stack entries per thread in shared memory: 24 with more blocks per SM and
-                                         // 16 were slower (soup 12.2 and 12.9 against 11.3 ms)
-// A warp whose rays have all started shares the last of them among its lanes once at most this many lanes have one
-// (16 and 8 within 1%, 0: 1M sphere 0.63 against 0.37 ms, 64k rays there 152 against 62 us).
-constexpr int kShareLanes = 24;
-constexpr int kLeafTurn = 8;             // lanes that hold a leaf before triangles are tested (1 to 16: within 1%, 24: -5%)
-constexpr int kRefillLanes = 4;          // idle lanes before a persistent warp takes new rays (1: +3%, 16: +10%)
-
-struct QRay {
-    float3 o, d, inv;
-    float tmin;
-};
-
-// False when the ray cannot hit anything under either leaf test: an empty interval, an origin that is not finite or
-// a NaN direction (t then comes out NaN or beyond kInfinity).
-__device__ __forceinline__ bool quad_load_ray(const dipl_ray* rays, int64_t i, QRay& q, float& tmax) {
-    const RayState r = load_ray(rays, i);
-    q.o = r.o, q.d = r.d, q.inv = r.inv, q.tmin = r.tmin;
-    tmax = r.tmax;
-    return r.tmax > r.tmin && isfinite(r.o.x) && isfinite(r.o.y) && isfinite(r.o.z) && !isnan(r.d.x) &&
-           !isnan(r.d.y) && !isnan(r.d.z);
-}
-
-// Traversal stack of references. The first kQShort entries live in shared memory, one column per thread (where the
-// warp's other lanes can read them), the rest in local memory.
-template <int STACK>
-struct QStack {
-    int* column;
-    int rest[STACK - kQShort];
-    int sp = 0;
-    __device__ __forceinline__ void push_short(int ref) { column[sp++ * kTraceThreads] = ref; }
-    __device__ __forceinline__ void push(int ref) {
-        if (sp < kQShort) column[sp * kTraceThreads] = ref;
-        else rest[sp - kQShort] = ref;
-        ++sp;
-    }
-    __device__ __forceinline__ int pop() {
-        --sp;
-        return sp < kQShort ? column[sp * kTraceThreads] : rest[sp - kQShort];
-    }
-};
-
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-__device__ __forceinline__ float min3(float a, float b, float c) {
-    float d;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
+constexpr float kMiss = 3.40282346638528859812e+38f;  // entry distance of a child that is not entered
+// Stack entries per thread in shared memory: 24 with more blocks per SM and 16 were slower (soup 12.2 and 12.9 against
+// 11.3 ms).
+constexpr int kQuadShort = 32;
 
 // Byte k of a plane word as the float 32768 + byte.
 __device__ __forceinline__ float quad_plane(uint32_t w, int k) {
     return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7504u | (uint32_t)(k << 4)));
 }
 
-// The children of a node by entry distance (kQMiss when not entered), nearest first, and their references.
+// The children of a node by entry distance (kMiss when not entered), nearest first, and their references.
 //
 // A plane at p + Q s (Q = 32768 + byte) is met at t = (p - o) / d + Q (s / d). With a = p - o in FP32 and C = a / d
 // the rounding of a and C is at most 2^-23 |C|; near planes move back and far planes on by 2^-22 |C|. What is
 // relative to t (the reciprocal of d, the last FMA) stays below 2e-7 on either side and the final comparison allows
 // 2e-6. A NaN plane (an overflowing product) does not constrain the interval.
-__device__ __forceinline__ void quad_children(const QNode* __restrict__ quads, int node, const QRay& r, float lim,
+template <class R>
+__device__ __forceinline__ void quad_children(const QNode* __restrict__ quads, int node, const R& r, float lim,
                                               float (&key)[4], int (&ref)[4]) {
     float4 f0, f1, f2, f3;
     const float4* np = reinterpret_cast<const float4*>(quads + node);
@@ -582,7 +483,7 @@ __device__ __forceinline__ void quad_children(const QNode* __restrict__ quads, i
         const float tnz = __fmaf_rn(quad_plane(nz, k), Sz, nCz), tfz = __fmaf_rn(quad_plane(fz, k), Sz, fCz);
         const float tn = fmaxf(max3(tnx, tny, tnz), r.tmin);
         const float tf = fminf(min3(tfx, tfy, tfz), lim);
-        key[k] = tn <= __fmaf_rn(fabsf(tf), 2e-6f, tf) ? tn : kQMiss;
+        key[k] = tn <= __fmaf_rn(fabsf(tf), 2e-6f, tf) ? tn : kMiss;
     }
     auto order = [&](int i, int j) {
         const bool swap = key[j] < key[i];
@@ -597,283 +498,56 @@ __device__ __forceinline__ void quad_children(const QNode* __restrict__ quads, i
     order(1, 2);
 }
 
-// Triangle i's three float4 in two loads: records are 48 bytes, so either the first or the last 32 bytes of a record
-// are aligned for a 32-byte load.
-__device__ __forceinline__ void load_leaf_triangle(const float4* __restrict__ tris, int i, float4& p0, float4& p1,
-                                                   float4& p2) {
-    const float4* tp = tris + 3 * (int64_t)i;
-    const bool odd = i & 1;
-    float4 a, b;
-    ldg_v8(tp + (odd ? 1 : 0), a, b);
-    const float4 c = __ldg(tp + (odd ? 0 : 2));
-    p0 = odd ? c : a;
-    p1 = odd ? a : b;
-    p2 = odd ? b : c;
-}
+template <int STACK>
+struct QuadWork : RefWork<STACK, kQuadShort> {
+    const QNode* quads;
+    int num_nodes;
 
-// PERSIST: a grid of resident warps that walk the batch together, a warp's k-th ray at position ((k / 32) * warps +
-// warp) * 32 + k % 32; idle lanes take new rays. Otherwise warp w has the `group` rays from w * group on.
-template <int LEAF, bool ANY, bool PERSIST, int STACK>
-__global__ void __launch_bounds__(kTraceThreads, PERSIST ? 8 : 9) quad_trace_kernel(
-    const QNode* __restrict__ quads, const float4* __restrict__ tris, int root, int num_nodes,
-    const dipl_ray* __restrict__ rays, int64_t n, dipl_hit* __restrict__ hits, uint8_t* __restrict__ occluded,
-    uint32_t flags, uint32_t* __restrict__ err, uint32_t step_limit, int group, const uint32_t* __restrict__ order) {
-    const unsigned full = 0xffffffffu;
-    __shared__ int sh_stack[kQShort * kTraceThreads];
-    // rays shared by a warp, one column per ray (the lane it started on)
-    __shared__ float4 s_best[ANY ? 1 : kTraceThreads];  // closest hit of the lanes that are done: t, u, v, primitive
-    __shared__ float s_tmax[ANY ? 1 : kTraceThreads];
-    __shared__ unsigned s_lim[kTraceThreads];           // ordered bits of the least t of all lanes; any hit: 0 once hit
-    __shared__ int s_lanes[kTraceThreads];              // lanes at work on the ray
-    __shared__ long long s_ray[kTraceThreads];          // the ray's index
-    const int lane = threadIdx.x & 31, wbase = threadIdx.x & ~31;
-    const uint32_t lt_mask = lanemask_lt();
-    const int64_t warp_id = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    auto position = [&](int64_t k) -> int64_t { return (((k >> 5) * warps + warp_id) << 5) + (k & 31); };
-    const bool backface = (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u;
-    int64_t next = 0;   // rays this warp has taken (warp-uniform)
-    int64_t my = -1;    // this lane's ray, -1 when idle
-    QRay r{};
-    WtRay w{};
-    float tmax = 0.0f, best_t = 0.0f, best_u = 0.0f, best_v = 0.0f;
-    int best_prim = -1;
-    bool found = false, bad = false;
-    // The lane's work: a node (cur >= 0), kQIdle, or a leaf (cur < 0) that waits for `leaf` to be taken; `leaf`: the
-    // leaf range whose triangles are tested next, 0 for none.
-    int cur = kQIdle, leaf = 0;
-    uint32_t steps = 0;
-    QStack<STACK> st;
-    st.column = sh_stack + threadIdx.x;
-
-    auto start_ray = [&](int64_t cand) {
-        my = order ? (int64_t)__ldg(order + cand) : cand;  // the ray's own index (hits go there)
-        const bool live = quad_load_ray(rays, my, r, tmax);
-        if (LEAF == DIPL_LEAF_WATERTIGHT) w = wt_setup(r.d);
-        best_t = tmax, best_u = 0.0f, best_v = 0.0f, best_prim = -1, found = false;
-        cur = live && num_nodes >= 0 ? root : kQIdle;
-        leaf = 0;
-        if (cur < 0) leaf = cur, cur = kQIdle;  // the root is a leaf
-        st.sp = 0;
-        steps = 0;
-    };
-    // Pops until a node comes up, the leaf slot and cur both hold a leaf, or the stack is down to `bot`.
-    auto advance = [&](int bot) {
-        for (;;) {
-            if (cur == kQPop) {
-                if (st.sp <= bot) {
-                    cur = kQIdle;
-                    return;
-                }
-                cur = st.pop();
-            }
-            if (cur >= 0 || leaf != 0) return;
-            leaf = cur;
-            cur = kQPop;
-        }
-    };
-    auto give_up = [&]() {  // only a corrupted tree or a step limit gets here
-        bad = true;
-        cur = kQIdle;
-        leaf = 0;
-    };
-    auto node_step = [&](float lim, int bot) {
-        if (++steps > step_limit || cur >= num_nodes || st.sp + 3 > STACK) {
-            give_up();
+    template <class R>
+    __device__ __forceinline__ void begin(const R&) { this->enter(this->root); }
+    template <class R>
+    __device__ __forceinline__ void take(const R&, int thread, int entry, int) {
+        this->enter(this->column[entry * kTraceThreads + thread - (int)threadIdx.x]);
+    }
+    template <class R>
+    __device__ __forceinline__ void node(const R& r, float lim, int bot) {
+        if (this->cur >= num_nodes || this->sp + 3 > STACK) {  // only a corrupted tree gets here
+            this->bad = true;
+            this->drop();
             return;
         }
         float key[4];
         int ref[4];
-        quad_children(quads, cur, r, lim, key, ref);
-        cur = kQPop;
-        if (key[0] < kQMiss) {
-            if (st.sp + 3 <= kQShort) {
-                if (key[3] < kQMiss) st.push_short(ref[3]);
-                if (key[2] < kQMiss) st.push_short(ref[2]);
-                if (key[1] < kQMiss) st.push_short(ref[1]);
+        quad_children(quads, this->cur, r, lim, key, ref);
+        this->cur = kRefPop;
+        if (key[0] < kMiss) {
+            if (this->sp + 3 <= kQuadShort) {
+                if (key[3] < kMiss) this->push_short(ref[3]);
+                if (key[2] < kMiss) this->push_short(ref[2]);
+                if (key[1] < kMiss) this->push_short(ref[1]);
             } else {
-                if (key[3] < kQMiss) st.push(ref[3]);
-                if (key[2] < kQMiss) st.push(ref[2]);
-                if (key[1] < kQMiss) st.push(ref[1]);
+                if (key[3] < kMiss) this->push(ref[3]);
+                if (key[2] < kMiss) this->push(ref[2]);
+                if (key[1] < kMiss) this->push(ref[1]);
             }
-            cur = ref[0];
+            this->cur = ref[0];
         }
-        advance(bot);
-    };
-    auto leaf_step = [&](int bot) {
-        if (++steps > step_limit) {
-            give_up();
-            return;
-        }
-        const int first = leaf_first(leaf), cnt = leaf_count(leaf);
-        if (cnt > 0) {  // an unused child slot has no triangles
-            float4 p0, p1, p2;
-            load_leaf_triangle(tris, first, p0, p1, p2);
-            const int prim = __float_as_int(p0.w);
-            const float3 a = make_float3(p0.x, p0.y, p0.z), b = make_float3(p1.x, p1.y, p1.z),
-                         c = make_float3(p2.x, p2.y, p2.z);
-            float b1 = 0.0f, b2 = 0.0f;
-            const float t = LEAF == DIPL_LEAF_REF_MT ? mt_ref(a, b, c, r.o, r.d, backface, b1, b2)
-                                                     : wt_test(a, b, c, r.o, w, backface, b1, b2);
-            // t == kInfinity is the tests' miss value (also when tmax is +inf)
-            if (ANY) {
-                if (t > r.tmin && t < best_t && t < kInfinity) found = true;
-            } else if (t > r.tmin && t < kInfinity && (t < best_t || (t == best_t && found && prim < best_prim))) {
-                best_t = t, best_u = b1, best_v = b2, best_prim = prim, found = true;
-            }
-        }
-        if (ANY && found) {
-            cur = kQIdle;
-            leaf = 0;
-        } else if (cnt > 1) {
-            leaf = make_leaf_ref(first + 1, cnt - 1);
-        } else {
-            leaf = 0;
-            if (cur < 0) {
-                leaf = cur;
-                cur = kQPop;
-                advance(bot);
-            }
-        }
-    };
-    // One step of the warp (called by all lanes; `on`: this lane has work): a node for every lane that has one, then,
-    // once kLeafTurn lanes hold a leaf or no lane has a node left, a triangle for every lane that holds a leaf. True
-    // when triangles were tested.
-    auto warp_step = [&](bool on, float lim, int bot) {
-        if (on && cur >= 0 && cur != kQIdle) node_step(lim, bot);
-        const uint32_t holds = __ballot_sync(full, on && leaf != 0);
-        const uint32_t nodes = __ballot_sync(full, on && cur >= 0 && cur != kQIdle);
-        if (holds == 0u || (nodes != 0u && __popc(holds) < kLeafTurn)) return false;
-        if (on && leaf != 0) leaf_step(bot);
-        return true;
-    };
-    auto write_hit = [&](int64_t i, float t, float u, float v, int prim) {
-        reinterpret_cast<int4*>(hits)[i] =
-            prim >= 0 ? make_int4(prim, __float_as_int(t), __float_as_int(u), __float_as_int(v))
-                      : make_int4(-1, 0x7F800000, 0, 0);
-    };
+        this->advance(bot);
+    }
+};
 
-    // ---- every lane its own ray --------------------------------------------------------------------------------
-    if (!PERSIST) {
-        const int64_t cand = warp_id * group + lane;
-        if (lane < group && cand < n) start_ray(cand);
-    }
-    for (;;) {
-        bool more = false;
-        if (PERSIST) {
-            const uint32_t idle = __ballot_sync(full, my < 0);
-            more = position(next) < n;
-            if (more && __popc(idle) >= kRefillLanes) {
-                if (my < 0) {
-                    const int64_t cand = position(next + __popc(idle & lt_mask));
-                    if (cand < n) start_ray(cand);
-                }
-                next += __popc(idle);
-                more = position(next) < n;
-            }
-        }
-        const uint32_t active = __ballot_sync(full, my >= 0);
-        if (!more && __popc(active) <= kShareLanes) break;
-        warp_step(my >= 0, prune_limit(best_t), 0);
-        if (my >= 0 && cur == kQIdle && leaf == 0) {
-            if (ANY) occluded[my] = found ? 1 : 0;
-            else write_hit(my, best_t, best_u, best_v, found ? best_prim : -1);
-            my = -1;
-        }
-    }
-
-    // ---- the warp's last rays, shared by its lanes -----------------------------------------------------------------
-    // A lane without work takes the bottom stack entry (the largest pending subtree) of a lane that has one, with that
-    // lane's ray. Lanes prune by the least t any lane has found for the ray (s_lim) but accept hits against their own,
-    // so that the smallest (t, primitive id) of all lanes is the record a single lane would produce; each lane that
-    // runs out of work merges its best into s_best, and the last one writes the record. Entries leave a stack at the
-    // bottom (bot) only while they are in shared memory.
-    int owner = lane, bot = 0;
-    bool working = my >= 0;
-    if (working) {
-        s_ray[threadIdx.x] = my;
-        s_lanes[threadIdx.x] = 1;
-        s_lim[threadIdx.x] = ANY ? 1u : ordered_bits(best_t);
-        if (!ANY) {
-            s_tmax[threadIdx.x] = tmax;
-            s_best[threadIdx.x] = found ? make_float4(best_t, best_u, best_v, __int_as_float(best_prim))
-                                        : make_float4(__int_as_float(0x7F800000), 0.0f, 0.0f, __int_as_float(-1));
-        }
-    }
-    for (;;) {
-        __syncwarp();  // the last step's shared-memory writes, before other lanes read them
-        const uint32_t idle = __ballot_sync(full, !working);
-        if (idle == full) break;
-        const bool can_give = working && st.sp > bot && bot < kQShort;
-        const uint32_t givers = __ballot_sync(full, can_give);
-        if (idle && givers) {
-            const int rank = __popc(idle & lt_mask);
-            const bool take = !working && rank < __popc(givers);
-            const int src = take ? nth_set_bit(givers, rank) : lane;
-            const int sbot = __shfl_sync(full, bot, src), sowner = __shfl_sync(full, owner, src);
-            QRay q;
-            q.o.x = __shfl_sync(full, r.o.x, src), q.o.y = __shfl_sync(full, r.o.y, src);
-            q.o.z = __shfl_sync(full, r.o.z, src), q.d.x = __shfl_sync(full, r.d.x, src);
-            q.d.y = __shfl_sync(full, r.d.y, src), q.d.z = __shfl_sync(full, r.d.z, src);
-            q.inv.x = __shfl_sync(full, r.inv.x, src), q.inv.y = __shfl_sync(full, r.inv.y, src);
-            q.inv.z = __shfl_sync(full, r.inv.z, src), q.tmin = __shfl_sync(full, r.tmin, src);
-            const uint32_t ssteps = __shfl_sync(full, steps, src);
-            const float stmax = ANY ? __shfl_sync(full, best_t, src) : 0.0f;
-            if (take) {
-                owner = sowner;
-                r = q;
-                if (LEAF == DIPL_LEAF_WATERTIGHT) w = wt_setup(r.d);
-                best_t = ANY ? stmax : s_tmax[wbase + owner];
-                best_prim = -1, found = false;
-                cur = sh_stack[sbot * kTraceThreads + wbase + src], leaf = 0;
-                if (cur < 0) leaf = cur, cur = kQIdle;
-                steps = ssteps;
-                st.sp = bot = 0;
-                working = true;
-                atomicAdd(&s_lanes[wbase + owner], 1);
-            }
-            __syncwarp();  // entries read, before their lanes overwrite them
-            if (can_give && __popc(givers & lt_mask) < __popc(idle)) {
-                ++bot;
-                if (bot == st.sp) bot = st.sp = 0;
-            }
-        }
-        const unsigned lb = working ? s_lim[wbase + owner] : 0u;
-        if (ANY && working && lb == 0u) cur = kQIdle, leaf = 0;
-        const float before = best_t;
-        if (warp_step(working, prune_limit(ANY ? best_t : from_ordered_bits(lb)), bot) && working) {
-            if (ANY) {
-                if (found) s_lim[wbase + owner] = 0u;
-            } else if (best_t < before) {
-                atomicMin(&s_lim[wbase + owner], ordered_bits(best_t));
-            }
-        }
-        uint32_t done = __ballot_sync(full, working && cur == kQIdle && leaf == 0);
-        while (done) {  // one lane at a time: several may have worked on one ray
-            if (lane == __ffs(done) - 1) {
-                const int o = wbase + owner;
-                if (!ANY && found) {
-                    const float4 b = s_best[o];
-                    if (best_t < b.x || (best_t == b.x && (unsigned)best_prim < (unsigned)__float_as_int(b.w)))
-                        s_best[o] = make_float4(best_t, best_u, best_v, __int_as_float(best_prim));
-                }
-                const int left = s_lanes[o] - 1;
-                s_lanes[o] = left;
-                if (left == 0) {
-                    if (ANY) {
-                        occluded[s_ray[o]] = s_lim[o] == 0u ? 1 : 0;
-                    } else {
-                        const float4 b = s_best[o];
-                        write_hit(s_ray[o], b.x, b.y, b.z, __float_as_int(b.w));
-                    }
-                }
-                working = false;
-            }
-            done &= done - 1u;
-            __syncwarp();
-        }
-    }
-    if (bad) atomicOr(err, kErrStack);
+template <int LEAF, bool ANY, bool PERSIST, int STACK>
+__global__ void __launch_bounds__(kTraceThreads, PERSIST ? 8 : 9) quad_trace_kernel(
+    const QNode* __restrict__ quads, const float4* __restrict__ tris, int root, int num_nodes, uint32_t flags, Batch B) {
+    __shared__ int s_stack[kQuadShort * kTraceThreads];
+    __shared__ SharedRays<ANY> S;
+    int rest[STACK - kQuadShort];
+    QuadWork<STACK> v;
+    v.tris = tris, v.column = s_stack + threadIdx.x, v.rest = rest, v.root = root;
+    v.backface = (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u;
+    v.quads = quads, v.num_nodes = num_nodes;
+    LaneRay<LEAF, ANY> r{};
+    trace_batch<LEAF, ANY, PERSIST>(v, r, S, B);
 }
 
 // ---- ray order ----------------------------------------------------------------------------------------
@@ -937,20 +611,6 @@ __global__ void __launch_bounds__(256) ray_keys_kernel(const dipl_ray* __restric
     keys[i] = (oct << 27) | (spread3_9(cell[0]) << 2) | (spread3_9(cell[1]) << 1) | spread3_9(cell[2]);
 }
 
-// Blocks of a persistent trace launch: every resident block on every SM (per kernel instantiation and device).
-template <auto Kernel>
-int persistent_grid() {
-    static DeviceProbe probe;  // per instantiation
-    return probe_per_device(probe, [] {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, Kernel, kTraceThreads, 0);
-        (void)cudaGetLastError();
-        return std::max(1, sms * std::max(1, per_sm));
-    });
-}
-
 template <int LEAF, int STACK, int SHORT>
 dipl_status launch_trace(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint32_t flags,
                          unsigned long long* counters, cudaStream_t s) {
@@ -970,10 +630,7 @@ dipl_status launch_trace(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dip
         set_last_error("trace: node array is not 64-byte aligned");
         return DIPL_ERR_INTERNAL;
     }
-    // a ray takes at most one step per inner node and one per leaf triangle
-    const uint32_t steps_cap = trace_step_limit() ? trace_step_limit()
-                                                  : (uint32_t)std::min<int64_t>(0xFFFFFFFFll, 2ll * std::max(num_nodes, 0) +
-                                                                                                b->num_refs + 64);
+    const uint32_t steps_cap = steps_bound(num_nodes, b->num_refs);
     TailQueue tq{nullptr, nullptr, 0, kTailHeaderInts + 2 * STACK, n >= kTailMinRays ? kTailSteps : 0, kTailLanes,
                  steps_cap};
     void* tail_mem = nullptr;
@@ -1022,10 +679,6 @@ template <int LEAF, bool ANY, int STACK>
 dipl_status launch_quad(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ,
                         uint32_t flags, cudaStream_t s) {
     const int num_nodes = b->num_triangles == 0 ? -1 : (int)b->node_capacity;
-    // a ray takes at most one step per node and one per leaf triangle
-    const uint32_t steps_cap = trace_step_limit() ? trace_step_limit()
-                                                  : (uint32_t)std::min<int64_t>(0xFFFFFFFFll, 2ll * std::max(num_nodes, 0) +
-                                                                                                  b->num_refs + 64);
     RayOrder ro;
     if (reorder_rays(n, flags)) {
         dipl_status st = make_ray_order(rays, n, b->d_err, s, ro);
@@ -1034,23 +687,12 @@ dipl_status launch_quad(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl
             return st;
         }
     }
-    // Batches that the resident lanes hold at once are spread over all warps, down to one ray per warp, whose other
-    // lanes then share it (4096 rays of a small frame: 28 us, 60 with 32 rays per warp). Larger ones in the given order
-    // run on resident warps that refill idle lanes, since their rays may differ most in length (1M sphere, 4M rays
-    // 0.38 ms against 1.11 with one ray per lane; 1M occlusion rays 1.17 against 1.69; where all rays are alike one
-    // ray per lane is a little faster: 1M primary rays 0.41 against 0.36). Sorted rays get one lane each: a warp's
-    // rays are then of similar length and start together (4M-triangle soup 11.2 against 13.8 ms).
-    const int64_t warps = (int64_t)persistent_grid<quad_trace_kernel<LEAF, ANY, false, STACK>>() * (kTraceThreads / 32);
-    if (!ro.order && n > warps * 32) {
-        const int grid = persistent_grid<quad_trace_kernel<LEAF, ANY, true, STACK>>();
-        quad_trace_kernel<LEAF, ANY, true, STACK><<<(unsigned)grid, kTraceThreads, 0, s>>>(
-            b->quads, b->tris, b->root, num_nodes, rays, n, hits, occ, flags, b->d_err, steps_cap, 32, nullptr);
-    } else {
-        const int group = (int)std::min<int64_t>(32, std::max<int64_t>(1, (n + warps - 1) / warps));
-        const int64_t per_block = (int64_t)group * (kTraceThreads / 32);
-        quad_trace_kernel<LEAF, ANY, false, STACK><<<(unsigned)((n + per_block - 1) / per_block), kTraceThreads, 0, s>>>(
-            b->quads, b->tris, b->root, num_nodes, rays, n, hits, occ, flags, b->d_err, steps_cap, group, ro.order);
-    }
+    Batch B{rays, n, hits, occ, ro.order, b->d_err, steps_bound(num_nodes, b->num_refs), 32, num_nodes < 0};
+    launch_batch<quad_trace_kernel<LEAF, ANY, false, STACK>, quad_trace_kernel<LEAF, ANY, true, STACK>>(
+        n, ro.order != nullptr, [&](auto kernel, unsigned grid, int group) {
+            B.group = group;
+            kernel<<<grid, kTraceThreads, 0, s>>>(b->quads, b->tris, b->root, num_nodes, flags, B);
+        });
     note_launches();
     const cudaError_t e = cudaGetLastError();
     if (ro.mem) device_free(ro.mem, s);

@@ -12,8 +12,7 @@
 // scale 2^e with extent / 2^e <= 255; child bounds q_lo = floor, q_hi = ceil, then adjusted until the FP32
 // decode fmaf(q, 2^e, p) lies outside the padded child box. The traversal decodes with the same fmaf, so
 // every decoded box contains its (already padded) child box: no ray can lose a hit against the FP32 nodes.
-#include "internal.h"
-#include "intersect.cuh"
+#include "traverse.cuh"
 
 namespace dipl {
 namespace {
@@ -275,7 +274,6 @@ __global__ void copy_tris_kernel(const float4* __restrict__ src, float4* __restr
 // tested as soon as the node is intersected. A node taken from a group is not re-tested against its own
 // box: its children's boxes are tested against the best t when it is visited.
 // ------------------------------------------------------------------------------------------------
-constexpr int kWTraceThreads = 128;
 constexpr int kWTraceMinBlocks = 8;  // 8 resident blocks of 128 threads per SM: at most 64 registers
 constexpr float kWSlabWiden = 1e-6f;
 constexpr float kWPruneSlack = 1e-5f;
@@ -384,15 +382,15 @@ __device__ __forceinline__ int wide_pop(int2* stack, int& sp, uint32_t oct) {
     return next;
 }
 
-// One thread per ray in the work order, blocks launched in order: at any time the GPU traces one window of the
+// Counted traces. One thread per ray in the work order, blocks launched in order: at any time the GPU traces one window of the
 // order, and a warp's lanes start their rays together. Used for rays in the coherent order, where keeping the
 // lanes of a warp on neighbouring rays matters more than not waiting for a warp's longest ray (16M-ray pre-split
 // soup: 162.5 ms against 202 ms for the persistent kernel; given order 206.7 against 215.4 ms).
-template <int LEAF, bool ANY, bool COUNT, int STACK>
-__global__ void __launch_bounds__(kWTraceThreads) wide_block_kernel(
+template <int LEAF, int STACK>
+__global__ void __launch_bounds__(kTraceThreads) wide_block_kernel(
     const WNode* __restrict__ nodes, const float4* __restrict__ tris, int root, int num_nodes,
-    const dipl_ray* __restrict__ rays, int64_t n, dipl_hit* __restrict__ hits, uint8_t* __restrict__ occluded,
-    uint32_t flags, unsigned long long* __restrict__ counters, uint32_t* __restrict__ err, uint32_t step_limit,
+    const dipl_ray* __restrict__ rays, int64_t n, dipl_hit* __restrict__ hits, uint32_t flags,
+    unsigned long long* __restrict__ counters, uint32_t* __restrict__ err, uint32_t step_limit,
     const uint32_t* __restrict__ order) {
     const int64_t work = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // position in the work order
     unsigned visits = 0, tests = 0;
@@ -413,10 +411,8 @@ __global__ void __launch_bounds__(kWTraceThreads) wide_block_kernel(
             float b1 = 0.0f, b2 = 0.0f;
             const float t = wleaf_test<LEAF>(make_float3(p0.x, p0.y, p0.z), make_float3(p1.x, p1.y, p1.z),
                                              make_float3(p2.x, p2.y, p2.z), r, w, backface, b1, b2);
-            if (COUNT) ++tests;
-            if (ANY) {
-                if (t > r.tmin && t < r.tmax && t < kInfinity) found = true;
-            } else if (t > r.tmin && t < kInfinity && (t < best_t || (t == best_t && found && prim < best_prim))) {
+            ++tests;
+            if (t > r.tmin && t < kInfinity && (t < best_t || (t == best_t && found && prim < best_prim))) {
                 best_t = t, best_prim = prim, best_u = b1, best_v = b2, found = true;
             }
         };
@@ -426,7 +422,7 @@ __global__ void __launch_bounds__(kWTraceThreads) wide_block_kernel(
         if (num_nodes < 0) {
             done = true;  // empty BVH
         } else if (root < 0) {
-            for (int k = 0, c = leaf_count(root); k < c && !(ANY && found); ++k) test_tri(leaf_first(root) + k);
+            for (int k = 0, c = leaf_count(root); k < c; ++k) test_tri(leaf_first(root) + k);
             done = true;
         } else {
             node = root;
@@ -442,13 +438,9 @@ __global__ void __launch_bounds__(kWTraceThreads) wide_block_kernel(
                     bad = true;
                     break;
                 }
-                if (COUNT) ++visits;
+                ++visits;
                 const WideHits h = wide_node_hits(nodes, node, r, oct, best_t + fabsf(best_t) * kWPruneSlack);
-                for (uint32_t tm = h.tris; tm; tm &= tm - 1u) {
-                    test_tri(h.tri_base + __ffs(tm) - 1);
-                    if (ANY && found) break;
-                }
-                if (ANY && found) break;
+                for (uint32_t tm = h.tris; tm; tm &= tm - 1u) test_tri(h.tri_base + __ffs(tm) - 1);
                 if (!wide_descend<STACK>(h, oct, node, stack, sp)) {
                     bad = true;
                     break;
@@ -459,24 +451,18 @@ __global__ void __launch_bounds__(kWTraceThreads) wide_block_kernel(
             }
         }
         if (bad) atomicOr(err, kErrStack);
-        if (ANY) {
-            occluded[i] = found ? 1 : 0;
-        } else {
-            int4 out;
-            out.x = found ? best_prim : -1;
-            out.y = __float_as_int(found ? best_t : __int_as_float(0x7F800000));
-            out.z = __float_as_int(found ? best_u : 0.0f);
-            out.w = __float_as_int(found ? best_v : 0.0f);
-            reinterpret_cast<int4*>(hits)[i] = out;
-        }
+        int4 out;
+        out.x = found ? best_prim : -1;
+        out.y = __float_as_int(found ? best_t : __int_as_float(0x7F800000));
+        out.z = __float_as_int(found ? best_u : 0.0f);
+        out.w = __float_as_int(found ? best_v : 0.0f);
+        reinterpret_cast<int4*>(hits)[i] = out;
     }
-    if (COUNT) {
-        const unsigned v = __reduce_add_sync(0xffffffffu, visits);
-        const unsigned t = __reduce_add_sync(0xffffffffu, tests);
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&counters[0], (unsigned long long)v);
-            atomicAdd(&counters[1], (unsigned long long)t);
-        }
+    const unsigned v = __reduce_add_sync(0xffffffffu, visits);
+    const unsigned t = __reduce_add_sync(0xffffffffu, tests);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&counters[0], (unsigned long long)v);
+        atomicAdd(&counters[1], (unsigned long long)t);
     }
 }
 
@@ -484,11 +470,11 @@ __global__ void __launch_bounds__(kWTraceThreads) wide_block_kernel(
 // step; a lane whose ray has ended takes the warp's next ray at the following step, so lanes do not idle behind
 // the warp's longest ray (the 1M sphere's 4M rays: 0.82 ms against 1.75 ms with one thread per ray). Used for rays
 // in the given order.
-template <int LEAF, bool ANY, bool COUNT, int STACK>
-__global__ void __launch_bounds__(kWTraceThreads, kWTraceMinBlocks) wide_trace_kernel(
+template <int LEAF, int STACK>
+__global__ void __launch_bounds__(kTraceThreads, kWTraceMinBlocks) wide_trace_kernel(
     const WNode* __restrict__ nodes, const float4* __restrict__ tris, int root, int num_nodes,
-    const dipl_ray* __restrict__ rays, int64_t n, dipl_hit* __restrict__ hits, uint8_t* __restrict__ occluded,
-    uint32_t flags, unsigned long long* __restrict__ counters, uint32_t* __restrict__ err, uint32_t step_limit,
+    const dipl_ray* __restrict__ rays, int64_t n, dipl_hit* __restrict__ hits, uint32_t flags,
+    unsigned long long* __restrict__ counters, uint32_t* __restrict__ err, uint32_t step_limit,
     const uint32_t* __restrict__ order) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -521,10 +507,8 @@ __global__ void __launch_bounds__(kWTraceThreads, kWTraceMinBlocks) wide_trace_k
         float b1 = 0.0f, b2 = 0.0f;
         const float t = wleaf_test<LEAF>(make_float3(p0.x, p0.y, p0.z), make_float3(p1.x, p1.y, p1.z),
                                          make_float3(p2.x, p2.y, p2.z), r, w, backface, b1, b2);
-        if (COUNT) ++tests;
-        if (ANY) {
-            if (t > r.tmin && t < r.tmax && t < kInfinity) found = true;
-        } else if (t > r.tmin && t < kInfinity && (t < best_t || (t == best_t && found && prim < best_prim))) {
+        ++tests;
+        if (t > r.tmin && t < kInfinity && (t < best_t || (t == best_t && found && prim < best_prim))) {
             best_t = t, best_prim = prim, best_u = b1, best_v = b2, found = true;
         }
     };
@@ -547,7 +531,7 @@ __global__ void __launch_bounds__(kWTraceThreads, kWTraceMinBlocks) wide_trace_k
                     if (num_nodes < 0) {
                         done = true;  // empty BVH
                     } else if (root < 0) {
-                        for (int k = 0, c = leaf_count(root); k < c && !(ANY && found); ++k) test_tri(leaf_first(root) + k);
+                        for (int k = 0, c = leaf_count(root); k < c; ++k) test_tri(leaf_first(root) + k);
                         done = true;
                     } else {
                         node = root;
@@ -568,16 +552,10 @@ __global__ void __launch_bounds__(kWTraceThreads, kWTraceMinBlocks) wide_trace_k
                 bad = true;
                 done = true;
             } else {
-                if (COUNT) ++visits;
+                ++visits;
                 const WideHits h = wide_node_hits(nodes, node, r, oct, best_t + fabsf(best_t) * kWPruneSlack);
-                for (uint32_t tm = h.tris; tm; tm &= tm - 1u) {
-                    test_tri(h.tri_base + __ffs(tm) - 1);
-                    if (ANY && found) break;
-                }
-                if (ANY && found) {
-                    node = -1;
-                    done = true;
-                } else if (!wide_descend<STACK>(h, oct, node, stack, sp)) {
+                for (uint32_t tm = h.tris; tm; tm &= tm - 1u) test_tri(h.tri_base + __ffs(tm) - 1);
+                if (!wide_descend<STACK>(h, oct, node, stack, sp)) {
                     bad = true;
                     done = true;
                 }
@@ -587,85 +565,253 @@ __global__ void __launch_bounds__(kWTraceThreads, kWTraceMinBlocks) wide_trace_k
             if (node < 0) done = true;
         }
         if (done) {
-            if (ANY) {
-                occluded[my] = found ? 1 : 0;
-            } else {
-                int4 out;
-                out.x = found ? best_prim : -1;
-                out.y = __float_as_int(found ? best_t : __int_as_float(0x7F800000));
-                out.z = __float_as_int(found ? best_u : 0.0f);
-                out.w = __float_as_int(found ? best_v : 0.0f);
-                reinterpret_cast<int4*>(hits)[my] = out;
-            }
+            int4 out;
+            out.x = found ? best_prim : -1;
+            out.y = __float_as_int(found ? best_t : __int_as_float(0x7F800000));
+            out.z = __float_as_int(found ? best_u : 0.0f);
+            out.w = __float_as_int(found ? best_v : 0.0f);
+            reinterpret_cast<int4*>(hits)[my] = out;
             my = -1;
         }
     }
     if (bad) atomicOr(err, kErrStack);
-    if (COUNT) {
-        const unsigned v = __reduce_add_sync(full, visits);
-        const unsigned t = __reduce_add_sync(full, tests);
-        if (lane == 0) {
-            atomicAdd(&counters[0], (unsigned long long)v);
-            atomicAdd(&counters[1], (unsigned long long)t);
-        }
+    const unsigned v = __reduce_add_sync(full, visits);
+    const unsigned t = __reduce_add_sync(full, tests);
+    if (lane == 0) {
+        atomicAdd(&counters[0], (unsigned long long)v);
+        atomicAdd(&counters[1], (unsigned long long)t);
     }
 }
 
-// Resident blocks of the traversal kernel on the current device (probed once per device and kernel).
-template <typename Kernel>
-int wide_grid(Kernel kernel) {
-    static DeviceProbe probe;
-    return probe_per_device(probe, [kernel] {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWTraceThreads, 0);
-        (void)cudaGetLastError();
-        return std::max(1, sms * std::max(1, per_sm));
-    });
+// ------------------------------------------------------------------------------------------------
+// The uncounted traversal (trace_batch over the same nodes, groups and octant order). The counted kernels spend a
+// quarter of their instructions on byte conversions (a quarter-rate unit, 42% busy), a lane tests all triangles of a
+// node while its warp waits (10 of 32 lanes active) and a warp waits for its longest ray. Here a byte becomes a float
+// by one byte permute (32768 + byte, as in QNode), planes are met at one FMA, triangles wait as bits while the lane
+// goes on with nodes, and the warp's last rays are shared. 2M-triangle soup, 2M sorted rays: 14.3 -> 10.1 ms; 1M sphere,
+// 4M rays in the given order 0.81 -> 0.39 ms. Now bound by issue slots (80%) and the ALU pipe (65%: permutes, minima); 7
+// blocks of 128 per SM, 8 spill (10.7 ms) and 6 hide less (10.7 ms).
+// ------------------------------------------------------------------------------------------------
+constexpr int kWideShort = 12;  // stack groups per thread in shared memory (one per wide level)
+
+// As wide_node_hits. A plane at p + q s is met at t = (p - o) / d + q (s / d) = C + q S; with Q = 32768 + q,
+// t = (C - 32768 S) + Q S. The rounding of p - o, C and the constant is at most 2^-22 of |C| + 32768 |S|, by which near
+// planes move back and far planes on (1/128 of a step and less); the rest is relative to t and covered by 2e-6.
+template <class R>
+__device__ __forceinline__ WideHits wide_node_entered(const WNode* __restrict__ nodes, int node, const R& r,
+                                                      uint32_t oct, float lim) {
+    const float4* np = reinterpret_cast<const float4*>(nodes + node);
+    const float4 f0 = __ldg(np), f1 = __ldg(np + 1), f2 = __ldg(np + 2), f3 = __ldg(np + 3), f4 = __ldg(np + 4);
+    const uint32_t eb = __float_as_uint(f0.w);
+    constexpr float kE = 2.384185791015625e-07f;  // 2^-22
+    auto axis = [&](float p, uint32_t e, float o, float inv, float& S, float& n, float& f) {
+        S = __fmul_rn(fabsf(__uint_as_float(e << 23)), inv);  // the next byte's low bit lands in the sign
+        const float C = __fmul_rn(__fsub_rn(p, o), inv), c = __fmaf_rn(-32768.0f, S, C);
+        const float err = __fmaf_rn(fabsf(C), kE, fabsf(S) * (32768.0f * kE));
+        n = __fsub_rn(c, err);
+        f = __fadd_rn(c, err);
+    };
+    float Sx, nx, fx, Sy, ny, fy, Sz, nz, fz;
+    axis(f0.x, eb, r.o.x, r.inv.x, Sx, nx, fx);
+    axis(f0.y, eb >> 8, r.o.y, r.inv.y, Sy, ny, fy);
+    axis(f0.z, (eb >> 16) & 0xFFu, r.o.z, r.inv.z, Sz, nz, fz);
+    auto plane = [](uint32_t w, int k) {
+        return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7504u | (uint32_t)(k << 4)));
+    };
+    const uint32_t lox[2] = {__float_as_uint(f2.x), __float_as_uint(f2.y)}, loy[2] = {__float_as_uint(f2.z), __float_as_uint(f2.w)},
+                   loz[2] = {__float_as_uint(f3.x), __float_as_uint(f3.y)}, hix[2] = {__float_as_uint(f3.z), __float_as_uint(f3.w)},
+                   hiy[2] = {__float_as_uint(f4.x), __float_as_uint(f4.y)}, hiz[2] = {__float_as_uint(f4.z), __float_as_uint(f4.w)};
+    uint32_t hit = 0u;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t wnx = r.inv.x < 0.0f ? hix[h] : lox[h], wfx = r.inv.x < 0.0f ? lox[h] : hix[h];
+        const uint32_t wny = r.inv.y < 0.0f ? hiy[h] : loy[h], wfy = r.inv.y < 0.0f ? loy[h] : hiy[h];
+        const uint32_t wnz = r.inv.z < 0.0f ? hiz[h] : loz[h], wfz = r.inv.z < 0.0f ? loz[h] : hiz[h];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float tn = fmaxf(max3(__fmaf_rn(plane(wnx, k), Sx, nx), __fmaf_rn(plane(wny, k), Sy, ny),
+                                        __fmaf_rn(plane(wnz, k), Sz, nz)), r.tmin);
+            const float tf = fminf(min3(__fmaf_rn(plane(wfx, k), Sx, fx), __fmaf_rn(plane(wfy, k), Sy, fy),
+                                        __fmaf_rn(plane(wfz, k), Sz, fz)), lim);
+            if (tn <= __fmaf_rn(fabsf(tf), 2e-6f, tf)) hit |= 1u << (4 * h + k);
+        }
+    }
+    WideHits out;
+    out.imask = eb >> 24;
+    out.child_base = __float_as_int(f1.x);
+    out.tri_base = __float_as_int(f1.y);
+    // inner children to visiting order: bit slot ^ octant
+    uint32_t in = hit & out.imask;
+    if (oct & 1u) in = ((in & 0x55u) << 1) | ((in >> 1) & 0x55u);
+    if (oct & 2u) in = ((in & 0x33u) << 2) | ((in >> 2) & 0x33u);
+    if (oct & 4u) in = ((in & 0x0Fu) << 4) | (in >> 4);
+    out.inner = in;
+    out.tris = 0u;
+    const uint32_t meta_lo = __float_as_uint(f1.z), meta_hi = __float_as_uint(f1.w);
+    for (uint32_t m = hit & ~out.imask; m; m &= m - 1u) {  // an empty slot's meta is 0: no triangles
+        const int k = __ffs(m) - 1;
+        const uint32_t meta = ((k < 4 ? meta_lo : meta_hi) >> (8 * (k & 3))) & 0xFFu;
+        out.tris |= ((1u << (meta >> 5)) - 1u) << (meta & 31u);
+    }
+    return out;
 }
 
-template <int LEAF, bool ANY, bool COUNT, int STACK>
+// The lane's work: a node, the triangles it tests next and those of the node after that (as bits from a base), and the
+// stack of groups.
+template <int STACK>
+struct WideWork {
+    static constexpr int kShort = kWideShort;
+    const WNode* nodes;
+    const float4* tris;
+    int2* column;  // this thread's stack column in shared memory
+    int2* rest;    // groups from kShort on
+    int root, num_nodes;
+    bool backface;
+    bool bad = false;
+    int current = -1;
+    int held_base = 0, next_base = 0;
+    uint32_t held = 0u, next = 0u;
+    uint32_t oct = 0u, steps = 0;
+    int sp = 0;
+
+    __device__ __forceinline__ bool has_node() const { return current >= 0 && next == 0u; }
+    __device__ __forceinline__ bool has_leaf() const { return held != 0u; }
+    __device__ __forceinline__ void drop() { current = -1, held = next = 0u; }
+    template <class R>
+    __device__ __forceinline__ void set_octant(const R& r) {
+        oct = (r.inv.x < 0.0f ? 1u : 0u) | (r.inv.y < 0.0f ? 2u : 0u) | (r.inv.z < 0.0f ? 4u : 0u);
+    }
+    template <class R>
+    __device__ __forceinline__ void begin(const R& r) {
+        set_octant(r);
+        if (root < 0) held_base = leaf_first(root), held = (1u << leaf_count(root)) - 1u;
+        else current = root;
+    }
+    __device__ __forceinline__ int2 get(int k) const { return k < kShort ? column[k * kTraceThreads] : rest[k - kShort]; }
+    __device__ __forceinline__ void set(int k, int2 e) {
+        if (k < kShort) column[k * kTraceThreads] = e;
+        else rest[k - kShort] = e;
+    }
+    // The first child of a group (child base; hits in visiting order << 8 | inner mask), and the group without it.
+    __device__ __forceinline__ int first_child(int2& e) const {
+        const uint32_t hits = (uint32_t)e.y >> 8;
+        const int b = __ffs(hits) - 1;
+        e.y = (int)(((hits & (hits - 1u)) << 8) | ((uint32_t)e.y & 0xFFu));
+        return e.x + __popc((uint32_t)e.y & 0xFFu & ((1u << ((uint32_t)b ^ oct)) - 1u));
+    }
+    __device__ __forceinline__ void pop(int bot) {
+        current = -1;
+        if (sp <= bot) return;
+        int2 e = get(sp - 1);
+        current = first_child(e);
+        if ((uint32_t)e.y >> 8) set(sp - 1, e);
+        else --sp;
+    }
+    template <class R>
+    __device__ __forceinline__ void take(const R& r, int thread, int entry, int) {
+        set_octant(r);
+        held = next = 0u;
+        int2 e = column[entry * kTraceThreads + thread - (int)threadIdx.x];
+        current = first_child(e);
+        if ((uint32_t)e.y >> 8) column[0] = e, sp = 1;
+    }
+    template <class R>
+    __device__ __forceinline__ void node(const R& r, float lim, int bot) {
+        if (current >= num_nodes || sp >= STACK) {  // only a corrupted tree gets here
+            bad = true;
+            drop();
+            return;
+        }
+        const WideHits h = wide_node_entered(nodes, current, r, oct, lim);
+        if (h.tris) {
+            if (held == 0u) held = h.tris, held_base = h.tri_base;
+            else next = h.tris, next_base = h.tri_base;
+        }
+        if (h.inner) {
+            int2 e = make_int2(h.child_base, (int)((h.inner << 8) | h.imask));
+            current = first_child(e);
+            if ((uint32_t)e.y >> 8) set(sp++, e);
+        } else {
+            pop(bot);
+        }
+    }
+    template <class R>
+    __device__ __forceinline__ void leaf(R& r, int) {
+        r.test(tris, held_base + __ffs(held) - 1, backface);
+        held &= held - 1u;
+        if (held == 0u) held = next, held_base = next_base, next = 0u;
+    }
+};
+
+template <int LEAF, bool ANY, bool PERSIST, int STACK>
+__global__ void __launch_bounds__(kTraceThreads, 7) wide_batch_kernel(const WNode* __restrict__ nodes,
+                                                                      const float4* __restrict__ tris, int root,
+                                                                      int num_nodes, uint32_t flags, Batch B) {
+    __shared__ int2 s_stack[kWideShort * kTraceThreads];
+    __shared__ SharedRays<ANY> S;
+    int2 rest[STACK - kWideShort];
+    WideWork<STACK> v;
+    v.nodes = nodes, v.tris = tris, v.column = s_stack + threadIdx.x, v.rest = rest, v.root = root;
+    v.num_nodes = num_nodes, v.backface = (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u;
+    LaneRay<LEAF, ANY> r{};
+    trace_batch<LEAF, ANY, PERSIST>(v, r, S, B);
+}
+
+template <int LEAF, int STACK>
+dipl_status launch_wide_counted(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint32_t flags,
+                                unsigned long long* counters, const RayOrder& ro, cudaStream_t s) {
+    const int num_nodes = b->num_triangles == 0 ? -1 : (int)b->node_capacity;
+    const uint32_t cap = trace_step_limit() ? trace_step_limit() : 2u * (uint32_t)std::max(num_nodes, 0) + 64u;
+    const int64_t blocks = (n + kTraceThreads - 1) / kTraceThreads;
+    if (ro.order) {
+        wide_block_kernel<LEAF, STACK><<<(unsigned)blocks, kTraceThreads, 0, s>>>(
+            static_cast<const WNode*>(b->nodes), b->tris, b->root, num_nodes, rays, n, hits, flags, counters, b->d_err,
+            cap, ro.order);
+    } else {
+        const int64_t grid =
+            std::max<int64_t>(1, std::min<int64_t>(persistent_grid<wide_trace_kernel<LEAF, STACK>>(), blocks));
+        wide_trace_kernel<LEAF, STACK><<<(unsigned)grid, kTraceThreads, 0, s>>>(
+            static_cast<const WNode*>(b->nodes), b->tris, b->root, num_nodes, rays, n, hits, flags, counters, b->d_err,
+            cap, nullptr);
+    }
+    note_launches();
+    DIPL_CUDA(cudaGetLastError());
+    return DIPL_OK;
+}
+
+template <int LEAF, bool ANY, int STACK>
 dipl_status launch_wide(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ, uint32_t flags,
                         unsigned long long* counters, cudaStream_t s) {
     const int num_nodes = b->num_triangles == 0 ? -1 : (int)b->node_capacity;
     RayOrder ro;
-    if (reorder_rays(n, flags)) {
-        const dipl_status st = make_ray_order(rays, n, b->d_err, s, ro);
-        if (st != DIPL_OK) {
-            if (ro.mem) device_free(ro.mem, s);
-            return st;
-        }
+    dipl_status st = DIPL_OK;
+    if (reorder_rays(n, flags)) st = make_ray_order(rays, n, b->d_err, s, ro);
+    if (st == DIPL_OK && !ANY && counters) {
+        st = launch_wide_counted<LEAF, STACK>(b, rays, n, hits, flags, counters, ro, s);
+    } else if (st == DIPL_OK) {
+        Batch B{rays, n, hits, occ, ro.order, b->d_err, steps_bound(num_nodes, b->num_refs), 32, num_nodes < 0};
+        launch_batch<wide_batch_kernel<LEAF, ANY, false, STACK>, wide_batch_kernel<LEAF, ANY, true, STACK>>(
+            n, ro.order != nullptr, [&](auto kernel, unsigned grid, int group) {
+                B.group = group;
+                kernel<<<grid, kTraceThreads, 0, s>>>(static_cast<const WNode*>(b->nodes), b->tris, b->root, num_nodes,
+                                                      flags, B);
+            });
+        note_launches();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) st = cuda_status(e, "wide_batch_kernel");
     }
-    const uint32_t cap = trace_step_limit() ? trace_step_limit() : 2u * (uint32_t)std::max(num_nodes, 0) + 64u;
-    if (ro.order) {
-        wide_block_kernel<LEAF, ANY, COUNT, STACK><<<(unsigned)((n + kWTraceThreads - 1) / kWTraceThreads),
-                                                     kWTraceThreads, 0, s>>>(
-            static_cast<const WNode*>(b->nodes), b->tris, b->root, num_nodes, rays, n, hits, occ, flags, counters,
-            b->d_err, cap, ro.order);
-    } else {
-        auto kernel = wide_trace_kernel<LEAF, ANY, COUNT, STACK>;
-        const int64_t grid =
-            std::max<int64_t>(1, std::min<int64_t>(wide_grid(kernel), (n + kWTraceThreads - 1) / kWTraceThreads));
-        kernel<<<(unsigned)grid, kWTraceThreads, 0, s>>>(static_cast<const WNode*>(b->nodes), b->tris, b->root,
-                                                         num_nodes, rays, n, hits, occ, flags, counters, b->d_err, cap,
-                                                         nullptr);
-    }
-    note_launches();
-    const cudaError_t e = cudaGetLastError();
     if (ro.mem) device_free(ro.mem, s);
-    DIPL_CUDA(e);
-    return DIPL_OK;
+    return st;
 }
 
 // At most one group per wide level is on the stack (depth = wide levels of the layout).
-template <int LEAF, bool ANY, bool COUNT>
+template <int LEAF, bool ANY>
 dipl_status launch_wide_stack(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ,
                               uint32_t flags, unsigned long long* counters, cudaStream_t s) {
     const int need = b->depth + 1;
-    if (need <= 32) return launch_wide<LEAF, ANY, COUNT, 32>(b, rays, n, hits, occ, flags, counters, s);
-    if (need <= 96) return launch_wide<LEAF, ANY, COUNT, 96>(b, rays, n, hits, occ, flags, counters, s);
-    return launch_wide<LEAF, ANY, COUNT, 512>(b, rays, n, hits, occ, flags, counters, s);
+    if (need <= 32) return launch_wide<LEAF, ANY, 32>(b, rays, n, hits, occ, flags, counters, s);
+    if (need <= 96) return launch_wide<LEAF, ANY, 96>(b, rays, n, hits, occ, flags, counters, s);
+    return launch_wide<LEAF, ANY, 512>(b, rays, n, hits, occ, flags, counters, s);
 }
 
 }  // namespace
@@ -760,15 +906,11 @@ dipl_status trace_wide(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_
                        uint32_t flags, unsigned long long* counters, bool any, cudaStream_t s) {
     if (any)
         return leaf_test == DIPL_LEAF_REF_MT
-                   ? launch_wide_stack<DIPL_LEAF_REF_MT, true, false>(b, rays, n, nullptr, occ, flags, nullptr, s)
-                   : launch_wide_stack<DIPL_LEAF_WATERTIGHT, true, false>(b, rays, n, nullptr, occ, flags, nullptr, s);
-    if (counters)
-        return leaf_test == DIPL_LEAF_REF_MT
-                   ? launch_wide_stack<DIPL_LEAF_REF_MT, false, true>(b, rays, n, hits, nullptr, flags, counters, s)
-                   : launch_wide_stack<DIPL_LEAF_WATERTIGHT, false, true>(b, rays, n, hits, nullptr, flags, counters, s);
+                   ? launch_wide_stack<DIPL_LEAF_REF_MT, true>(b, rays, n, nullptr, occ, flags, nullptr, s)
+                   : launch_wide_stack<DIPL_LEAF_WATERTIGHT, true>(b, rays, n, nullptr, occ, flags, nullptr, s);
     return leaf_test == DIPL_LEAF_REF_MT
-               ? launch_wide_stack<DIPL_LEAF_REF_MT, false, false>(b, rays, n, hits, nullptr, flags, nullptr, s)
-               : launch_wide_stack<DIPL_LEAF_WATERTIGHT, false, false>(b, rays, n, hits, nullptr, flags, nullptr, s);
+               ? launch_wide_stack<DIPL_LEAF_REF_MT, false>(b, rays, n, hits, nullptr, flags, counters, s)
+               : launch_wide_stack<DIPL_LEAF_WATERTIGHT, false>(b, rays, n, hits, nullptr, flags, counters, s);
 }
 
 }  // namespace dipl
