@@ -13,8 +13,7 @@
 #include <cmath>
 #include <mutex>
 
-#include "internal.h"
-#include "intersect.cuh"
+#include "traverse.cuh"
 
 namespace dipl {
 
@@ -279,7 +278,6 @@ __global__ void __launch_bounds__(kSobbNodeThreads) sobb_node_kernel(
 // ------------------------------------------------------------------------------------------------
 // Traversal: the ray's projections on the table directions are computed once per ray into shared memory.
 // ------------------------------------------------------------------------------------------------
-constexpr int kSThreads = 128;
 constexpr float kSSlabWiden = 1e-6f;
 constexpr float kSPruneSlack = 1e-5f;
 
@@ -294,7 +292,7 @@ __device__ __forceinline__ float sleaf_test(float3 a, float3 b, float3 c, float3
 // direction, and the two widening terms (the rounding of the projected origin as a distance along the ray,
 // absolute, and of the projected direction as a relative error of every distance on this slab, large for grazing
 // slabs), so a slab costs one shared load.
-__device__ __forceinline__ void sobb_ray_setup(float4 (*s_ray)[kSThreads], int tid, int dirs, float3 o, float3 d) {
+__device__ __forceinline__ void sobb_ray_setup(float4 (*s_ray)[kTraceThreads], int tid, int dirs, float3 o, float3 d) {
     const float omag = fabsf(o.x) + fabsf(o.y) + fabsf(o.z);
     const float dmag = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
     for (int k = 0; k < dirs; ++k) {
@@ -307,7 +305,7 @@ __device__ __forceinline__ void sobb_ray_setup(float4 (*s_ray)[kSThreads], int t
 
 // Entry distance of the ray into one child's three slabs (directions packed in `axes`, one per byte), widened by
 // the ray's rounding terms; +inf when the slabs are missed, end before tmin or start beyond lim.
-__device__ __forceinline__ float sobb_slab_box(const float4 (*s_ray)[kSThreads], int tid, int axes, float l0, float h0,
+__device__ __forceinline__ float sobb_slab_box(const float4 (*s_ray)[kTraceThreads], int tid, int axes, float l0, float h0,
                                                float l1, float h1, float l2, float h2, float tmin, float lim) {
     float tn = __int_as_float(0xFF800000), tf = __int_as_float(0x7F800000);
     const float ls[3] = {l0, l1, l2}, hs[3] = {h0, h1, h2};
@@ -326,7 +324,7 @@ __device__ __forceinline__ float sobb_slab_box(const float4 (*s_ray)[kSThreads],
 
 // One SOBB node: both children's entry distances (t0, t1; +inf when missed) and their references (dd.x, dd.y).
 __device__ __forceinline__ int4 sobb_children(const SNode* __restrict__ nodes, int cur,
-                                              const float4 (*s_ray)[kSThreads], int tid, float tmin, float lim,
+                                              const float4 (*s_ray)[kTraceThreads], int tid, float tmin, float lim,
                                               float& t0, float& t1) {
     const float4* np = reinterpret_cast<const float4*>(nodes + cur);
     const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
@@ -336,16 +334,15 @@ __device__ __forceinline__ int4 sobb_children(const SNode* __restrict__ nodes, i
     return dd;
 }
 
-template <int LEAF, bool ANY, bool COUNT, int STACK>
-__global__ void __launch_bounds__(kSThreads) sobb_trace_kernel(const SNode* __restrict__ nodes,
+template <int LEAF, int STACK>
+__global__ void __launch_bounds__(kTraceThreads) sobb_trace_kernel(const SNode* __restrict__ nodes,
                                                                const float4* __restrict__ tris, int root,
                                                                int num_nodes, int dirs, const dipl_ray* __restrict__ rays,
-                                                               int64_t n, dipl_hit* __restrict__ hits,
-                                                               uint8_t* __restrict__ occluded, uint32_t flags,
+                                                               int64_t n, dipl_hit* __restrict__ hits, uint32_t flags,
                                                                unsigned long long* __restrict__ counters,
                                                                uint32_t* __restrict__ err, uint32_t step_limit,
                                                                const uint32_t* __restrict__ order) {
-    __shared__ float4 s_ray[kDirs][kSThreads];  // the rays' records per direction (sobb_ray_setup)
+    __shared__ float4 s_ray[kDirs][kTraceThreads];  // the rays' records per direction (sobb_ray_setup)
     const int64_t work = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // position in the work order
     unsigned visits = 0, tests = 0;
     if (work < n) {
@@ -377,7 +374,7 @@ __global__ void __launch_bounds__(kSThreads) sobb_trace_kernel(const SNode* __re
                     bad = true;
                     break;
                 }
-                if (COUNT) ++visits;
+                ++visits;
                 float t0, t1;
                 const int4 dd = sobb_children(nodes, cur, s_ray, tid, tmin, best_t + fabsf(best_t) * kSPruneSlack,
                                               t0, t1);
@@ -412,13 +409,10 @@ __global__ void __launch_bounds__(kSThreads) sobb_trace_kernel(const SNode* __re
                 float b1 = 0.0f, b2 = 0.0f;
                 const float t = sleaf_test<LEAF>(make_float3(p0.x, p0.y, p0.z), make_float3(p1.x, p1.y, p1.z),
                                                  make_float3(p2.x, p2.y, p2.z), o, d, w, backface, b1, b2);
-                if (COUNT) ++tests;
-                if (ANY) {
-                    if (t > tmin && t < tmax && t < kInfinity) found = true;
-                } else if (t > tmin && t < kInfinity && (t < best_t || (t == best_t && found && prim < best_prim))) {
+                ++tests;
+                if (t > tmin && t < kInfinity && (t < best_t || (t == best_t && found && prim < best_prim))) {
                     best_t = t, best_prim = prim, best_u = b1, best_v = b2, found = true;
                 }
-                if (ANY && found) break;
                 if (cnt > 1) {
                     cur = make_leaf_ref(first + 1, cnt - 1);
                     continue;
@@ -435,24 +429,18 @@ __global__ void __launch_bounds__(kSThreads) sobb_trace_kernel(const SNode* __re
             }
         }
         if (bad) atomicOr(err, kErrStack);
-        if (ANY) {
-            occluded[i] = found ? 1 : 0;
-        } else {
-            int4 out;
-            out.x = found ? best_prim : -1;
-            out.y = __float_as_int(found ? best_t : __int_as_float(0x7F800000));
-            out.z = __float_as_int(found ? best_u : 0.0f);
-            out.w = __float_as_int(found ? best_v : 0.0f);
-            reinterpret_cast<int4*>(hits)[i] = out;
-        }
+        int4 out;
+        out.x = found ? best_prim : -1;
+        out.y = __float_as_int(found ? best_t : __int_as_float(0x7F800000));
+        out.z = __float_as_int(found ? best_u : 0.0f);
+        out.w = __float_as_int(found ? best_v : 0.0f);
+        reinterpret_cast<int4*>(hits)[i] = out;
     }
-    if (COUNT) {
-        const unsigned v = __reduce_add_sync(0xffffffffu, visits);
-        const unsigned t = __reduce_add_sync(0xffffffffu, tests);
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&counters[0], (unsigned long long)v);
-            atomicAdd(&counters[1], (unsigned long long)t);
-        }
+    const unsigned v = __reduce_add_sync(0xffffffffu, visits);
+    const unsigned t = __reduce_add_sync(0xffffffffu, tests);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&counters[0], (unsigned long long)v);
+        atomicAdd(&counters[1], (unsigned long long)t);
     }
 }
 
@@ -460,18 +448,17 @@ __global__ void __launch_bounds__(kSThreads) sobb_trace_kernel(const SNode* __re
 // pop per step and takes the warp's next ray when its own ends, and the warps take 32-ray groups interleaved over
 // the batch (warp w takes groups w, w + W, ...), so no lane waits for its warp's longest ray (the one-thread-per-ray
 // kernel above stays for the coherent order, where lanes that start neighbouring rays together matter more).
-template <int LEAF, bool ANY, bool COUNT, int STACK>
-__global__ void __launch_bounds__(kSThreads) sobb_persist_kernel(const SNode* __restrict__ nodes,
+template <int LEAF, int STACK>
+__global__ void __launch_bounds__(kTraceThreads) sobb_persist_kernel(const SNode* __restrict__ nodes,
                                                                  const float4* __restrict__ tris, int root,
                                                                  int num_nodes, int dirs,
                                                                  const dipl_ray* __restrict__ rays, int64_t n,
-                                                                 dipl_hit* __restrict__ hits,
-                                                                 uint8_t* __restrict__ occluded, uint32_t flags,
+                                                                 dipl_hit* __restrict__ hits, uint32_t flags,
                                                                  unsigned long long* __restrict__ counters,
                                                                  uint32_t* __restrict__ err, uint32_t step_limit,
                                                                  const uint32_t* __restrict__ order) {
     constexpr int kDone = 0x7FFFFFFF;
-    __shared__ float4 s_ray[kDirs][kSThreads];
+    __shared__ float4 s_ray[kDirs][kTraceThreads];
     const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t warp_id = (blockIdx.x * (int64_t)blockDim.x + tid) >> 5;
@@ -530,7 +517,7 @@ __global__ void __launch_bounds__(kSThreads) sobb_persist_kernel(const SNode* __
             bad = true;  // only a corrupted tree gets here
             finished = true;
         } else if (cur >= 0) {
-            if (COUNT) ++visits;
+            ++visits;
             float t0, t1;
             const int4 dd = sobb_children(nodes, cur, s_ray, tid, tmin, best_t + fabsf(best_t) * kSPruneSlack, t0, t1);
             const bool h0 = t0 != __int_as_float(0x7F800000), h1 = t1 != __int_as_float(0x7F800000);
@@ -561,14 +548,11 @@ __global__ void __launch_bounds__(kSThreads) sobb_persist_kernel(const SNode* __
             float b1 = 0.0f, b2 = 0.0f;
             const float t = sleaf_test<LEAF>(make_float3(p0.x, p0.y, p0.z), make_float3(p1.x, p1.y, p1.z),
                                              make_float3(p2.x, p2.y, p2.z), o, d, w, backface, b1, b2);
-            if (COUNT) ++tests;
-            if (ANY) {
-                if (t > tmin && t < tmax && t < kInfinity) found = true;
-            } else if (t > tmin && t < kInfinity && (t < best_t || (t == best_t && found && prim < best_prim))) {
+            ++tests;
+            if (t > tmin && t < kInfinity && (t < best_t || (t == best_t && found && prim < best_prim))) {
                 best_t = t, best_prim = prim, best_u = b1, best_v = b2, found = true;
             }
-            if (ANY && found) finished = true;
-            else if (cnt > 1) cur = make_leaf_ref(first + 1, cnt - 1);
+            if (cnt > 1) cur = make_leaf_ref(first + 1, cnt - 1);
             else pop = true;
         }
         if (pop) {
@@ -584,84 +568,171 @@ __global__ void __launch_bounds__(kSThreads) sobb_persist_kernel(const SNode* __
             if (cur == kDone) finished = true;
         }
         if (finished) {
-            if (ANY) {
-                occluded[my] = found ? 1 : 0;
-            } else {
-                int4 out;
-                out.x = found ? best_prim : -1;
-                out.y = __float_as_int(found ? best_t : __int_as_float(0x7F800000));
-                out.z = __float_as_int(found ? best_u : 0.0f);
-                out.w = __float_as_int(found ? best_v : 0.0f);
-                reinterpret_cast<int4*>(hits)[my] = out;
-            }
+            int4 out;
+            out.x = found ? best_prim : -1;
+            out.y = __float_as_int(found ? best_t : __int_as_float(0x7F800000));
+            out.z = __float_as_int(found ? best_u : 0.0f);
+            out.w = __float_as_int(found ? best_v : 0.0f);
+            reinterpret_cast<int4*>(hits)[my] = out;
             my = -1;
         }
     }
     if (bad) atomicOr(err, kErrStack);
-    if (COUNT) {
-        const unsigned v = __reduce_add_sync(full, visits);
-        const unsigned t = __reduce_add_sync(full, tests);
-        if (lane == 0) {
-            atomicAdd(&counters[0], (unsigned long long)v);
-            atomicAdd(&counters[1], (unsigned long long)t);
-        }
+    const unsigned v = __reduce_add_sync(full, visits);
+    const unsigned t = __reduce_add_sync(full, tests);
+    if (lane == 0) {
+        atomicAdd(&counters[0], (unsigned long long)v);
+        atomicAdd(&counters[1], (unsigned long long)t);
     }
 }
 
-// Resident blocks of a traversal kernel on the current device (probed once per device and kernel).
-template <typename Kernel>
-int sobb_grid(Kernel kernel) {
-    static DeviceProbe probe;
-    return probe_per_device(probe, [kernel] {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSThreads, 0);
-        (void)cudaGetLastError();
-        return std::max(1, sms * std::max(1, per_sm));
-    });
+// ------------------------------------------------------------------------------------------------
+// The uncounted traversal (trace_batch over the same nodes; the counted kernels above walk them one ray per lane or
+// with persistent warps). The ray's record per table direction is the projected origin and the reciprocal projected
+// direction; the widening terms follow from the latter, so that the records take 16 KB of shared memory a block instead
+// of 32 and leave room for the stack. Lanes that share a ray read the record in the column of the lane it started on.
+// Was bound by a warp's longest ray and by local-memory stacks: 1M-triangle soup, 2M sorted rays 18.1 -> 12.3 ms; 250k
+// sphere, 2M rays in the given order 357 -> 281 us, 100k rays 188 -> 65 us. Now by the six shared-memory records and
+// the issue slots of a node visit.
+// ------------------------------------------------------------------------------------------------
+constexpr int kSobbShort = 12;  // stack entries per thread in shared memory (24: 1M-triangle soup +6%, 250k sphere +13%)
+
+template <int STACK>
+struct SobbWork : RefWork<STACK, kSobbShort> {
+    const SNode* nodes;
+    int num_nodes, dirs;
+    float2 (*s_ray)[kTraceThreads];
+    int col = 0;            // the shared-memory column of this lane's ray
+    float omag4, dmag4;     // 4e-7 times the 1-norms of origin and direction
+
+    template <class R>
+    __device__ __forceinline__ void magnitudes(const R& r) {
+        omag4 = (fabsf(r.o.x) + fabsf(r.o.y) + fabsf(r.o.z)) * 4.0e-7f;
+        dmag4 = (fabsf(r.d.x) + fabsf(r.d.y) + fabsf(r.d.z)) * 4.0e-7f;
+    }
+    template <class R>
+    __device__ __forceinline__ void begin(const R& r) {
+        col = threadIdx.x;
+        magnitudes(r);
+        for (int k = 0; k < dirs; ++k) {
+            const float dk = proj(k, r.d.x, r.d.y, r.d.z);
+            s_ray[k][col] = make_float2(proj(k, r.o.x, r.o.y, r.o.z),
+                                        __frcp_rn(fabsf(dk) < 1e-20f ? copysignf(1e-20f, dk) : dk));
+        }
+        this->enter(this->root);
+    }
+    template <class R>
+    __device__ __forceinline__ void take(const R& r, int thread, int entry, int owner) {
+        col = owner;
+        magnitudes(r);
+        this->enter(this->column[entry * kTraceThreads + thread - (int)threadIdx.x]);
+    }
+    // As sobb_slab_box.
+    __device__ __forceinline__ float entry(int axes, float l0, float h0, float l1, float h1, float l2, float h2,
+                                           float tmin, float lim) const {
+        float tn = tmin, tf = lim;
+        const float ls[3] = {l0, l1, l2}, hs[3] = {h0, h1, h2};
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const float2 q = s_ray[(axes >> (8 * j)) & 0xFF][col];
+            const float ai = fabsf(q.y), tol = omag4 * ai, rel = __fmaf_rn(dmag4, ai, kSSlabWiden);
+            const float t0 = __fmul_rn(__fsub_rn(ls[j], q.x), q.y), t1 = __fmul_rn(__fsub_rn(hs[j], q.x), q.y);
+            const float a0 = fminf(t0, t1), a1 = fmaxf(t0, t1);
+            tn = fmaxf(tn, a0 - __fmaf_rn(fabsf(a0), rel, tol));
+            tf = fminf(tf, a1 + __fmaf_rn(fabsf(a1), rel, tol));
+        }
+        return tn <= tf ? tn : __int_as_float(0x7F800000);
+    }
+    template <class R>
+    __device__ __forceinline__ void node(const R& r, float lim, int bot) {
+        if (this->cur >= num_nodes || this->sp >= STACK) {  // only a corrupted tree gets here
+            this->bad = true;
+            this->drop();
+            return;
+        }
+        const float4* np = reinterpret_cast<const float4*>(nodes + this->cur);
+        float4 a, b, c, df;
+        ldg_v8(np, a, b);
+        ldg_v8(np + 2, c, df);
+        const int c0 = __float_as_int(df.x), c1 = __float_as_int(df.y);
+        const float t0 = entry(__float_as_int(df.z), a.x, a.y, a.z, a.w, b.x, b.y, r.tmin, lim);
+        const float t1 = entry(__float_as_int(df.w), b.z, b.w, c.x, c.y, c.z, c.w, r.tmin, lim);
+        const bool swap = t1 < t0;
+        if (fmaxf(t0, t1) != __int_as_float(0x7F800000)) this->push(swap ? c0 : c1);
+        this->cur = fminf(t0, t1) != __int_as_float(0x7F800000) ? (swap ? c1 : c0) : kRefPop;
+        this->advance(bot);
+    }
+};
+
+template <int LEAF, bool ANY, bool PERSIST, int STACK>
+__global__ void __launch_bounds__(kTraceThreads, 6) sobb_batch_kernel(const SNode* __restrict__ nodes,
+                                                                      const float4* __restrict__ tris, int root,
+                                                                      int num_nodes, int dirs, uint32_t flags, Batch B) {
+    __shared__ int s_stack[kSobbShort * kTraceThreads];
+    __shared__ float2 s_ray[kDirs][kTraceThreads];
+    __shared__ SharedRays<ANY> S;
+    int rest[STACK - kSobbShort];
+    SobbWork<STACK> v;
+    v.tris = tris, v.column = s_stack + threadIdx.x, v.rest = rest, v.root = root;
+    v.backface = (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u;
+    v.nodes = nodes, v.num_nodes = num_nodes, v.dirs = dirs, v.s_ray = s_ray;
+    LaneRay<LEAF, ANY> r{};
+    trace_batch<LEAF, ANY, PERSIST>(v, r, S, B);
 }
 
-template <int LEAF, bool ANY, bool COUNT, int STACK>
+template <int LEAF, int STACK>
+dipl_status launch_sobb_counted(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint32_t flags,
+                                unsigned long long* counters, const RayOrder& ro, cudaStream_t s) {
+    const int num_nodes = b->num_triangles == 0 ? -1 : (int)b->node_capacity;
+    const uint32_t cap = steps_bound(num_nodes, b->num_refs);
+    const int64_t blocks = (n + kTraceThreads - 1) / kTraceThreads;
+    if (ro.order) {
+        sobb_trace_kernel<LEAF, STACK><<<(unsigned)blocks, kTraceThreads, 0, s>>>(
+            static_cast<const SNode*>(b->nodes), b->tris, b->root, num_nodes, b->kdop / 2, rays, n, hits, flags, counters,
+            b->d_err, cap, ro.order);
+    } else {
+        const int64_t grid =
+            std::max<int64_t>(1, std::min<int64_t>(persistent_grid<sobb_persist_kernel<LEAF, STACK>>(), blocks));
+        sobb_persist_kernel<LEAF, STACK><<<(unsigned)grid, kTraceThreads, 0, s>>>(
+            static_cast<const SNode*>(b->nodes), b->tris, b->root, num_nodes, b->kdop / 2, rays, n, hits, flags, counters,
+            b->d_err, cap, nullptr);
+    }
+    note_launches();
+    DIPL_CUDA(cudaGetLastError());
+    return DIPL_OK;
+}
+
+template <int LEAF, bool ANY, int STACK>
 dipl_status launch_sobb(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ,
                         uint32_t flags, unsigned long long* counters, cudaStream_t s) {
     const int num_nodes = b->num_triangles == 0 ? -1 : (int)b->node_capacity;
     RayOrder ro;
-    if (reorder_rays(n, flags)) {
-        const dipl_status st = make_ray_order(rays, n, b->d_err, s, ro);
-        if (st != DIPL_OK) {
-            if (ro.mem) device_free(ro.mem, s);
-            return st;
-        }
+    dipl_status st = DIPL_OK;
+    if (reorder_rays(n, flags)) st = make_ray_order(rays, n, b->d_err, s, ro);
+    if (st == DIPL_OK && !ANY && counters) {
+        st = launch_sobb_counted<LEAF, STACK>(b, rays, n, hits, flags, counters, ro, s);
+    } else if (st == DIPL_OK) {
+        Batch B{rays, n, hits, occ, ro.order, b->d_err, steps_bound(num_nodes, b->num_refs), 32, num_nodes < 0};
+        launch_batch<sobb_batch_kernel<LEAF, ANY, false, STACK>, sobb_batch_kernel<LEAF, ANY, true, STACK>>(
+            n, ro.order != nullptr, [&](auto kernel, unsigned grid, int group) {
+                B.group = group;
+                kernel<<<grid, kTraceThreads, 0, s>>>(static_cast<const SNode*>(b->nodes), b->tris, b->root, num_nodes,
+                                                      b->kdop / 2, flags, B);
+            });
+        note_launches();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) st = cuda_status(e, "sobb_batch_kernel");
     }
-    const uint32_t cap =
-        trace_step_limit() ? trace_step_limit()
-                           : (uint32_t)std::min<int64_t>(0xFFFFFFFFll, 2ll * std::max(num_nodes, 0) + b->num_refs + 64);
-    if (ro.order) {
-        sobb_trace_kernel<LEAF, ANY, COUNT, STACK><<<(unsigned)((n + kSThreads - 1) / kSThreads), kSThreads, 0, s>>>(
-            static_cast<const SNode*>(b->nodes), b->tris, b->root, num_nodes, b->kdop / 2, rays, n, hits, occ, flags,
-            counters, b->d_err, cap, ro.order);
-    } else {
-        auto kernel = sobb_persist_kernel<LEAF, ANY, COUNT, STACK>;
-        const int64_t grid =
-            std::max<int64_t>(1, std::min<int64_t>(sobb_grid(kernel), (n + kSThreads - 1) / kSThreads));
-        kernel<<<(unsigned)grid, kSThreads, 0, s>>>(static_cast<const SNode*>(b->nodes), b->tris, b->root, num_nodes,
-                                                    b->kdop / 2, rays, n, hits, occ, flags, counters, b->d_err, cap,
-                                                    nullptr);
-    }
-    note_launches();
-    const cudaError_t e = cudaGetLastError();
     if (ro.mem) device_free(ro.mem, s);
-    DIPL_CUDA(e);
-    return DIPL_OK;
+    return st;
 }
 
-template <int LEAF, bool ANY, bool COUNT>
+template <int LEAF, bool ANY>
 dipl_status launch_sobb_stack(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ,
                               uint32_t flags, unsigned long long* counters, cudaStream_t s) {
-    if (b->depth < 64) return launch_sobb<LEAF, ANY, COUNT, 64>(b, rays, n, hits, occ, flags, counters, s);
-    if (b->depth < 128) return launch_sobb<LEAF, ANY, COUNT, 128>(b, rays, n, hits, occ, flags, counters, s);
-    return launch_sobb<LEAF, ANY, COUNT, 512>(b, rays, n, hits, occ, flags, counters, s);
+    if (b->depth < 64) return launch_sobb<LEAF, ANY, 64>(b, rays, n, hits, occ, flags, counters, s);
+    if (b->depth < 128) return launch_sobb<LEAF, ANY, 128>(b, rays, n, hits, occ, flags, counters, s);
+    return launch_sobb<LEAF, ANY, 512>(b, rays, n, hits, occ, flags, counters, s);
 }
 
 DeviceProbe g_triples_uploaded;  // per device: the table lives in each device's constant memory
@@ -748,15 +819,11 @@ dipl_status trace_sobb(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_
                        uint32_t flags, unsigned long long* counters, bool any, cudaStream_t s) {
     if (any)
         return leaf_test == DIPL_LEAF_REF_MT
-                   ? launch_sobb_stack<DIPL_LEAF_REF_MT, true, false>(b, rays, n, nullptr, occ, flags, nullptr, s)
-                   : launch_sobb_stack<DIPL_LEAF_WATERTIGHT, true, false>(b, rays, n, nullptr, occ, flags, nullptr, s);
-    if (counters)
-        return leaf_test == DIPL_LEAF_REF_MT
-                   ? launch_sobb_stack<DIPL_LEAF_REF_MT, false, true>(b, rays, n, hits, nullptr, flags, counters, s)
-                   : launch_sobb_stack<DIPL_LEAF_WATERTIGHT, false, true>(b, rays, n, hits, nullptr, flags, counters, s);
+                   ? launch_sobb_stack<DIPL_LEAF_REF_MT, true>(b, rays, n, nullptr, occ, flags, nullptr, s)
+                   : launch_sobb_stack<DIPL_LEAF_WATERTIGHT, true>(b, rays, n, nullptr, occ, flags, nullptr, s);
     return leaf_test == DIPL_LEAF_REF_MT
-               ? launch_sobb_stack<DIPL_LEAF_REF_MT, false, false>(b, rays, n, hits, nullptr, flags, nullptr, s)
-               : launch_sobb_stack<DIPL_LEAF_WATERTIGHT, false, false>(b, rays, n, hits, nullptr, flags, nullptr, s);
+               ? launch_sobb_stack<DIPL_LEAF_REF_MT, false>(b, rays, n, hits, nullptr, flags, counters, s)
+               : launch_sobb_stack<DIPL_LEAF_WATERTIGHT, false>(b, rays, n, hits, nullptr, flags, counters, s);
 }
 
 }  // namespace dipl
