@@ -519,19 +519,16 @@ struct QuadWork : RefWork<STACK, kQuadShort> {
         float key[4];
         int ref[4];
         quad_children(quads, this->cur, r, lim, key, ref);
-        this->cur = kRefPop;
-        if (key[0] < kMiss) {
-            if (this->sp + 3 <= kQuadShort) {
-                if (key[3] < kMiss) this->push_short(ref[3]);
-                if (key[2] < kMiss) this->push_short(ref[2]);
-                if (key[1] < kMiss) this->push_short(ref[1]);
-            } else {
-                if (key[3] < kMiss) this->push(ref[3]);
-                if (key[2] < kMiss) this->push(ref[2]);
-                if (key[1] < kMiss) this->push(ref[1]);
-            }
-            this->cur = ref[0];
+        if (this->sp + 3 <= kQuadShort) {  // stored past the top either way
+            this->push_short(ref[3], key[3] < kMiss);
+            this->push_short(ref[2], key[2] < kMiss);
+            this->push_short(ref[1], key[1] < kMiss);
+        } else {
+            if (key[3] < kMiss) this->push(ref[3]);
+            if (key[2] < kMiss) this->push(ref[2]);
+            if (key[1] < kMiss) this->push(ref[1]);
         }
+        this->cur = key[0] < kMiss ? ref[0] : kRefPop;
         this->advance(bot);
     }
 };

@@ -355,42 +355,39 @@ struct RefWork {
         cur = ref, held = 0;
         if (ref < 0) held = ref, cur = kRefIdle;
     }
-    __device__ __forceinline__ void push_short(int ref) { column[sp++ * kTraceThreads] = ref; }
+    __device__ __forceinline__ void push_short(int ref, bool on) {
+        column[sp * kTraceThreads] = ref;
+        sp += on ? 1 : 0;
+    }
     __device__ __forceinline__ void push(int ref) {
         if (sp < SHORT) column[sp * kTraceThreads] = ref;
         else rest[sp - SHORT] = ref;
         ++sp;
     }
-    // Pops until a node comes up, `held` and cur both hold a leaf, or the stack is down to `bot`.
+    __device__ __forceinline__ int pop(int bot) {
+        int ref = kRefIdle;
+        if (sp > bot) {
+            --sp;
+            ref = column[min(sp, SHORT - 1) * kTraceThreads];
+            if (sp >= SHORT) ref = rest[sp - SHORT];
+        }
+        return ref;
+    }
+    // After cur was entered (or set to kRefPop): a leaf moves to a free `held`, and cur is popped where it is empty. Two
+    // pops at most: the second leaf waits in cur.
     __device__ __forceinline__ void advance(int bot) {
-        for (;;) {
-            if (cur == kRefPop) {
-                if (sp <= bot) {
-                    cur = kRefIdle;
-                    return;
-                }
-                --sp;
-                cur = sp < SHORT ? column[sp * kTraceThreads] : rest[sp - SHORT];
-            }
-            if (cur >= 0 || held != 0) return;
+        if (cur == kRefPop) cur = pop(bot);
+        if (cur < 0 && held == 0) {
             held = cur;
-            cur = kRefPop;
+            cur = pop(bot);
         }
     }
     template <class R>
     __device__ __forceinline__ void leaf(R& r, int bot) {
         const int first = leaf_first(held), cnt = leaf_count(held);
         if (cnt > 0) r.test(tris, first, backface);  // an unused child slot has no triangles
-        if (cnt > 1) {
-            held = make_leaf_ref(first + 1, cnt - 1);
-        } else {
-            held = 0;
-            if (cur < 0) {
-                held = cur;
-                cur = kRefPop;
-                advance(bot);
-            }
-        }
+        held = cnt > 1 ? make_leaf_ref(first + 1, cnt - 1) : 0;
+        advance(bot);
     }
 };
 
