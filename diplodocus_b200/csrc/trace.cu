@@ -13,7 +13,7 @@
 // the best t by more than 1e-5 relative, so a node can never be skipped for rounding of its own box.
 #include <limits>
 
-#include "traverse.cuh"
+#include "traverse_pool.cuh"
 
 namespace dipl {
 namespace {
@@ -428,25 +428,26 @@ __global__ void __launch_bounds__(kTraceThreads) tail_kernel(const BNode* __rest
 
 // ---- 4-wide traversal -------------------------------------------------------------------------------------------
 // Closest and any hits over QNodes. What bounds it: instruction issue and the L1 data pipe (one cycle per lane and
-// load instruction, whatever its width), with a third to a half of the lanes idle because the lanes of a warp are at
-// different kinds of work. Hence: nodes of 64 bytes in two loads for four children, triangles in two loads, a stack
-// entry of one word (no entry distance: on the soup 96% of the popped entries are visited anyway, and the distances
-// cost a third of the stack's shared memory and 1.3x of the time), one node or one triangle per lane and step, one
-// leaf held back per lane so that it goes on with nodes until enough lanes of the warp hold one, and rays shared by
+// load instruction, whatever its width), and lanes that are at different kinds of work. Hence: nodes of 64 bytes in two
+// loads for four children, triangles in two loads, a stack entry of one word (no entry distance: on the soup 90% of the
+// popped entries are visited anyway, and the distances cost a third of the stack's shared memory and 1.3x of the time),
+// children stored at their place by distance instead of sorted (4M soup 9.3 -> 9.1 ms), one node per lane and step,
+// leaves tested by any lane of the warp (trace_batch_pool) or held back by their own (trace_batch), and rays shared by
 // all lanes of the warp when few are left. Measured against the binary traversal it replaces (node visits of the
 // pre-split soup 359 -> 192 a ray, L1 cycles 1474 -> 760): 4M-triangle soup, 2M rays in the coherent order 15.2 ->
-// 11.2 ms; 16M soup, 16M rays 127 -> 90 ms; 1M sphere, 4M rays 0.52 -> 0.38 ms; 4096 rays of a small frame 60 -> 28 us.
+// 9.1 ms; 16M soup, 16M rays 127 -> 75 ms; 1M sphere, 4M rays 0.52 -> 0.32 ms; 4096 rays of a small frame 60 -> 28 us.
 constexpr float kMiss = 3.40282346638528859812e+38f;  // entry distance of a child that is not entered
-// Stack entries per thread in shared memory: 24 with more blocks per SM and 16 were slower (soup 12.2 and 12.9 against
-// 11.3 ms).
+// Stack entries per thread in shared memory. Held leaves: 24 with more blocks per SM and 16 were slower (soup 12.2 and 12.9
+// against 11.3 ms). Pool: only nodes are on the stack, and rays and pool take 14 KB a block; 32 is no faster.
 constexpr int kQuadShort = 32;
+constexpr int kQuadPoolShort = 24;
 
 // Byte k of a plane word as the float 32768 + byte.
 __device__ __forceinline__ float quad_plane(uint32_t w, int k) {
     return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7504u | (uint32_t)(k << 4)));
 }
 
-// The children of a node by entry distance (kMiss when not entered), nearest first, and their references.
+// The entry distances of a node's children (kMiss when not entered) and their references.
 //
 // A plane at p + Q s (Q = 32768 + byte) is met at t = (p - o) / d + Q (s / d). With a = p - o in FP32 and C = a / d
 // the rounding of a and C is at most 2^-23 |C|; near planes move back and far planes on by 2^-22 |C|. What is
@@ -481,21 +482,42 @@ __device__ __forceinline__ void quad_children(const QNode* __restrict__ quads, i
         const float tnx = __fmaf_rn(quad_plane(nx, k), Sx, nCx), tfx = __fmaf_rn(quad_plane(fx, k), Sx, fCx);
         const float tny = __fmaf_rn(quad_plane(ny, k), Sy, nCy), tfy = __fmaf_rn(quad_plane(fy, k), Sy, fCy);
         const float tnz = __fmaf_rn(quad_plane(nz, k), Sz, nCz), tfz = __fmaf_rn(quad_plane(fz, k), Sz, fCz);
-        const float tn = fmaxf(max3(tnx, tny, tnz), r.tmin);
+        const float tn = max3(max3(tnx, tny, tnz), r.tmin, -kMiss);
         const float tf = fminf(min3(tfx, tfy, tfz), lim);
         key[k] = tn <= __fmaf_rn(fabsf(tf), 2e-6f, tf) ? tn : kMiss;
     }
-    auto order = [&](int i, int j) {
-        const bool swap = key[j] < key[i];
-        const float a = swap ? key[j] : key[i], b = swap ? key[i] : key[j];
-        const int c = swap ? ref[j] : ref[i], d = swap ? ref[i] : ref[j];
-        key[i] = a, key[j] = b, ref[i] = c, ref[j] = d;
-    };
-    order(0, 1);
-    order(2, 3);
-    order(0, 2);
-    order(1, 3);
-    order(1, 2);
+}
+
+// The places of n children on the stack, the farthest first: a child's place is the number of children farther away. Of
+// those that are not pushed, key is -inf (those of entered children are finite), so that they count as nearer.
+__device__ __forceinline__ void quad_places(const float (&key)[4], int (&at)[4]) {
+    const int c01 = key[0] < key[1], c02 = key[0] < key[2], c03 = key[0] < key[3], c12 = key[1] < key[2],
+              c13 = key[1] < key[3], c23 = key[2] < key[3];
+    at[0] = c01 + c02 + c03;
+    at[1] = 1 - c01 + c12 + c13;
+    at[2] = 2 - c02 - c12 + c23;
+    at[3] = 3 - c03 - c13 - c23;
+}
+
+// Pushes the children whose key is not -inf, the nearest last.
+template <class V>
+__device__ __forceinline__ void quad_push(V& v, const float (&key)[4], const int (&ref)[4]) {
+    const float none = __int_as_float(0xFF800000);
+    int at[4], n = 0;
+    quad_places(key, at);
+    if (v.sp + 4 <= V::kShort) {
+        int* const top = v.column + v.sp * kTraceThreads;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (key[k] != none) top[at[k] * kTraceThreads] = ref[k];
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (key[k] != none) v.put(v.sp + at[k], ref[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) n += key[k] != none ? 1 : 0;
+    v.sp += n;
 }
 
 template <int STACK>
@@ -511,7 +533,7 @@ struct QuadWork : RefWork<STACK, kQuadShort> {
     }
     template <class R>
     __device__ __forceinline__ void node(const R& r, float lim, int bot) {
-        if (this->cur >= num_nodes || this->sp + 3 > STACK) {  // only a corrupted tree gets here
+        if (this->cur >= num_nodes || this->sp + 4 > STACK) {  // only a corrupted tree gets here
             this->bad = true;
             this->drop();
             return;
@@ -519,32 +541,62 @@ struct QuadWork : RefWork<STACK, kQuadShort> {
         float key[4];
         int ref[4];
         quad_children(quads, this->cur, r, lim, key, ref);
-        if (this->sp + 3 <= kQuadShort) {  // stored past the top either way
-            this->push_short(ref[3], key[3] < kMiss);
-            this->push_short(ref[2], key[2] < kMiss);
-            this->push_short(ref[1], key[1] < kMiss);
-        } else {
-            if (key[3] < kMiss) this->push(ref[3]);
-            if (key[2] < kMiss) this->push(ref[2]);
-            if (key[1] < kMiss) this->push(ref[1]);
-        }
-        this->cur = key[0] < kMiss ? ref[0] : kRefPop;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) key[k] = key[k] < kMiss ? key[k] : __int_as_float(0xFF800000);
+        quad_push(*this, key, ref);
+        this->cur = kRefPop;
         this->advance(bot);
     }
 };
 
-template <int LEAF, bool ANY, bool PERSIST, int STACK>
+// With the leaves in the warp's pool: only nodes go on the stack.
+template <int STACK>
+struct QuadPoolWork : RefStack<STACK, kQuadPoolShort> {
+    const QNode* quads;
+
+    __device__ __forceinline__ void begin(const NodeRay&) { this->cur = this->root; }
+    __device__ __forceinline__ void take(const NodeRay&, int thread, int entry, int) {
+        this->cur = this->entry_of(thread, entry);
+    }
+    __device__ __forceinline__ void node(const NodeRay& r, float lim, int bot, int (&lf)[kStepLeaves]) {
+        if (!this->check(4, lf)) return;
+        float key[4];
+        int ref[4];
+        quad_children(quads, this->cur, r, lim, key, ref);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool hit = key[k] < kMiss;
+            lf[k] = hit && ref[k] < 0 ? ref[k] : 0;
+            key[k] = hit && ref[k] >= 0 ? key[k] : __int_as_float(0xFF800000);
+        }
+        quad_push(*this, key, ref);
+        this->pop(bot);
+    }
+};
+
+template <bool PERSIST, int STACK>
 __global__ void __launch_bounds__(kTraceThreads, PERSIST ? 8 : 9) quad_trace_kernel(
     const QNode* __restrict__ quads, const float4* __restrict__ tris, int root, int num_nodes, uint32_t flags, Batch B) {
     __shared__ int s_stack[kQuadShort * kTraceThreads];
-    __shared__ SharedRays<ANY> S;
+    __shared__ SharedRays<false> S;
     int rest[STACK - kQuadShort];
     QuadWork<STACK> v;
     v.tris = tris, v.column = s_stack + threadIdx.x, v.rest = rest, v.root = root;
     v.backface = (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u;
     v.quads = quads, v.num_nodes = num_nodes;
-    LaneRay<LEAF, ANY> r{};
-    trace_batch<LEAF, ANY, PERSIST>(v, r, S, B);
+    LaneRay<DIPL_LEAF_REF_MT, false> r{};
+    trace_batch<DIPL_LEAF_REF_MT, false, PERSIST>(v, r, S, B);
+}
+
+template <int LEAF, bool ANY, bool PERSIST, int STACK>
+__global__ void __launch_bounds__(kTraceThreads, 7) quad_pool_kernel(  // 8: frames +6%
+    const QNode* __restrict__ quads, const float4* __restrict__ tris, int root, int num_nodes, uint32_t flags, Batch B) {
+    __shared__ int s_stack[kQuadPoolShort * kTraceThreads];
+    __shared__ PoolRays<LEAF, ANY> S;
+    int rest[STACK - kQuadPoolShort];
+    QuadPoolWork<STACK> v;
+    v.column = s_stack + threadIdx.x, v.rest = rest, v.root = root, v.quads = quads, v.num_nodes = num_nodes;
+    trace_batch_pool<LEAF, ANY, PERSIST>(v, S, tris, (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u, B);
 }
 
 // ---- ray order ----------------------------------------------------------------------------------------
@@ -672,6 +724,13 @@ dipl_status launch_trace(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dip
     return DIPL_OK;
 }
 
+// Closest hits with the leaf test that keeps its state in few registers (ref_mt) and more rays than this run on the
+// loop whose lanes hold their leaves. Pool against held leaves, 3M-triangle soup and 1M sphere in the given order: 100k
+// rays 318 against 391 us and 55 against 64, 400k 977 against 979 and 87 against 86, 1.6M 3.62 against 3.43 ms and 163
+// against 166 us, 16M soup, 16M sorted rays 85 against 75 ms (the pool's rays leave room for 28 warps instead of 36, and
+// deep traversals wait for memory). The watertight test gains at all sizes: 2M-triangle soup, 2M rays 4.22 -> 4.0 ms.
+constexpr int64_t kPoolRays = 1 << 19;
+
 template <int LEAF, bool ANY, int STACK>
 dipl_status launch_quad(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ,
                         uint32_t flags, cudaStream_t s) {
@@ -685,11 +744,15 @@ dipl_status launch_quad(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl
         }
     }
     Batch B{rays, n, hits, occ, ro.order, b->d_err, steps_bound(num_nodes, b->num_refs), 32, num_nodes < 0};
-    launch_batch<quad_trace_kernel<LEAF, ANY, false, STACK>, quad_trace_kernel<LEAF, ANY, true, STACK>>(
-        n, ro.order != nullptr, [&](auto kernel, unsigned grid, int group) {
-            B.group = group;
-            kernel<<<grid, kTraceThreads, 0, s>>>(b->quads, b->tris, b->root, num_nodes, flags, B);
-        });
+    auto launch = [&](auto kernel, unsigned grid, int group) {
+        B.group = group;
+        kernel<<<grid, kTraceThreads, 0, s>>>(b->quads, b->tris, b->root, num_nodes, flags, B);
+    };
+    if (!ANY && LEAF == DIPL_LEAF_REF_MT && n > kPoolRays)
+        launch_batch<quad_trace_kernel<false, STACK>, quad_trace_kernel<true, STACK>>(n, ro.order != nullptr, launch);
+    else
+        launch_batch<quad_pool_kernel<LEAF, ANY, false, STACK>, quad_pool_kernel<LEAF, ANY, true, STACK>>(
+            n, ro.order != nullptr, launch);
     note_launches();
     const cudaError_t e = cudaGetLastError();
     if (ro.mem) device_free(ro.mem, s);

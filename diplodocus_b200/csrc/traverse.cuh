@@ -355,15 +355,11 @@ struct RefWork {
         cur = ref, held = 0;
         if (ref < 0) held = ref, cur = kRefIdle;
     }
-    __device__ __forceinline__ void push_short(int ref, bool on) {
-        column[sp * kTraceThreads] = ref;
-        sp += on ? 1 : 0;
+    __device__ __forceinline__ void put(int at, int ref) {
+        if (at < SHORT) column[at * kTraceThreads] = ref;
+        else rest[at - SHORT] = ref;
     }
-    __device__ __forceinline__ void push(int ref) {
-        if (sp < SHORT) column[sp * kTraceThreads] = ref;
-        else rest[sp - SHORT] = ref;
-        ++sp;
-    }
+    __device__ __forceinline__ void push(int ref) { put(sp++, ref); }
     __device__ __forceinline__ int pop(int bot) {
         int ref = kRefIdle;
         if (sp > bot) {

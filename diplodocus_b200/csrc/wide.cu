@@ -12,7 +12,7 @@
 // scale 2^e with extent / 2^e <= 255; child bounds q_lo = floor, q_hi = ceil, then adjusted until the FP32
 // decode fmaf(q, 2^e, p) lies outside the padded child box. The traversal decodes with the same fmaf, so
 // every decoded box contains its (already padded) child box: no ray can lose a hit against the FP32 nodes.
-#include "traverse.cuh"
+#include "traverse_pool.cuh"
 
 namespace dipl {
 namespace {
@@ -584,13 +584,13 @@ __global__ void __launch_bounds__(kTraceThreads, kWTraceMinBlocks) wide_trace_ke
 }
 
 // ------------------------------------------------------------------------------------------------
-// The uncounted traversal (trace_batch over the same nodes, groups and octant order). The counted kernels spend a
+// The uncounted traversal (trace_batch_pool over the same nodes, groups and octant order). The counted kernels spend a
 // quarter of their instructions on byte conversions (a quarter-rate unit, 42% busy), a lane tests all triangles of a
 // node while its warp waits (10 of 32 lanes active) and a warp waits for its longest ray. Here a byte becomes a float
-// by one byte permute (32768 + byte, as in QNode), planes are met at one FMA, triangles wait as bits while the lane
-// goes on with nodes, and the warp's last rays are shared. 2M-triangle soup, 2M sorted rays: 14.3 -> 10.1 ms; 1M sphere,
-// 4M rays in the given order 0.81 -> 0.39 ms. Now bound by issue slots (80%) and the ALU pipe (65%: permutes, minima); 7
-// blocks of 128 per SM, 8 spill (10.7 ms) and 6 hide less (10.7 ms).
+// by one byte permute (32768 + byte, as in QNode), planes are met at one FMA, triangles go to the warp's pool, four a
+// step, and the warp's last rays are shared. 2M-triangle soup, 2M sorted rays: 14.3 -> 8.6 ms; 1M sphere, 4M rays in the
+// given order 0.81 -> 0.36 ms. Now bound by issue slots and the ALU pipe (permutes, minima); 7 blocks of 128 per SM, 8
+// spill and 6 hide less.
 // ------------------------------------------------------------------------------------------------
 constexpr int kWideShort = 12;  // stack groups per thread in shared memory (one per wide level)
 
@@ -656,27 +656,25 @@ __device__ __forceinline__ WideHits wide_node_entered(const WNode* __restrict__ 
     return out;
 }
 
-// The lane's work: a node, the triangles it tests next and those of the node after that (as bits from a base), and the
-// stack of groups.
+// The lane's work: a node, the last node's triangles that are not in the pool yet (as bits from a base), and the stack
+// of groups.
 template <int STACK>
 struct WideWork {
     static constexpr int kShort = kWideShort;
     const WNode* nodes;
-    const float4* tris;
     int2* column;  // this thread's stack column in shared memory
     int2* rest;    // groups from kShort on
     int root, num_nodes;
-    bool backface;
     bool bad = false;
     int current = -1;
-    int held_base = 0, next_base = 0;
-    uint32_t held = 0u, next = 0u;
+    int held_base = 0;
+    uint32_t held = 0u;
     uint32_t oct = 0u, steps = 0;
     int sp = 0;
 
-    __device__ __forceinline__ bool has_node() const { return current >= 0 && next == 0u; }
-    __device__ __forceinline__ bool has_leaf() const { return held != 0u; }
-    __device__ __forceinline__ void drop() { current = -1, held = next = 0u; }
+    __device__ __forceinline__ bool has_node() const { return current >= 0 || held != 0u; }
+    __device__ __forceinline__ void drop() { current = -1, held = 0u; }
+    __device__ __forceinline__ void clear() { drop(), sp = 0; }
     template <class R>
     __device__ __forceinline__ void set_octant(const R& r) {
         oct = (r.inv.x < 0.0f ? 1u : 0u) | (r.inv.y < 0.0f ? 2u : 0u) | (r.inv.z < 0.0f ? 4u : 0u);
@@ -710,36 +708,35 @@ struct WideWork {
     template <class R>
     __device__ __forceinline__ void take(const R& r, int thread, int entry, int) {
         set_octant(r);
-        held = next = 0u;
         int2 e = column[entry * kTraceThreads + thread - (int)threadIdx.x];
         current = first_child(e);
         if ((uint32_t)e.y >> 8) column[0] = e, sp = 1;
     }
     template <class R>
-    __device__ __forceinline__ void node(const R& r, float lim, int bot) {
-        if (current >= num_nodes || sp >= STACK) {  // only a corrupted tree gets here
-            bad = true;
-            drop();
-            return;
-        }
-        const WideHits h = wide_node_entered(nodes, current, r, oct, lim);
-        if (h.tris) {
-            if (held == 0u) held = h.tris, held_base = h.tri_base;
-            else next = h.tris, next_base = h.tri_base;
-        }
-        if (h.inner) {
-            int2 e = make_int2(h.child_base, (int)((h.inner << 8) | h.imask));
-            current = first_child(e);
-            if ((uint32_t)e.y >> 8) set(sp++, e);
+    __device__ __forceinline__ void node(const R& r, float lim, int bot, int (&lf)[kStepLeaves]) {
+        if (held == 0u) {
+            if (current >= num_nodes || sp >= STACK) {  // only a corrupted tree gets here
+                bad = true;
+                drop();
+                return;
+            }
+            const WideHits h = wide_node_entered(nodes, current, r, oct, lim);
+            held = h.tris, held_base = h.tri_base;
+            if (h.inner) {
+                int2 e = make_int2(h.child_base, (int)((h.inner << 8) | h.imask));
+                current = first_child(e);
+                if ((uint32_t)e.y >> 8) set(sp++, e);
+            } else {
+                pop(bot);
+            }
         } else {
-            pop(bot);
+            --steps;  // a node's step goes on
         }
-    }
-    template <class R>
-    __device__ __forceinline__ void leaf(R& r, int) {
-        r.test(tris, held_base + __ffs(held) - 1, backface);
-        held &= held - 1u;
-        if (held == 0u) held = next, held_base = next_base, next = 0u;
+#pragma unroll
+        for (int k = 0; k < kStepLeaves; ++k) {
+            if (held) lf[k] = make_leaf_ref(held_base + __ffs(held) - 1, 1);
+            held &= held - 1u;
+        }
     }
 };
 
@@ -748,13 +745,11 @@ __global__ void __launch_bounds__(kTraceThreads, 7) wide_batch_kernel(const WNod
                                                                       const float4* __restrict__ tris, int root,
                                                                       int num_nodes, uint32_t flags, Batch B) {
     __shared__ int2 s_stack[kWideShort * kTraceThreads];
-    __shared__ SharedRays<ANY> S;
+    __shared__ PoolRays<LEAF, ANY> S;
     int2 rest[STACK - kWideShort];
     WideWork<STACK> v;
-    v.nodes = nodes, v.tris = tris, v.column = s_stack + threadIdx.x, v.rest = rest, v.root = root;
-    v.num_nodes = num_nodes, v.backface = (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u;
-    LaneRay<LEAF, ANY> r{};
-    trace_batch<LEAF, ANY, PERSIST>(v, r, S, B);
+    v.nodes = nodes, v.column = s_stack + threadIdx.x, v.rest = rest, v.root = root, v.num_nodes = num_nodes;
+    trace_batch_pool<LEAF, ANY, PERSIST>(v, S, tris, (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u, B);
 }
 
 template <int LEAF, int STACK>

@@ -98,3 +98,24 @@ def test_deep_trees(name, count, least):
     rays[:, 0:3] *= 1.25 ** -(np.arange(4096, dtype=np.float32)[:, None] % count)
     h = check(bvh, rays, leaf_test="watertight")
     assert int((h.prim >= 0).sum()) > 100
+
+
+# Closest hits of the binary layout change from pooled to held leaves above 2^19 rays.
+@pytest.mark.parametrize("n", [1 << 19, (1 << 19) + 1])
+@pytest.mark.parametrize("leaf", [2, 8])
+def test_binary_layout_around_the_pool_limit(n, leaf):
+    bvh = build(S.soup(5000, seed=4), T.kPlocEmc, max_triangles_per_leaf=leaf)
+    rays = S.random_rays(n, seed=5)
+    rays[: n // 4, 3] = -np.inf
+    rays[n // 4: n // 2, 3] = -0.5
+    h = check(bvh, rays)
+    assert 0 < int((h.prim >= 0).sum()) < n
+
+
+@pytest.mark.parametrize("name", list(LAYOUTS))
+def test_unbounded_intervals(name):
+    rays = S.random_rays(5000, seed=5)
+    rays[:2500, 3] = -np.inf
+    rays[1250:, 7] = np.inf
+    for lt in ("ref_mt", "watertight"):
+        check(make(name, S.soup(5000, seed=4)), rays, leaf_test=lt)
