@@ -299,18 +299,18 @@ def cpu_baseline_and_parity(tris, rays_np, gpu_hits_np, args, threads):
 # DRAM bytes (read + write) per unit measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum, one pass) on
 # the current kernels, per ray of one closest-hit trace and per triangle of one build, for the configuration each
 # was captured with (split budget, ray order, size); other configurations report no traffic. Soup trace: the full
-# 16M-triangle, 16M-ray launch, 14.71 GB read + 0.84 GB written (profiles/trace_dram_soup16m.md).
+# 16M-triangle, 16M-ray launch, 10.46 GB read + 0.54 GB written (profiles/trace_dram_soup16m.md).
 MEASURED_TRAFFIC = {("soup16m", "emc60", "trace"): {"split_budget": 40, "order": "coherent", "triangles": 16777216,
-                                                    "per_unit": (14.71e9 + 0.845e9) / 16777216},
-                    # the first build of the run, all 34 launches (profiles/dram_traffic_build_soup16m.md)
+                                                    "per_unit": (10.46e9 + 0.538e9) / 16777216},
+                    # the first build of the run, all 27 launches (profiles/dram_traffic_build_soup16m.md)
                     ("soup16m", "emc60", "build"): {"split_budget": 40, "order": "coherent", "triangles": 16777216,
-                                                    "per_unit": (22778e6 + 7764e6) / 16777216},
+                                                    "per_unit": (22974e6 + 6345e6) / 16777216},
                     ("displaced_sphere", "morton30", "build"): {"split_budget": 0, "order": "given",
                                                                 "triangles": 1046528,
-                                                                "per_unit": (502e6 + 71e6) / 1046528},
+                                                                "per_unit": (478e6 + 49e6) / 1046528},
                     ("displaced_sphere", "morton30", "trace"): {"split_budget": 0, "order": "given",
                                                                 "triangles": 1046528,
-                                                                "per_unit": (284.2e6 + 74.6e6 + 28.5e6 + 0.2e6)
+                                                                "per_unit": (240.6e6 + 57.3e6)
                                                                 / 4194304}}
 
 
@@ -345,7 +345,9 @@ def build_bytes_per_tri(code_type, digit_bits=8, node_bytes_per_tri=None, leaves
 
 def trace_bytes_per_ray(visits, tests, node_bytes):
     """Algorithmic bytes of one closest-hit ray: the ray in, the hit out, every node visited, every triangle
-    tested (the counts come from the counting build of the same kernel on the same rays)."""
+    tested. The counts are those of the counted traversal of the layout's own nodes on the same rays; the timed kernel
+    of the binary layout reads 4-wide nodes of the same size, about half as many, so that its fraction of a peak can
+    pass 1 without more bytes moved (`traffic` has the measured ones)."""
     return 32 + 16 + visits * node_bytes + tests * 36
 
 
@@ -501,7 +503,7 @@ def run_gpu(args, rank, world, local_rank):
                   "frac": round(achieved_trace / peak, 4),
                   "traffic": (measured_traffic(args.workload, code, "trace", nr, split, order_name, n)
                               if args.leaf_test == "ref_mt" else None),
-                  "kernel": "closest-hit trace (trace_kernel + tail_kernel)", "ms": round(trace_s * 1e3, 4),
+                  "kernel": "closest-hit trace (quad_trace_kernel; bytes of the counted binary traversal)", "ms": round(trace_s * 1e3, 4),
                   "bytes_per_unit": round(ray_bytes, 1), "unit_of_bytes": "ray", "node_bytes": round(node_bytes, 1),
                   "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)"}
     line = {
