@@ -413,7 +413,8 @@ inline uint32_t steps_bound(int64_t nodes, int64_t triangles) {
 // run on resident warps that refill idle lanes, since their rays may differ most in length (1M sphere, 4M rays
 // 0.38 ms against 1.11 with one ray per lane; 1M occlusion rays 1.17 against 1.69; where all rays are alike one
 // ray per lane is a little faster: 1M primary rays 0.41 against 0.36). Sorted rays get one lane each: a warp's
-// rays are then of similar length and start together (4M-triangle soup 11.2 against 13.8 ms).
+// rays are then of similar length and start together (4M-triangle soup 11.2 against 13.8 ms). Both sides of each pair
+// with the 4-wide nodes and held leaves.
 template <auto ONE, auto MANY, class L>
 void launch_batch(int64_t n, bool sorted, L&& launch) {
     const int64_t warps = (int64_t)persistent_grid<ONE>() * (kTraceThreads / 32);

@@ -78,8 +78,9 @@ typedef enum dipl_leaf_test { DIPL_LEAF_REF_MT = 0, DIPL_LEAF_WATERTIGHT = 1 } d
  * (computed and sorted on the device inside the call), so that the rays of a warp start close together and head
  * the same way; each record still goes to its ray's index and the records are the same either way. Without it
  * the rays are traced in the order given. On a B200 it pays for incoherent batches (16M random rays in a
- * pre-split 16M-triangle soup: 163 ms against 211 ms) but not for camera-like rays that already come in order
- * (4M rays on a 1M-triangle sphere: the sort costs more than it saves), so it is an option of the call. */
+ * pre-split 16M-triangle soup: 75 ms against 146 ms) but not for camera-like rays that already come in order
+ * (4M rays on a 1M-triangle sphere: 1.07 ms against 0.33 ms, the sort costs more than it saves), so it is an
+ * option of the call. */
 #define DIPL_TRACE_COHERENT_ORDER 2u
 
 /* Build description. The three vertex arrays are the reference GPU scene's SoA positions
