@@ -132,9 +132,14 @@ __device__ __forceinline__ void trace_batch_pool(V& v, PoolRays<LEAF, ANY>& S, c
                         if (ANY) {
                             if (t < S.tmax[c]) S.open[c] = 0u;
                         } else {
-                            prim = __float_as_int(p0.w);
-                            key = ((unsigned long long)ordered_bits(t + 0.0f) << 32) | (unsigned)prim;
-                            if (key < S.best[c]) atomicMin(&S.best[c], key);
+                            const int id = __float_as_int(p0.w);
+                            key = ((unsigned long long)ordered_bits(t + 0.0f) << 32) | (unsigned)id;
+                            // Only what is below the word may win it: as it starts, it equals the key of primitive 0 at
+                            // t == tmax, which is no hit.
+                            if (key < S.best[c]) {
+                                prim = id;
+                                atomicMin(&S.best[c], key);
+                            }
                         }
                     }
                     --n, ++i;
