@@ -2120,7 +2120,10 @@ __device__ __forceinline__ QChild leaf_part(const float4* __restrict__ tris, con
 }
 
 // Frame and bytes of one axis. The bytes are chosen in FP64, where the distance of a plane from p in steps is off by
-// less than 2^-36 of a step (the boxes are padded by far more): every child's interval lies within its planes.
+// less than 2^-36 of a step (the boxes are padded by far more): every child's interval lies within its planes. 2^111 is
+// the largest step whose 33,023-fold is finite; where 255 of those don't reach (an extent above 6.6e35, a coordinate
+// below -2.5e38, a plane that padding made infinite) p = -inf, whose planes come out infinite on the open side or NaN
+// and so constrain no ray on this axis.
 __device__ __forceinline__ void quad_axis(const float* lo, const float* hi, uint32_t valid, float& p, uint32_t& ebias,
                                           uint32_t& qlo, uint32_t& qhi) {
     float mn = __int_as_float(0x7F800000), mx = __int_as_float(0xFF800000);
@@ -2148,7 +2151,11 @@ __device__ __forceinline__ void quad_axis(const float* lo, const float* hi, uint
             qlo |= (uint32_t)fmin(fmax(a, 0.0), 255.0) << (8 * k);
             qhi |= (uint32_t)fmin(fmax(b, 0.0), 255.0) << (8 * k);
         }
-        if (ok || eb >= 238u) break;
+        if (ok) break;
+        if (eb >= 238u) {
+            p = __int_as_float(0xFF800000);
+            break;
+        }
     }
     ebias = eb;
 }

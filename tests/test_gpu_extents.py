@@ -1,0 +1,50 @@
+"""GPU: scenes and rays near the ends of FP32's range. Every layout's traversal against the brute force over all triangles
+and against the counted traversal: quantised nodes and slab distances that overflow may cost visits, never a hit."""
+import numpy as np
+import pytest
+import torch
+
+from diplodocus_b200 import accel as A
+from diplodocus_b200 import scenes as S
+from gpu_util import build
+
+pytestmark = pytest.mark.gpu
+
+T = A.AccelerationStructureType
+LAYOUTS = {
+    "binary": dict(),
+    "sobb": dict(kind=T.kPlocSobb, kdop_size=14),
+}
+LEAF_TESTS = ("ref_mt", "watertight")
+
+
+def check(bvh, rays, leaf_test, many=False):
+    """`many`: once more with the rays repeated past 2^19, where the binary layout changes its loop."""
+    rd = torch.from_numpy(np.ascontiguousarray(rays, np.float32)).cuda()
+    want = bvh.Intersect(A.Stats(), rd, leaf_test=leaf_test, count=True)
+    got = bvh.Intersect(A.Stats(), rd, leaf_test=leaf_test)
+    occ = bvh.IntersectAny(A.Stats(), rd, leaf_test=leaf_test)
+    torch.cuda.synchronize()
+    bvh.check_errors()
+    assert torch.equal(got.raw, want.raw)
+    assert torch.equal(occ, want.prim >= 0)
+    if many:
+        times = (1 << 19) // len(rd) + 1
+        got = bvh.Intersect(A.Stats(), rd.repeat(times, 1), leaf_test=leaf_test)
+        assert torch.equal(got.raw, want.raw.repeat(times, 1))
+    return want
+
+
+@pytest.mark.parametrize("at", [-1e36, -1e37, -1e38, -3.4e38, 1e36, 3.4e38])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("name", list(LAYOUTS))
+def test_one_far_vertex(orc, name, axis, at):
+    tris = S.uv_sphere(32, 16, 1.0, displacement=0.1, seed=3)
+    tris[100, 1, axis] = at
+    bvh = build(tris, **LAYOUTS[name])
+    rays = S.sphere_inward_rays(3000, 9)
+    for k, leaf_test in enumerate(LEAF_TESTS):
+        h = check(bvh, rays, leaf_test, many=True)
+        truth = orc.brute(tris, rays, leaf_test=k)
+        assert int((truth.prim >= 0).sum()) > 100
+        np.testing.assert_array_equal(h.prim.cpu().numpy(), truth.prim)
