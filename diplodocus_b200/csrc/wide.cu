@@ -595,8 +595,11 @@ __global__ void __launch_bounds__(kTraceThreads, kWTraceMinBlocks) wide_trace_ke
 constexpr int kWideShort = 12;  // stack groups per thread in shared memory (one per wide level)
 
 // As wide_node_hits. A plane at p + q s is met at t = (p - o) / d + q (s / d) = C + q S; with Q = 32768 + q,
-// t = (C - 32768 S) + Q S. The rounding of p - o, C and the constant is at most 2^-22 of |C| + 32768 |S|, by which near
-// planes move back and far planes on (1/128 of a step and less); the rest is relative to t and covered by 2e-6.
+// t = c + Q S, c = C - 32768 S. The rounding of p - o and C is at most 2^-23 |C|, that of c and of c with its margin 2^-23
+// |c|: near planes move back and far planes on by 2^-22 of the larger, at least that much in all. (What remains of second
+// order when |C| and |c| are equal is relative to t, as |t| >= |C| then, and all that is covered by 2e-6.) 1e-36 stands for
+// the roundings of subnormal products. Where c overflows, as on an axis without direction in a scene of 3e16, so does its
+// margin, and the near plane comes out as -inf or NaN, the far one as +inf or NaN: they constrain nothing.
 template <class R>
 __device__ __forceinline__ WideHits wide_node_entered(const WNode* __restrict__ nodes, int node, const R& r,
                                                       uint32_t oct, float lim) {
@@ -607,9 +610,9 @@ __device__ __forceinline__ WideHits wide_node_entered(const WNode* __restrict__ 
     auto axis = [&](float p, uint32_t e, float o, float inv, float& S, float& n, float& f) {
         S = __fmul_rn(fabsf(__uint_as_float(e << 23)), inv);  // the next byte's low bit lands in the sign
         const float C = __fmul_rn(__fsub_rn(p, o), inv), c = __fmaf_rn(-32768.0f, S, C);
-        const float err = __fmaf_rn(fabsf(C), kE, fabsf(S) * (32768.0f * kE));
-        n = __fsub_rn(c, err);
-        f = __fadd_rn(c, err);
+        const float m = max3(fabsf(C), fabsf(c), 1e-36f);
+        n = __fmaf_rn(-kE, m, c);
+        f = __fmaf_rn(kE, m, c);
     };
     float Sx, nx, fx, Sy, ny, fy, Sz, nz, fz;
     axis(f0.x, eb, r.o.x, r.inv.x, Sx, nx, fx);

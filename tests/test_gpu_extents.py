@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
 T = A.AccelerationStructureType
 LAYOUTS = {
     "binary": dict(),
+    "wide": dict(layout="wide8_q8"),
     "sobb": dict(kind=T.kPlocSobb, kdop_size=14),
 }
 LEAF_TESTS = ("ref_mt", "watertight")
@@ -47,4 +48,29 @@ def test_one_far_vertex(orc, name, axis, at):
         h = check(bvh, rays, leaf_test, many=True)
         truth = orc.brute(tris, rays, leaf_test=k)
         assert int((truth.prim >= 0).sum()) > 100
+        np.testing.assert_array_equal(h.prim.cpu().numpy(), truth.prim)
+
+
+def scattered(count, extent, size, away, seed):
+    """Triangles of about `size` anywhere within +-extent, and for each a ray parallel to an axis towards its centroid from
+    `away` (towards the positive and the negative end in turn)."""
+    g = np.random.default_rng(seed)
+    centre = g.uniform(-extent, extent, (count, 1, 3)).astype(np.float32)
+    tris = (centre + g.uniform(-size, size, (count, 3, 3)).astype(np.float32)).astype(np.float32)
+    c = tris.astype(np.float64).mean(axis=1)
+    d = np.zeros((count, 3))
+    d[np.arange(count), np.arange(count) % 3] = np.where(np.arange(count) % 2, 1.0, -1.0)
+    return tris, S.pack_rays((c - away * d).astype(np.float32), d.astype(np.float32))
+
+
+@pytest.mark.parametrize("extent,size", [(1e8, 1e4), (3e16, 1e11), (1e18, 1e12)])
+@pytest.mark.parametrize("name", list(LAYOUTS))
+def test_axis_parallel_rays_in_large_scenes(orc, name, extent, size):
+    """A ray without a component on an axis has slab distances that overflow in scenes larger than 1e18 steps."""
+    tris, rays = scattered(3000, extent, size, 10.0 * size, seed=11)
+    bvh = build(tris, **LAYOUTS[name])
+    for k, leaf_test in enumerate(LEAF_TESTS):
+        h = check(bvh, rays, leaf_test)
+        truth = orc.brute(tris, rays, leaf_test=k)
+        assert int((truth.prim >= 0).sum()) > 500
         np.testing.assert_array_equal(h.prim.cpu().numpy(), truth.prim)
