@@ -29,6 +29,8 @@ __device__ __forceinline__ void ldg_v8(const void* p, float4& x, float4& y) {
         : "l"(p));
 }
 
+// ROUNDED: reciprocals rounded to nearest, those of directions above 8.5e37 subnormal (0 otherwise).
+template <bool ROUNDED = false>
 __device__ __forceinline__ RayState load_ray(const dipl_ray* rays, int64_t i) {
     const float4* r4 = reinterpret_cast<const float4*>(rays) + 2 * i;
     const float4 a = __ldg(r4), b = __ldg(r4 + 1);
@@ -42,7 +44,8 @@ __device__ __forceinline__ RayState load_ray(const dipl_ray* rays, int64_t i) {
     // their interval by 1e-6 relative: the hardware reciprocal (relative error below 2^-22) is well inside
     // that margin.
     auto safe = [](float x) { return fabsf(x) < 1e-20f ? copysignf(1e-20f, x) : x; };
-    r.inv = make_float3(rcp_approx(safe(r.d.x)), rcp_approx(safe(r.d.y)), rcp_approx(safe(r.d.z)));
+    auto rcp = [](float x) { return ROUNDED ? __frcp_rn(x) : rcp_approx(x); };
+    r.inv = make_float3(rcp(safe(r.d.x)), rcp(safe(r.d.y)), rcp(safe(r.d.z)));
     return r;
 }
 

@@ -46,6 +46,7 @@ struct PoolRays {
 //   node(ray, lim, bot, lf)  one step; up to kStepLeaves leaf references come back in lf (0: none); the stack is used down
 //                         to `bot`
 //   sp, kShort, steps, bad, take(ray, thread, entry, column)  as in trace_batch
+//   kRoundedInverse       load_ray's ROUNDED
 template <int LEAF, bool ANY, bool PERSIST, class V>
 __device__ __forceinline__ void trace_batch_pool(V& v, PoolRays<LEAF, ANY>& S, const float4* __restrict__ tris, bool backface,
                                             const Batch& B) {
@@ -65,7 +66,7 @@ __device__ __forceinline__ void trace_batch_pool(V& v, PoolRays<LEAF, ANY>& S, c
     bool working = false;  // this lane has a ray
     auto start_ray = [&](int64_t cand) {
         const int64_t my = B.order ? (int64_t)__ldg(B.order + cand) : cand;  // the ray's own index (hits go there)
-        const RayState q = load_ray(B.rays, my);
+        const RayState q = load_ray<V::kRoundedInverse>(B.rays, my);
         working = true;
         S.ray[threadIdx.x] = my;
         r.o = q.o, r.inv = q.inv, r.tmin = q.tmin;
@@ -290,6 +291,7 @@ __device__ __forceinline__ void trace_batch_pool(V& v, PoolRays<LEAF, ANY>& S, c
 template <int STACK, int SHORT>
 struct RefStack {
     static constexpr int kShort = SHORT;
+    static constexpr bool kRoundedInverse = false;
     int* column;  // this thread's stack column
     int* rest;    // entries from SHORT on: an array of the kernel's (inside this object it would keep the rest in memory)
     int root, num_nodes;

@@ -664,6 +664,7 @@ __device__ __forceinline__ WideHits wide_node_entered(const WNode* __restrict__ 
 template <int STACK>
 struct WideWork {
     static constexpr int kShort = kWideShort;
+    static constexpr bool kRoundedInverse = true;  // as the counted traversal: such rays meet the same children
     const WNode* nodes;
     int2* column;  // this thread's stack column in shared memory
     int2* rest;    // groups from kShort on

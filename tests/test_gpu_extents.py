@@ -74,3 +74,15 @@ def test_axis_parallel_rays_in_large_scenes(orc, name, extent, size):
         truth = orc.brute(tris, rays, leaf_test=k)
         assert int((truth.prim >= 0).sum()) > 500
         np.testing.assert_array_equal(h.prim.cpu().numpy(), truth.prim)
+
+
+@pytest.mark.parametrize("name", ["wide", "sobb"])  # the binary layout's reciprocal flushes such directions to zero
+def test_long_directions(orc, name):
+    """Directions whose reciprocals are subnormal (watertight: products in the other test overflow)."""
+    tris, rays = scattered(3000, 1e3, 0.3, 1e3, seed=12)
+    rays[:, 4:7] *= np.float32(1.5e38)
+    rays[:, 3] = 1e-42
+    h = check(build(tris, **LAYOUTS[name]), rays, "watertight")
+    truth = orc.brute(tris, rays, leaf_test=1)
+    assert int((truth.prim >= 0).sum()) > 500
+    np.testing.assert_array_equal(h.prim.cpu().numpy(), truth.prim)
