@@ -1751,6 +1751,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) hploc_kernel(HplocParams P) {
         const unsigned lm = __ballot_sync(full, leaves);
         if (leaves) S.exits[warp * kShare + exits + __popc(lm & lt)] = (unsigned)(l - b0) | ((unsigned)(r - b0) << 16);
         exits += __popc(lm);
+        __syncwarp();  // every lane's arrival and its fences before any lane of the warp loads a list
         process(todo, true, split);
     }
     __syncwarp();
