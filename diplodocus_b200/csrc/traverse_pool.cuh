@@ -150,6 +150,7 @@ __device__ __forceinline__ void trace_batch_pool(V& v, PoolRays<LEAF, ANY>& S, c
                     if (prim >= 0 && S.best[c] == key) S.hit[c] = make_float4(t, b1, b2, __int_as_float(prim));
                 }
                 if (!__any_sync(full, n > 0)) break;
+                __syncwarp();  // this round's reads and records before the next round's minima
             }
             head += 32;
         }
@@ -187,6 +188,7 @@ __device__ __forceinline__ void trace_batch_pool(V& v, PoolRays<LEAF, ANY>& S, c
         }
         __syncwarp();
         count = (int)S.leaves[threadIdx.x >> 5];
+        __syncwarp();  // read by every lane, before the next step counts on
         const uint32_t nodes = __ballot_sync(full, on && v.has_node());
         const int least = max(1, __popc(nodes));
         if (count >= least) test_leaves(least);
