@@ -54,7 +54,7 @@ class BvhInfo(C.Structure):
                 ("node_bytes", C.c_int64), ("triangle_bytes", C.c_int64), ("depth", C.c_int32),
                 ("ploc_iterations", C.c_int32), ("code_type", C.c_int32), ("bv_type", C.c_int32),
                 ("layout", C.c_int32), ("max_triangles_per_leaf", C.c_int32), ("nn_search_radius", C.c_int32),
-                ("kdop_size", C.c_int32), ("clustering", C.c_int32), ("reserved", C.c_int32)]
+                ("kdop_size", C.c_int32), ("clustering", C.c_int32), ("quad_nodes", C.c_int32)]
 
 
 class Limits(C.Structure):

@@ -192,7 +192,7 @@ class GpuPlocBvh:
         stats.accel_stats.inner_node_count = int(info.num_inner_nodes)
         stats.accel_stats.node_count = int(info.num_inner_nodes) * 2 + 1
         stats.accel_stats.leaf_node_count = stats.accel_stats.node_count - int(info.num_inner_nodes)
-        stats.accel_stats.memory_consumption = int(info.node_bytes + info.triangle_bytes)
+        stats.accel_stats.memory_consumption = int(info.node_bytes + 64 * info.quad_nodes + info.triangle_bytes)
         return self
 
     @classmethod

@@ -82,7 +82,8 @@ class GpuPlocBvh : public AccelerationStructure {
         stats.accel_stats.inner_node_count = static_cast<int>(info.num_inner_nodes);
         stats.accel_stats.node_count = static_cast<int>(2 * info.num_inner_nodes + 1);
         stats.accel_stats.leaf_node_count = static_cast<int>(info.num_inner_nodes + 1);
-        stats.accel_stats.memory_consumption = static_cast<int>(info.node_bytes + info.triangle_bytes);
+        stats.accel_stats.memory_consumption =
+            static_cast<int>(info.node_bytes + 64 * static_cast<int64_t>(info.quad_nodes) + info.triangle_bytes);
         stats.accel_stats.build_time =
             std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     }

@@ -309,6 +309,7 @@ dipl_status dipl_bvh_get_info(const dipl_bvh* b, dipl_bvh_info* info) {
     info->nn_search_radius = b->radius;
     info->kdop_size = b->kdop;
     info->clustering = b->clustering;
+    info->quad_nodes = b->quads ? (int32_t)b->num_nodes : 0;
     return DIPL_OK;
 }
 

@@ -131,12 +131,14 @@ typedef struct dipl_bvh_info {
     int64_t num_triangles;
     int64_t num_inner_nodes;     /* nodes of the traced layout */
     int64_t num_leaves;          /* clustering leaves: the triangles, and their pieces with pre-splitting */
-    int64_t node_bytes;          /* bytes of the traced node array */
+    int64_t node_bytes;          /* bytes of the layout's node array (dipl_bvh_download_layout), without quad_nodes */
     int64_t triangle_bytes;      /* bytes of the leaf triangle array (one record per clustering leaf) */
     int32_t depth;               /* levels of the clustering tree (bounds the traversal stack) */
     int32_t ploc_iterations;     /* PLOC: global iterations; HPLOC: iterations of all tree nodes, summed */
     int32_t code_type, bv_type, layout, max_triangles_per_leaf, nn_search_radius, kdop_size;
-    int32_t clustering, reserved; /* dipl_clustering (ABI version 2) */
+    int32_t clustering;          /* dipl_clustering (ABI version 2) */
+    int32_t quad_nodes;          /* 4-wide nodes of 64 bytes that the handle holds beside the binary layout's nodes:
+                                    uncounted traces walk these, counted ones the binary nodes; 0 = none */
 } dipl_bvh_info;
 
 /* Fills a description with the defaults (Morton30, AABB, binary, leaves < 4, r = 16, 32-DOP, auto, HPLOC, no
