@@ -2549,7 +2549,7 @@ static dipl_status count_references(BuildPlan& P, cudaStream_t stream) {
 }
 
 static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int count, cudaStream_t stream,
-                                bool own_summary) {
+                                bool own_summary, bool tight) {
     DIPL_CHECK_ARG(descs && count >= 1, "descs must be non-NULL and count >= 1");
     for (int i = 0; i < count; ++i) {
         dipl_status st = validate_desc(descs[i]);
@@ -2591,6 +2591,7 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
     P.out->kept = true;
     P.work = std::make_shared<Storage>();
     P.work->stream = stream;
+    P.out->exact = P.work->exact = tight;
     dipl_status st;
     P.K = P.N - P.m;
     P.Kalloc = std::max<long long>(P.K, 1);
@@ -2607,13 +2608,11 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
     std::memcpy(table.data(), P.meshes.data(), mesh_bytes);
     std::memcpy(table.data() + mesh_bytes, P.offsets.data(), table_bytes - mesh_bytes);
     unsigned char* d_table = nullptr;
-    W.reserve(&d_table, table_bytes);
-    W.reserve(&P.d_bounds, m);
-    W.reserve(&P.d_params, m);
-    // Scratch is sized by a bound on the references, at most split_budget percent more than the triangles, so that it is
-    // one block taken before they are counted; what the handles keep is taken after, by the count.
-    const long long N = P.split ? P.T + P.T * d0.split_budget / 100 : P.T, K = N - m, Kalloc = std::max<long long>(K, 1);
-    if (P.split) {
+    auto reserve_tables = [&]() {
+        W.reserve(&d_table, table_bytes);
+        W.reserve(&P.d_bounds, m);
+        W.reserve(&P.d_params, m);
+        if (!P.split) return;
         W.reserve(&P.pieces, P.T);
         W.reserve(&P.piece_first, P.T);
         W.reserve(&P.mesh_wsum, m);
@@ -2621,7 +2620,14 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
         W.reserve(&P.d_total, 4);
         W.reserve(&P.piece_scan, scan_scratch_bytes(P.T));
         W.reserve(&P.d_split_err, 4);
-    }
+    };
+    auto upload_tables = [&]() -> dipl_status {
+        P.d_meshes = reinterpret_cast<MeshDesc*>(d_table);
+        P.d_offsets = reinterpret_cast<long long*>(d_table + mesh_bytes);
+        if (!P.split) P.d_coffsets = P.d_offsets;
+        DIPL_CUDA(cudaMemcpyAsync(d_table, table.data(), table_bytes, cudaMemcpyHostToDevice, stream));
+        return DIPL_OK;
+    };
     P.code_bits = d0.code_type == DIPL_CODE_MORTON30 ? 30 : 60;
     while ((1ll << P.mesh_bits) < m) ++P.mesh_bits;
     P.key_bits = P.code_bits + P.mesh_bits;
@@ -2633,77 +2639,92 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
     P.key_bytes = P.key_bits <= 32 ? 4 : 8;
     P.digit_bits = d0.sort_digit_bits > 0 ? d0.sort_digit_bits : 8;
     const bool hier = d0.clustering == DIPL_CLUSTER_HPLOC;
+    const bool wide = d0.layout == DIPL_LAYOUT_WIDE8_Q8, sobb = d0.bv_type == DIPL_BV_SOBB;
     auto set_tiles = [&P](long long n) {
         P.B = ploc_block_for(P.d0.ploc_block_size, (int64_t)n);
         P.tiles0 = (int)((n + P.B * ploc_ipt_max(P.B) - 1) / (P.B * ploc_ipt_max(P.B)));
         P.tiles_max = (int)((n + P.B - 1) / P.B);
     };
-    set_tiles(N);
-    W.reserve((unsigned char**)&P.keys, N * P.key_bytes);
-    W.reserve((unsigned char**)&P.keys_sorted, N * P.key_bytes);
-    W.reserve((unsigned char**)&P.keys_alt, N * P.key_bytes);
-    W.reserve(&P.perm_alt, N);
-    W.reserve(&P.tbox, 2 * N);
-    for (int k = 0; k < 2; ++k) {  // the hierarchical clustering keeps only the roots in the second buffer
-        W.reserve(&P.c_lo[k], hier && k ? m : N);
-        W.reserve(&P.c_hi[k], hier && k ? m : N);
-        W.reserve(&P.c_in[k], hier && k ? m : N);
-    }
-    if (hier) {
-        W.reserve(&P.hp_cnt, N);
-        W.reserve(&P.hp_fid, N);
-    }
-    W.reserve(&P.rev_flags, Kalloc);
-    W.reserve(&P.contrib, N);
-    W.reserve(&P.owner_leaf, N);
-    W.reserve(&P.leaf_start_of, N + Kalloc);
-    // what a build starts from all ones (parents, arrivals) and from zero, each in one block: one memset
-    P.ones_bytes = sizeof(int) * (size_t)(N + Kalloc + (hier ? N : 0));
-    W.reserve(&P.parent, P.ones_bytes / sizeof(int));
-    P.summary_bytes = sizeof(RootInfo) * m + sizeof(double) * 2 * m + 16;
     auto pad = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t sort_bytes = pad(radix_sort_scratch_bytes(N, 0, P.key_bits, P.digit_bits));
-    const size_t height_bytes = hier ? pad(radix_sort_scratch_bytes(Kalloc, 0, 8, 8)) : 0;
-    const size_t scan_bytes = pad(scan_scratch_bytes(std::max(N, Kalloc)));
-    const size_t status_bytes = hier ? 0 : pad(sizeof(unsigned long long) * (2 * P.tiles_max + 2));
-    P.zero_bytes = pad(P.summary_bytes) + pad(sizeof(PlocCtrl)) + sort_bytes + height_bytes + 2 * scan_bytes + status_bytes;
-    W.reserve(&P.zero, P.zero_bytes);
-    const bool wide = d0.layout == DIPL_LAYOUT_WIDE8_Q8, sobb = d0.bv_type == DIPL_BV_SOBB;
-    if (wide) {  // the binary layout is only a step towards the kept one
-        W.reserve(&P.nodes, Kalloc);
-        W.reserve(&P.tris, 3 * N);
-        wide_reserve(P.wide, W, Kalloc);
-    }
-    if (sobb) {
-        if ((st = sobb_prepare(N, K, W, &P.sobb)) != DIPL_OK) return st;
+    P.summary_bytes = sizeof(RootInfo) * m + sizeof(double) * 2 * m + 16;
+    size_t sort_bytes = 0, height_bytes = 0, scan_bytes = 0, status_bytes = 0;
+    long long arrivals = 0;  // where they start in the block of ones
+    auto reserve_scratch = [&](long long N) -> dipl_status {  // for up to N references
+        const long long K = N - m, Kalloc = std::max<long long>(K, 1);
+        set_tiles(N);
+        W.reserve((unsigned char**)&P.keys, N * P.key_bytes);
+        W.reserve((unsigned char**)&P.keys_sorted, N * P.key_bytes);
+        W.reserve((unsigned char**)&P.keys_alt, N * P.key_bytes);
+        W.reserve(&P.perm_alt, N);
+        W.reserve(&P.tbox, 2 * N);
+        for (int k = 0; k < 2; ++k) {  // the hierarchical clustering keeps only the roots in the second buffer
+            W.reserve(&P.c_lo[k], hier && k ? m : N);
+            W.reserve(&P.c_hi[k], hier && k ? m : N);
+            W.reserve(&P.c_in[k], hier && k ? m : N);
+        }
+        if (hier) {
+            W.reserve(&P.hp_cnt, N);
+            W.reserve(&P.hp_fid, N);
+        }
+        W.reserve(&P.rev_flags, Kalloc);
+        W.reserve(&P.leaf_start_of, N + Kalloc);
+        // what a build starts from all ones (parents, arrivals) and from zero, each in one block: one memset
+        P.ones_bytes = sizeof(int) * (size_t)(N + Kalloc + (hier ? N : 0));
+        W.reserve(&P.parent, P.ones_bytes / sizeof(int));
+        arrivals = N + Kalloc;
+        sort_bytes = pad(radix_sort_scratch_bytes(N, 0, P.key_bits, P.digit_bits));
+        height_bytes = hier ? pad(radix_sort_scratch_bytes(Kalloc, 0, 8, 8)) : 0;
+        scan_bytes = pad(scan_scratch_bytes(std::max(N, Kalloc)));
+        status_bytes = hier ? 0 : pad(sizeof(unsigned long long) * (2 * P.tiles_max + 2));
+        P.zero_bytes = pad(P.summary_bytes) + pad(sizeof(PlocCtrl)) + sort_bytes + height_bytes + 2 * scan_bytes + status_bytes;
+        W.reserve(&P.zero, P.zero_bytes);
+        if (wide) {  // the binary layout is only a step towards the kept one
+            W.reserve(&P.nodes, Kalloc);
+            W.reserve(&P.tris, 3 * N);
+            wide_reserve(P.wide, W, Kalloc);
+        }
+        if (!sobb) return DIPL_OK;
         if (P.split) W.reserve(&P.slot_pos, N);
+        return sobb_prepare(N, K, W, &P.sobb);
+    };
+    // Scratch is sized by a bound on the references, at most split_budget percent more than the triangles, so that it is
+    // one block taken before they are counted (tight: after); what the handles keep is taken after, by the count.
+    const bool count_first = tight && P.split;
+    reserve_tables();
+    if (!count_first && (st = reserve_scratch(P.split ? P.T + P.T * d0.split_budget / 100 : P.T)) != DIPL_OK) return st;
+    if ((st = W.commit()) != DIPL_OK || (st = upload_tables()) != DIPL_OK) return st;
+    if (P.split && (st = count_references(P, stream)) != DIPL_OK) return st;
+    if (count_first) {
+        if ((st = reserve_scratch(P.N)) != DIPL_OK || (st = W.commit()) != DIPL_OK) return st;
     }
-    if ((st = W.commit()) != DIPL_OK) return st;
-    P.d_meshes = reinterpret_cast<MeshDesc*>(d_table);
-    P.d_offsets = reinterpret_cast<long long*>(d_table + mesh_bytes);
-    if (!P.split) P.d_coffsets = P.d_offsets;
-    DIPL_CUDA(cudaMemcpyAsync(d_table, table.data(), table_bytes, cudaMemcpyHostToDevice, stream));
-    if (P.split) {
-        if ((st = count_references(P, stream)) != DIPL_OK) return st;
-        O.reserve(&P.ref_tri, P.N);
-    }
-    O.reserve(&P.d_err, 4);
-    O.reserve(&P.perm, P.N);
-    O.reserve(&P.child, P.Kalloc);
-    O.reserve(&P.nlo, P.Kalloc);
-    O.reserve(&P.nhi, P.Kalloc);
-    if (wide) {
-        O.reserve(&P.wide.nodes, P.Kalloc);
-        O.reserve(&P.wide.tris, 3 * P.N);
-    } else {
-        O.reserve(&P.nodes, P.Kalloc);
-        O.reserve(&P.tris, 3 * P.N);
-        if (sobb) O.reserve(&P.snodes, P.Kalloc);
-        else O.reserve(&P.quads, P.Kalloc);
-    }
-    if ((st = O.commit()) != DIPL_OK) return st;
+    // what the sort leaves behind, for what comes after it
+    P.contrib = static_cast<uint32_t*>(P.keys_alt);
+    P.owner_leaf = reinterpret_cast<int*>(P.perm_alt);
+    auto commit_kept = [&](bool quads) -> dipl_status {
+        if (P.split) O.reserve(&P.ref_tri, P.N);
+        O.reserve(&P.d_err, 4);
+        O.reserve(&P.perm, P.N);
+        O.reserve(&P.child, P.Kalloc);
+        O.reserve(&P.nlo, P.Kalloc);
+        O.reserve(&P.nhi, P.Kalloc);
+        if (wide) {
+            O.reserve(&P.wide.nodes, P.Kalloc);
+            O.reserve(&P.wide.tris, 3 * P.N);
+        } else {
+            O.reserve(&P.nodes, P.Kalloc);
+            O.reserve(&P.tris, 3 * P.N);
+            if (sobb) O.reserve(&P.snodes, P.Kalloc);
+            if (quads) O.reserve(&P.quads, P.Kalloc);
+        }
+        return O.commit();
+    };
+    const bool quads = !wide && !sobb;
+    st = commit_kept(quads);
+    // no memory for the 4-wide nodes: the handles go without, and traces walk the binary nodes
+    if (st == DIPL_ERR_OUT_OF_MEMORY && quads && tight) st = commit_kept(false);
+    if (st != DIPL_OK) return st;
     if (P.split) DIPL_CUDA(cudaMemsetAsync(P.d_err, 0, 4, stream));
-    if (hier) P.hp_other = P.parent + N + Kalloc;
+    if (hier) P.hp_other = P.parent + arrivals;
     unsigned char* z = P.zero;
     auto carve = [&](size_t bytes) {
         unsigned char* at = z;
@@ -2736,6 +2757,19 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
         }
     }
     return DIPL_OK;
+}
+
+// Prepares with room to spare and, where that is refused, tight: blocks of the exact sizes, scratch by the count of
+// references, and if need be without the 4-wide nodes. A build then fits wherever one with a block per array did.
+static dipl_status plan_make(std::unique_ptr<BuildPlan>& P, const dipl_build_desc* descs, int count, cudaStream_t stream,
+                             bool own_summary) {
+    dipl_status st = DIPL_OK;
+    for (const bool tight : {false, true}) {
+        P = std::make_unique<BuildPlan>();
+        st = plan_prepare(*P, descs, count, stream, own_summary, tight);
+        if (st != DIPL_ERR_OUT_OF_MEMORY) break;
+    }
+    return st;
 }
 
 template <int B>
@@ -2999,9 +3033,10 @@ static dipl_status plan_finish(BuildPlan& P, dipl_bvh** out, bool allow_wide) {
 dipl_status build_batched(const dipl_build_desc* descs, int count, dipl_bvh** out, cudaStream_t stream) {
     DIPL_CHECK_ARG(descs && out && count >= 1, "descs/out must be non-NULL and count >= 1");
     for (int i = 0; i < count; ++i) out[i] = nullptr;
-    BuildPlan P;
-    dipl_status st = plan_prepare(P, descs, count, stream, false);
+    std::unique_ptr<BuildPlan> plan;
+    dipl_status st = plan_make(plan, descs, count, stream, false);
     if (st != DIPL_OK) return st;
+    BuildPlan& P = *plan;
     if ((st = plan_enqueue(P, stream)) != DIPL_OK) return st;
     if (P.m > 0) DIPL_CUDA(cudaStreamSynchronize(stream));  // the build's one host synchronisation
     return plan_finish(P, out, true);
@@ -3011,7 +3046,7 @@ dipl_status build_batched(const dipl_build_desc* descs, int count, dipl_bvh** ou
 
 // ---- build plans: a batch captured once into a CUDA graph and replayed ---------------------------------
 struct dipl_build_plan {
-    dipl::BuildPlan plan;
+    std::unique_ptr<dipl::BuildPlan> plan;
 };
 
 namespace dipl {
@@ -3020,15 +3055,15 @@ dipl_status plan_create(const dipl_build_desc* descs, int count, dipl_build_plan
     DIPL_CHECK_ARG(out != nullptr, "out must be non-NULL");
     *out = nullptr;
     auto holder = std::make_unique<dipl_build_plan>();
-    BuildPlan& P = holder->plan;
     for (int i = 0; i < count && descs; ++i)
         if (descs[i].split_budget != 0) {
             // the pieces depend on the vertex positions, which a plan's replays may change
             set_last_error("pre-splitting (split_budget > 0) cannot be captured in a build plan");
             return DIPL_ERR_UNSUPPORTED;
         }
-    dipl_status st = plan_prepare(P, descs, count, stream, true);
+    dipl_status st = plan_make(holder->plan, descs, count, stream, true);
     if (st != DIPL_OK) return st;
+    BuildPlan& P = *holder->plan;
     if (P.d0.layout == DIPL_LAYOUT_WIDE8_Q8) {
         set_last_error("the 8-wide layout cannot be captured in a build plan (it reads level sizes back)");
         return DIPL_ERR_UNSUPPORTED;
@@ -3071,16 +3106,16 @@ dipl_status plan_create(const dipl_build_desc* descs, int count, dipl_build_plan
 
 dipl_status plan_launch(dipl_build_plan* plan, cudaStream_t stream) {
     DIPL_CHECK_ARG(plan != nullptr, "plan must be non-NULL");
-    if (plan->plan.m == 0) return DIPL_OK;
-    DIPL_CUDA(cudaGraphLaunch(plan->plan.graph_exec, stream));
-    note_launches(plan->plan.graph_kernels);
+    if (plan->plan->m == 0) return DIPL_OK;
+    DIPL_CUDA(cudaGraphLaunch(plan->plan->graph_exec, stream));
+    note_launches(plan->plan->graph_kernels);
     return DIPL_OK;
 }
 
 dipl_status plan_get_bvhs(dipl_build_plan* plan, dipl_bvh** out, cudaStream_t stream) {
     DIPL_CHECK_ARG(plan && out, "plan/out must be non-NULL");
     DIPL_CUDA(cudaStreamSynchronize(stream));
-    return plan_finish(plan->plan, out, false);
+    return plan_finish(*plan->plan, out, false);
 }
 
 void plan_destroy(dipl_build_plan* plan) { delete plan; }

@@ -98,13 +98,14 @@ class ScratchArena {
 // ---- the BVH handle ------------------------------------------------------------------------------
 // Device memory of one build; shared by the handles of a batched build. Arrays are asked for with reserve() and made by
 // commit() in one allocation, so a build takes two blocks (what the handles keep, scratch) instead of about forty: 40 us
-// of a small build's 380. Block sizes are rounded up to a sixteenth of their power of two, so that builds of nearly the
-// same size reuse each other's blocks. With blocks of many sizes in one pool, three 16M-triangle handles rebuilt in turn
-// took 30 to 62 ms a build and trace, half of it mapping memory; two blocks from two pools: 20 ms.
+// of a small build's 380. Block sizes are rounded up to a sixteenth of their power of two (unless `exact`), so
+// that builds of nearly the same size reuse each other's blocks. With blocks of many sizes in one pool, three 16M-triangle
+// handles rebuilt in turn took 30 to 62 ms a build and trace, half of it mapping memory; two blocks from two pools: 20 ms.
 struct Storage {
     std::vector<void*> ptrs;
     cudaStream_t stream = nullptr;
     bool kept = false;  // what a handle keeps: from the pool of those
+    bool exact = false;
     ~Storage() {
         for (void* p : ptrs) device_free(p, stream);
     }
@@ -118,7 +119,7 @@ struct Storage {
         size_t unit = 256;
         while (unit * 32 <= total_) unit *= 2;  // total_ / 32 < unit: at most 16 to 32 units
         void* p = nullptr;
-        dipl_status st = device_alloc(&p, (total_ + unit - 1) / unit * unit, stream, kept);
+        dipl_status st = device_alloc(&p, exact ? total_ : (total_ + unit - 1) / unit * unit, stream, kept);
         if (st == DIPL_OK) {
             ptrs.push_back(p);
             for (const auto& w : want_) {
@@ -151,7 +152,8 @@ struct dipl_bvh {
     // traced arrays (device)
     void* nodes = nullptr;      // BNode / SNode / WNode
     int64_t node_size = 64;     // bytes per node of the traced layout
-    dipl::QNode* quads = nullptr;  // binary AABB layout: the 4-wide node of every binary node, same indices
+    dipl::QNode* quads = nullptr;  // binary AABB layout: the 4-wide node of every binary node, same indices; nullptr
+                                   // where there was no memory for them
     float4* tris = nullptr;     // 3 float4 per triangle in leaf order (v0.w = primitive id bits)
     // clustering result (device), for downloads
     int32_t* perm = nullptr;    // triangle id per sorted position (of this mesh, local ids)

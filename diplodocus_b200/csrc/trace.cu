@@ -24,7 +24,8 @@ constexpr int kTraceMinBlocks = 9;
 constexpr float kSlabWiden = 1e-6f;
 
 // Conservative ray/box interval; returns entry t (or +inf when the box is missed or out of range).
-__device__ __forceinline__ float box_entry(const RayState& r, float lx, float hx, float ly, float hy, float lz, float hz,
+template <class R>
+__device__ __forceinline__ float box_entry(const R& r, float lx, float hx, float ly, float hy, float lz, float hz,
                                            float t_limit) {
     const float tx0 = __fmul_rn(__fsub_rn(lx, r.o.x), r.inv.x), tx1 = __fmul_rn(__fsub_rn(hx, r.o.x), r.inv.x);
     const float ty0 = __fmul_rn(__fsub_rn(ly, r.o.y), r.inv.y), ty1 = __fmul_rn(__fsub_rn(hy, r.o.y), r.inv.y);
@@ -599,6 +600,57 @@ __global__ void __launch_bounds__(kTraceThreads, 7) quad_pool_kernel(  // 8: fra
     trace_batch_pool<LEAF, ANY, PERSIST>(v, S, tris, (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u, B);
 }
 
+// ---- binary traversal ---------------------------------------------------------------------------------------------
+// Closest and any hits over the binary nodes, for handles whose build had no memory for the 4-wide ones. Bound like the
+// 4-wide loop, with twice the steps: 1M rays of a 2M-triangle soup 5.9 against 4.5 ms (counted: 8.4).
+constexpr int kBinaryShort = 24;
+
+template <int STACK>
+struct BinaryWork : RefWork<STACK, kBinaryShort> {
+    const BNode* nodes;
+    int num_nodes;
+
+    template <class R>
+    __device__ __forceinline__ void begin(const R&) { this->enter(this->root); }
+    template <class R>
+    __device__ __forceinline__ void take(const R&, int thread, int entry, int) {
+        this->enter(this->column[entry * kTraceThreads + thread - (int)threadIdx.x]);
+    }
+    template <class R>
+    __device__ __forceinline__ void node(const R& r, float lim, int bot) {
+        if (this->cur >= num_nodes || this->sp >= STACK) {  // only a corrupted tree gets here
+            this->bad = true;
+            this->drop();
+            return;
+        }
+        const float4* np = reinterpret_cast<const float4*>(nodes + this->cur);
+        float4 a, b, c, df;
+        ldg_v8(np, a, b);
+        ldg_v8(np + 2, c, df);
+        const int c0 = __float_as_int(df.x), c1 = __float_as_int(df.y);
+        const float t0 = box_entry(r, a.x, a.y, a.z, a.w, c.x, c.y, lim);
+        const float t1 = box_entry(r, b.x, b.y, b.z, b.w, c.z, c.w, lim);
+        const bool swap = t1 < t0;
+        if (fmaxf(t0, t1) != __int_as_float(0x7F800000)) this->push(swap ? c0 : c1);
+        this->cur = fminf(t0, t1) != __int_as_float(0x7F800000) ? (swap ? c1 : c0) : kRefPop;
+        this->advance(bot);
+    }
+};
+
+template <int LEAF, bool ANY, bool PERSIST, int STACK>
+__global__ void __launch_bounds__(kTraceThreads, 8) binary_batch_kernel(
+    const BNode* __restrict__ nodes, const float4* __restrict__ tris, int root, int num_nodes, uint32_t flags, Batch B) {
+    __shared__ int s_stack[kBinaryShort * kTraceThreads];
+    __shared__ SharedRays<ANY> S;
+    int rest[STACK - kBinaryShort];
+    BinaryWork<STACK> v;
+    v.tris = tris, v.column = s_stack + threadIdx.x, v.rest = rest, v.root = root;
+    v.backface = (flags & DIPL_TRACE_BACKFACE_CULLING) != 0u;
+    v.nodes = nodes, v.num_nodes = num_nodes;
+    LaneRay<LEAF, ANY> r{};
+    trace_batch<LEAF, ANY, PERSIST>(v, r, S, B);
+}
+
 // ---- ray order ----------------------------------------------------------------------------------------
 // On request, batches of at least kReorderMinRays rays are traced in the order of a 30-bit key: the direction's octant
 // above a 9-bit-per-axis Morton code of the origin within the batch's origin bounds. A warp's 32 rays then
@@ -731,9 +783,10 @@ dipl_status launch_trace(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dip
 // deep traversals wait for memory). The watertight test gains at all sizes: 2M-triangle soup, 2M rays 4.22 -> 4.0 ms.
 constexpr int64_t kPoolRays = 1 << 19;
 
-template <int LEAF, bool ANY, int STACK>
-dipl_status launch_quad(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ,
-                        uint32_t flags, cudaStream_t s) {
+// QUADS: the 4-wide nodes, else the binary ones.
+template <int LEAF, bool ANY, bool QUADS, int STACK>
+dipl_status launch_uncounted(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ,
+                             uint32_t flags, cudaStream_t s) {
     const int num_nodes = b->num_triangles == 0 ? -1 : (int)b->node_capacity;
     RayOrder ro;
     if (reorder_rays(n, flags)) {
@@ -746,9 +799,15 @@ dipl_status launch_quad(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl
     Batch B{rays, n, hits, occ, ro.order, b->d_err, steps_bound(num_nodes, b->num_refs), 32, num_nodes < 0};
     auto launch = [&](auto kernel, unsigned grid, int group) {
         B.group = group;
-        kernel<<<grid, kTraceThreads, 0, s>>>(b->quads, b->tris, b->root, num_nodes, flags, B);
+        if constexpr (QUADS)
+            kernel<<<grid, kTraceThreads, 0, s>>>(b->quads, b->tris, b->root, num_nodes, flags, B);
+        else
+            kernel<<<grid, kTraceThreads, 0, s>>>(static_cast<const BNode*>(b->nodes), b->tris, b->root, num_nodes, flags, B);
     };
-    if (!ANY && LEAF == DIPL_LEAF_REF_MT && n > kPoolRays)
+    if constexpr (!QUADS)
+        launch_batch<binary_batch_kernel<LEAF, ANY, false, STACK>, binary_batch_kernel<LEAF, ANY, true, STACK>>(
+            n, ro.order != nullptr, launch);
+    else if (!ANY && LEAF == DIPL_LEAF_REF_MT && n > kPoolRays)
         launch_batch<quad_trace_kernel<false, STACK>, quad_trace_kernel<true, STACK>>(n, ro.order != nullptr, launch);
     else
         launch_batch<quad_pool_kernel<LEAF, ANY, false, STACK>, quad_pool_kernel<LEAF, ANY, true, STACK>>(
@@ -761,13 +820,18 @@ dipl_status launch_quad(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl
 }
 
 template <int LEAF, bool ANY>
-dipl_status launch_quad_stack(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ,
-                              uint32_t flags, cudaStream_t s) {
+dipl_status launch_uncounted_stack(const dipl_bvh* b, const dipl_ray* rays, int64_t n, dipl_hit* hits, uint8_t* occ,
+                                   uint32_t flags, cudaStream_t s) {
+    if (!b->quads && b->num_triangles > 0) {  // at most one entry is pushed per binary level
+        if (b->depth < 64) return launch_uncounted<LEAF, ANY, false, 64>(b, rays, n, hits, occ, flags, s);
+        if (b->depth < 128) return launch_uncounted<LEAF, ANY, false, 128>(b, rays, n, hits, occ, flags, s);
+        return launch_uncounted<LEAF, ANY, false, 512>(b, rays, n, hits, occ, flags, s);
+    }
     // at most 3 entries are pushed per two binary levels
     const int need = 3 * ((b->depth + 1) / 2) + 3;
-    if (need <= 64) return launch_quad<LEAF, ANY, 64>(b, rays, n, hits, occ, flags, s);
-    if (need <= 160) return launch_quad<LEAF, ANY, 160>(b, rays, n, hits, occ, flags, s);
-    return launch_quad<LEAF, ANY, 776>(b, rays, n, hits, occ, flags, s);
+    if (need <= 64) return launch_uncounted<LEAF, ANY, true, 64>(b, rays, n, hits, occ, flags, s);
+    if (need <= 160) return launch_uncounted<LEAF, ANY, true, 160>(b, rays, n, hits, occ, flags, s);
+    return launch_uncounted<LEAF, ANY, true, 776>(b, rays, n, hits, occ, flags, s);
 }
 
 template <int LEAF>
@@ -824,8 +888,8 @@ dipl_status trace_closest(const dipl_bvh* b, const dipl_ray* rays, int64_t n, di
         return leaf_test == DIPL_LEAF_REF_MT
                    ? launch_trace_stack<DIPL_LEAF_REF_MT>(b, rays, n, hits, flags, counters, s)
                    : launch_trace_stack<DIPL_LEAF_WATERTIGHT>(b, rays, n, hits, flags, counters, s);
-    return leaf_test == DIPL_LEAF_REF_MT ? launch_quad_stack<DIPL_LEAF_REF_MT, false>(b, rays, n, hits, nullptr, flags, s)
-                                         : launch_quad_stack<DIPL_LEAF_WATERTIGHT, false>(b, rays, n, hits, nullptr, flags, s);
+    return leaf_test == DIPL_LEAF_REF_MT ? launch_uncounted_stack<DIPL_LEAF_REF_MT, false>(b, rays, n, hits, nullptr, flags, s)
+                                         : launch_uncounted_stack<DIPL_LEAF_WATERTIGHT, false>(b, rays, n, hits, nullptr, flags, s);
 }
 
 dipl_status trace_any(const dipl_bvh* b, const dipl_ray* rays, int64_t n, uint8_t* occ, int leaf_test, uint32_t flags,
@@ -837,8 +901,8 @@ dipl_status trace_any(const dipl_bvh* b, const dipl_ray* rays, int64_t n, uint8_
     if (n == 0) return DIPL_OK;
     if (b->layout != DIPL_LAYOUT_BINARY || b->bv_type != DIPL_BV_AABB) return trace_any_ext(b, rays, n, occ, leaf_test, flags, s);
     if (leaf_test == DIPL_LEAF_REF_MT)
-        return launch_quad_stack<DIPL_LEAF_REF_MT, true>(b, rays, n, nullptr, occ, flags, s);
-    return launch_quad_stack<DIPL_LEAF_WATERTIGHT, true>(b, rays, n, nullptr, occ, flags, s);
+        return launch_uncounted_stack<DIPL_LEAF_REF_MT, true>(b, rays, n, nullptr, occ, flags, s);
+    return launch_uncounted_stack<DIPL_LEAF_WATERTIGHT, true>(b, rays, n, nullptr, occ, flags, s);
 }
 
 }  // namespace dipl
