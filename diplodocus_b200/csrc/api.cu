@@ -89,9 +89,11 @@ dipl_status device_alloc(void** ptr, size_t bytes, cudaStream_t stream, bool kep
     });
     cudaMemPool_t own = kept ? kept_pool() : nullptr;
     cudaError_t e = own ? cudaMallocFromPoolAsync(ptr, bytes, own, stream) : cudaMallocAsync(ptr, bytes, stream);
-    if (e == cudaErrorMemoryAllocation) {
-        // the other pool may hold free blocks: give them back and try once more
-        (void)cudaGetLastError();
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError(), (void)cudaStreamIsCapturing(stream, &capture);
+    if (e == cudaErrorMemoryAllocation && capture == cudaStreamCaptureStatusNone) {
+        // the other pool may hold free blocks: give them back and try once more (not while the stream is captured: waiting
+        // for it would end the capture)
         int dev = 0;
         cudaMemPool_t pool;
         cudaStreamSynchronize(stream);
