@@ -303,7 +303,6 @@ struct RefStack {
     int sp = 0;
 
     __device__ __forceinline__ bool has_node() const { return cur != kRefIdle; }
-    __device__ __forceinline__ void drop() { cur = kRefIdle; }
     __device__ __forceinline__ void clear() { cur = kRefIdle, sp = 0; }
     __device__ __forceinline__ void put(int at, int ref) {
         if (at < SHORT) column[at * kTraceThreads] = ref;

@@ -689,7 +689,11 @@ struct WideWork {
         if (root < 0) held_base = leaf_first(root), held = (1u << leaf_count(root)) - 1u;
         else current = root;
     }
-    __device__ __forceinline__ int2 get(int k) const { return k < kShort ? column[k * kTraceThreads] : rest[k - kShort]; }
+    __device__ __forceinline__ int2 get(int k) const {
+        int2 e = column[min(k, kShort - 1) * kTraceThreads];
+        if (k >= kShort) e = rest[k - kShort];
+        return e;
+    }
     __device__ __forceinline__ void set(int k, int2 e) {
         if (k < kShort) column[k * kTraceThreads] = e;
         else rest[k - kShort] = e;
