@@ -2121,10 +2121,10 @@ __device__ __forceinline__ QChild leaf_part(const float4* __restrict__ tris, con
 }
 
 // Frame and bytes of one axis. The bytes are chosen in FP64, where the distance of a plane from p in steps is off by
-// less than 2^-36 of a step (the boxes are padded by far more): every child's interval lies within its planes. 2^111 is
-// the largest step whose 33,023-fold is finite; where 255 of those don't reach (an extent above 6.6e35, a coordinate
-// below -2.5e38, a plane that padding made infinite) p = -inf, whose planes come out infinite on the open side or NaN
-// and so constrain no ray on this axis.
+// less than 2^-36 of a step (the boxes are padded by far more): every child's interval lies within its planes. Steps end
+// at 2^111, so that p, 32768 steps below the boxes, is finite for all but the lowest coordinates. Where 255 of those don't
+// reach (an extent above 6.6e35, a coordinate below -2.5e38, a plane that padding made infinite) p = -inf, whose planes
+// come out infinite on the open side or NaN and so constrain no ray on this axis.
 __device__ __forceinline__ void quad_axis(const float* lo, const float* hi, uint32_t valid, float& p, uint32_t& ebias,
                                           uint32_t& qlo, uint32_t& qhi) {
     float mn = __int_as_float(0x7F800000), mx = __int_as_float(0xFF800000);
@@ -2158,7 +2158,7 @@ __device__ __forceinline__ void quad_axis(const float* lo, const float* hi, uint
             break;
         }
     }
-    ebias = eb;
+    ebias = eb + 14u;  // the traversal's scale: 16384 steps
 }
 
 __global__ void __launch_bounds__(128) quad_write_kernel(const BNode* __restrict__ nodes,
@@ -2222,7 +2222,7 @@ __global__ void __launch_bounds__(128) quad_write_kernel(const BNode* __restrict
     q.pad[0] = q.pad[1] = 0u;
     if (valid == 0u) {
         q.px = q.py = q.pz = 0.0f;
-        q.exps = 0x010101u;
+        q.exps = 0x0F0F0Fu;
         q.qlox = q.qloy = q.qloz = 0xFFFFFFFFu, q.qhix = q.qhiy = q.qhiz = 0u;
     } else {
         uint32_t ex, ey, ez;

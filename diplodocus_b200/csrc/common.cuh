@@ -47,10 +47,11 @@ struct __align__(16) BNode {
 static_assert(sizeof(BNode) == 64, "BNode must be 64 bytes");
 
 // 4-wide traversal node (64 bytes, two 32-byte loads): a binary inner node's grandchildren, their boxes in 8-bit
-// steps of a frame of their own. Plane q of axis a lies at p[a] + (32768 + q) * 2^(e[a] - 127): the offset makes
-// "32768 + q" a float whose bits are the byte q shifted by 8 under a constant exponent, so the traversal decodes a
-// byte with one byte permute and no integer-to-float conversion. An unused slot has planes in the wrong order
-// (255 .. 0) and a leaf reference of no triangles.
+// steps of a frame of their own. Plane q of axis a lies at p[a] + (2 + q / 16384) * 2^(e[a] - 127): the offset makes
+// "2 + q / 16384" a float whose bits are the byte q shifted by 8 under a constant exponent, so the traversal decodes a
+// byte with one byte permute and no integer-to-float conversion. (2 is the least offset of this form, so that the scale
+// as a distance along a ray is the last to turn subnormal, and the largest scale that no plane at a finite distance
+// overflows.) An unused slot has planes in the wrong order (255 .. 0) and a leaf reference of no triangles.
 struct __align__(64) QNode {
     float px, py, pz;
     uint32_t exps;          // biased exponents: x | y << 8 | z << 16

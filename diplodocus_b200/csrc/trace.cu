@@ -443,17 +443,19 @@ constexpr float kMiss = 3.40282346638528859812e+38f;  // entry distance of a chi
 constexpr int kQuadShort = 32;
 constexpr int kQuadPoolShort = 24;
 
-// Byte k of a plane word as the float 32768 + byte.
+// Byte k of a plane word as the float 2 + byte / 16384.
 __device__ __forceinline__ float quad_plane(uint32_t w, int k) {
-    return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7504u | (uint32_t)(k << 4)));
+    return __uint_as_float(__byte_perm(w, 0x40000000u, 0x7504u | (uint32_t)(k << 4)));
 }
 
 // The entry distances of a node's children (kMiss when not entered) and their references.
 //
-// A plane at p + Q s (Q = 32768 + byte) is met at t = (p - o) / d + Q (s / d). With a = p - o in FP32 and C = a / d
+// A plane at p + Q s (Q = 2 + byte / 16384) is met at t = (p - o) / d + Q (s / d). With a = p - o in FP32 and C = a / d
 // the rounding of a and C is at most 2^-23 |C|; near planes move back and far planes on by 2^-22 |C|. What is
 // relative to t (the reciprocal of d, the last FMA) stays below 2e-7 on either side and the final comparison allows
-// 2e-6. A NaN plane (an overflowing product) does not constrain the interval.
+// 2e-6 (as much as the binary nodes, whose two distances move by 1e-6 each). A subnormal s / d is off by 2^-150, which Q
+// makes one unit of t. A NaN plane (an overflowing product) does not constrain the interval: s / d overflows only where
+// a / d does too or the box begins beyond FLT_MAX.
 template <class R>
 __device__ __forceinline__ void quad_children(const QNode* __restrict__ quads, int node, const R& r, float lim,
                                               float (&key)[4], int (&ref)[4]) {

@@ -86,3 +86,20 @@ def test_long_directions(orc, name):
     truth = orc.brute(tris, rays, leaf_test=1)
     assert int((truth.prim >= 0).sum()) > 500
     np.testing.assert_array_equal(h.prim.cpu().numpy(), truth.prim)
+
+
+@pytest.mark.parametrize("length", [1e30, 1e33, 1e36])
+@pytest.mark.parametrize("name", list(LAYOUTS))
+def test_short_parameters(orc, name, length):
+    """Directions so long that a node's steps are subnormal as distances along the ray, towards the corners of small
+    triangles (ref_mt: products of the other test underflow)."""
+    tris, _ = scattered(3000, 1e-3, 1e-5, 0.0, seed=13)
+    g = np.random.default_rng(14)
+    d = g.standard_normal((len(tris), 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    corner = 0.98 * tris[:, 0].astype(np.float64) + 0.02 * tris.astype(np.float64).mean(axis=1)
+    rays = S.pack_rays((corner - 0.05 * d).astype(np.float32), (d * length).astype(np.float32), tmin=0.0)
+    h = check(build(tris, **LAYOUTS[name]), rays, "ref_mt", many=True)
+    truth = orc.brute(tris, rays, leaf_test=0)
+    assert int((truth.prim >= 0).sum()) > 1000
+    np.testing.assert_array_equal(h.prim.cpu().numpy(), truth.prim)
