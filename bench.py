@@ -11,8 +11,9 @@ A step = one build over the resident triangles + one closest-hit trace of the re
   trace          closest-hit throughput, Mrays/s (CUDA events around the trace launch)
   e2e            the same step through the public API with HOST inputs: pinned vertex arrays and rays copied in,
                  build, trace, hits copied out; Mtri/s over the whole step
-  roofline       the step's dominant kernel against HBM (algorithmic bytes over its measured time);
-                 roofline_build / roofline_trace give both
+  roofline       the step's dominant kernel; roofline_build / roofline_trace give both. Build: algorithmic bytes over
+                 its time, against HBM. Trace of the binary layout: DRAM bytes that ncu measured for this configuration
+                 (null for others) over its time, against HBM; it is bound by issue slots, not by HBM
   variants       (soup) Morton30, EMC60 + SOBB and the 8-wide quantised layout on the same triangles and rays
   errors         (soup) FP32 t/u/v of the reference-exact and the watertight leaf test against an FP64
                  re-intersection of the same triangle, and FP64 re-intersection of the rays whose hits differ
@@ -299,10 +300,10 @@ def cpu_baseline_and_parity(tris, rays_np, gpu_hits_np, args, threads):
 # DRAM bytes (read + write) per unit measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum, one pass) on
 # the current kernels, per ray of one closest-hit trace and per triangle of one build, for the configuration each
 # was captured with (split budget, ray order, size); other configurations report no traffic. Soup trace: the full
-# 16M-triangle, 16M-ray launch, 10.46 GB read + 0.54 GB written (profiles/trace_dram_soup16m.md).
+# 16M-triangle, 16M-ray launch, 10.46 GB read + 0.54 GB written.
 MEASURED_TRAFFIC = {("soup16m", "emc60", "trace"): {"split_budget": 40, "order": "coherent", "triangles": 16777216,
                                                     "per_unit": (10.46e9 + 0.538e9) / 16777216},
-                    # the first build of the run, all 27 launches (profiles/dram_traffic_build_soup16m.md)
+                    # the first build of the run, all 27 launches
                     ("soup16m", "emc60", "build"): {"split_budget": 40, "order": "coherent", "triangles": 16777216,
                                                     "per_unit": (22974e6 + 6345e6) / 16777216},
                     ("displaced_sphere", "morton30", "build"): {"split_budget": 0, "order": "given",
@@ -344,11 +345,21 @@ def build_bytes_per_tri(code_type, digit_bits=8, node_bytes_per_tri=None, leaves
 
 
 def trace_bytes_per_ray(visits, tests, node_bytes):
-    """Algorithmic bytes of one closest-hit ray: the ray in, the hit out, every node visited, every triangle
-    tested. The counts are those of the counted traversal of the layout's own nodes on the same rays; the timed kernel
-    of the binary layout reads 4-wide nodes of the same size, about half as many, so that its fraction of a peak can
-    pass 1 without more bytes moved (`traffic` has the measured ones)."""
+    """Algorithmic bytes of one closest-hit ray of the counted traversal: the ray in, the hit out, every node visited,
+    every triangle tested. The timed kernels of the 8-wide and the oriented-box layout walk the same nodes; that of the
+    binary layout walks 4-wide nodes, about half as many, so that these bytes are not its own."""
     return 32 + 16 + visits * node_bytes + tests * 36
+
+
+def trace_roofline(ms, rays, bytes_per_ray, traffic, own_bytes, peak):
+    """A trace against HBM: by the bytes that its own nodes and triangles are (`own_bytes`), else by the DRAM bytes
+    measured for the configuration; without either there is no fraction."""
+    moved = bytes_per_ray * rays if own_bytes else traffic
+    achieved = moved / (ms * 1e-3) / 1e9 if moved is not None else None
+    return {"bound": "hbm" if own_bytes else "issue slots",
+            "achieved": None if achieved is None else round(achieved, 1), "peak": peak, "unit": "GB/s",
+            "frac": None if achieved is None else round(achieved / peak, 4), "traffic": traffic,
+            "counted_bytes_per_ray": round(bytes_per_ray, 1)}
 
 
 def _quantiles(x, qs):
@@ -492,20 +503,17 @@ def run_gpu(args, rank, world, local_rank):
     bpt = build_bytes_per_tri(desc.code_type, 8, info.node_bytes / max(n, 1), info.num_leaves / max(n, 1))
     achieved_build = bpt * n / build_s / 1e9
     ray_bytes = trace_bytes_per_ray(visits / nr, tests / nr, node_bytes)
-    achieved_trace = ray_bytes * nr / trace_s / 1e9
     value = world * n / build_s / 1e6
     roof_build = {"bound": "hbm", "achieved": round(achieved_build, 1), "peak": peak, "unit": "GB/s",
                   "frac": round(achieved_build / peak, 4), "traffic": measured_traffic(args.workload, code, "build", n, split, order_name, n),
                   "kernel": "build pipeline (bounds, codes, sort, PLOC, layout)", "ms": round(build_s * 1e3, 4),
                   "bytes_per_unit": round(bpt, 1), "unit_of_bytes": "triangle",
                   "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)"}
-    roof_trace = {"bound": "hbm", "achieved": round(achieved_trace, 1), "peak": peak, "unit": "GB/s",
-                  "frac": round(achieved_trace / peak, 4),
-                  "traffic": (measured_traffic(args.workload, code, "trace", nr, split, order_name, n)
-                              if args.leaf_test == "ref_mt" else None),
-                  "kernel": "closest-hit trace (quad_trace_kernel; bytes of the counted binary traversal)", "ms": round(trace_s * 1e3, 4),
-                  "bytes_per_unit": round(ray_bytes, 1), "unit_of_bytes": "ray", "node_bytes": round(node_bytes, 1),
-                  "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)"}
+    traffic = (measured_traffic(args.workload, code, "trace", nr, split, order_name, n)
+               if args.leaf_test == "ref_mt" else None)
+    roof_trace = trace_roofline(trace_s * 1e3, nr, ray_bytes, traffic, False, peak)
+    roof_trace.update(kernel="closest-hit trace (4-wide nodes)", ms=round(trace_s * 1e3, 4),
+                      peak_source=peak_kind + " (MEASURED_PEAKS.json hbm_gbs)")
     line = {
         "metric": METRIC, "value": round(value, 3), "unit": "Mtri/s", "n_gpus": world, "steps": steps,
         "warmup": args.warmup, "ms_per_step": round(t_step / steps, 4), "higher_is_better": True,
@@ -710,7 +718,6 @@ def soup_forms(args, lib, L, A, torch, C, v, rays, hits, h_main, cfg, config, bu
         nb = info.node_bytes / max(info.num_inner_nodes, 1)
         rb = trace_bytes_per_ray(visits, tests, nb)
         tm = float(np.median(t_ms))
-        ach = rb * nr / (tm / 1e3) / 1e9
         same = float((vh[:, 0] == main_prim).float().mean().item())
         bm = float(np.median(b_ms))
         out["variants"][name] = {
@@ -720,8 +727,7 @@ def soup_forms(args, lib, L, A, torch, C, v, rays, hits, h_main, cfg, config, bu
             "trace_mrays_s": round(nr / tm / 1e3, 2), "sah_cost": round(sah.value, 4),
             "node_visits_per_ray": round(visits, 2), "tri_tests_per_ray": round(tests, 2),
             "node_bytes": int(info.node_bytes),
-            "roofline_trace": {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s",
-                               "frac": round(ach / peak, 4), "bytes_per_ray": round(rb, 1), "node_bytes": round(nb, 1)},
+            "roofline_trace": trace_roofline(tm, nr, rb, None, layout != "binary" or bv == "sobb", peak),
             "same_hits_as_main": same}
         if same < 1.0:
             out["disagreements"][f"main_vs_{name}"] = disagreement(hits, vh)

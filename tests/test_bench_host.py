@@ -97,3 +97,15 @@ def test_measured_traffic_is_reported_only_for_the_captured_configuration():
     assert bench.measured_traffic("soup16m", "emc60", "trace", n, 40, "given", n) is None
     assert bench.measured_traffic("soup16m", "emc60", "trace", n, 40, "coherent", n // 4) is None
     assert bench.measured_traffic("soup16m", "morton30", "trace", n, 40, "coherent", n) is None
+
+
+def test_trace_roofline_states_bytes_that_the_timed_kernel_moves():
+    """Counted bytes count for the layouts whose nodes the timed kernel walks, measured DRAM bytes for the binary one."""
+    sys.path.insert(0, ROOT)
+    import bench
+    own = bench.trace_roofline(1.0, 1000, 3.0e6, None, True, 6000.0)
+    assert (own["bound"], own["achieved"], own["frac"]) == ("hbm", 3000.0, 0.5)
+    binary = bench.trace_roofline(1.0, 1000, 9.0e6, 6.0e8, False, 6000.0)
+    assert (binary["bound"], binary["achieved"], binary["frac"], binary["traffic"]) == ("issue slots", 600.0, 0.1, 6.0e8)
+    unmeasured = bench.trace_roofline(1.0, 1000, 9.0e6, None, False, 6000.0)
+    assert unmeasured["achieved"] is None and unmeasured["frac"] is None and unmeasured["counted_bytes_per_ray"] == 9.0e6
