@@ -226,7 +226,11 @@ def run_reference(args, rank, world):
         sample_txt = f"SBvh::Build of all {n_sample:,} triangles on 1 thread per step"
     sample_rays = min(len(rays), args.ref_sample_rays)
     O = _ref_oracle()
-    ref = O.RefOracle()
+    try:
+        ref = O.RefOracle()
+    except FileNotFoundError as e:  # built only where the reference's sources are
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     for _ in range(args.warmup):
         ref.sbvh(tris[: min(len(tris), 65536)]).close()  # warm-up: code and allocator, not the measurement
     builds = []

@@ -109,3 +109,17 @@ def test_trace_roofline_states_bytes_that_the_timed_kernel_moves():
     assert (binary["bound"], binary["achieved"], binary["frac"], binary["traffic"]) == ("issue slots", 600.0, 0.1, 6.0e8)
     unmeasured = bench.trace_roofline(1.0, 1000, 9.0e6, None, False, 6000.0)
     assert unmeasured["achieved"] is None and unmeasured["frac"] is None and unmeasured["counted_bytes_per_ray"] == 9.0e6
+
+
+def test_reference_arm_without_its_library_prints_unavailable():
+    import json
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle as O
+    if os.path.exists(O.REF_LIB):
+        pytest.skip("the reference harness is built here")
+    r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1",
+                        "--warmup", "0", "--workload", "displaced_sphere", "--rays", "1024"],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    line = json.loads(r.stdout)
+    assert line["impl"] == "reference" and "not built" in line["unavailable"]
