@@ -2536,13 +2536,8 @@ static dipl_status count_references(BuildPlan& P, cudaStream_t stream) {
         set_last_error("build: a bounded device wait timed out while counting the pieces of large triangles");
         return DIPL_ERR_TIMEOUT;
     }
-    const long long bound = T + T * P.d0.split_budget / 100;
     P.N = P.coffsets[m];
     DIPL_CHECK_ARG(P.N < (1ll << 27), "references of a build (triangles and their pieces) must be < 2^27");
-    if (P.N > bound) {
-        set_last_error("build: more references than the budget allows (internal)");
-        return DIPL_ERR_INTERNAL;
-    }
     P.K = P.N - m;
     P.Kalloc = std::max<long long>(P.K, 1);
     return DIPL_OK;
@@ -2690,12 +2685,16 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
     // Scratch is sized by a bound on the references, at most split_budget percent more than the triangles, so that it is
     // one block taken before they are counted (tight: after); what the handles keep is taken after, by the count.
     const bool count_first = tight && P.split;
+    const long long bound = P.split ? P.T + P.T * d0.split_budget / 100 : P.T;
     reserve_tables();
-    if (!count_first && (st = reserve_scratch(P.split ? P.T + P.T * d0.split_budget / 100 : P.T)) != DIPL_OK) return st;
+    if (!count_first && (st = reserve_scratch(bound)) != DIPL_OK) return st;
     if ((st = W.commit()) != DIPL_OK || (st = upload_tables()) != DIPL_OK) return st;
     if (P.split && (st = count_references(P, stream)) != DIPL_OK) return st;
     if (count_first) {
         if ((st = reserve_scratch(P.N)) != DIPL_OK || (st = W.commit()) != DIPL_OK) return st;
+    } else if (P.N > bound) {  // weights of triangles near FP32's range saturate, and their sum passes 64 bits
+        set_last_error("build: more references than the bound");
+        return DIPL_ERR_OUT_OF_MEMORY;
     }
     // what the sort leaves behind, for what comes after it
     P.contrib = static_cast<uint32_t*>(P.keys_alt);
@@ -2759,8 +2758,9 @@ static dipl_status plan_prepare(BuildPlan& P, const dipl_build_desc* descs, int 
     return DIPL_OK;
 }
 
-// Prepares with room to spare and, where that is refused, tight: blocks of the exact sizes, scratch by the count of
-// references, and if need be without the 4-wide nodes. A build then fits wherever one with a block per array did.
+// Prepares with room to spare and, where that is refused or the references pass their bound, tight: blocks of the exact
+// sizes, scratch by the count of references, and if need be without the 4-wide nodes. A build then fits wherever one
+// with a block per array did.
 static dipl_status plan_make(std::unique_ptr<BuildPlan>& P, const dipl_build_desc* descs, int count, cudaStream_t stream,
                              bool own_summary) {
     dipl_status st = DIPL_OK;

@@ -103,3 +103,19 @@ def test_short_parameters(orc, name, length):
     truth = orc.brute(tris, rays, leaf_test=0)
     assert int((truth.prim >= 0).sum()) > 1000
     np.testing.assert_array_equal(h.prim.cpu().numpy(), truth.prim)
+
+
+@pytest.mark.parametrize("split", [10, 40])
+@pytest.mark.parametrize("name", list(LAYOUTS))
+def test_pre_splitting_of_huge_triangles(orc, name, split):
+    """Triangles whose area overflows saturate the weights of pre-splitting: more pieces than the budget, and a build."""
+    tris = S.uv_sphere(32, 16, 1.0, displacement=0.1, seed=3)
+    for k in range(20):
+        tris[19 * k, k % 3, :2] = 1e22, -1e22
+    assert orc.presplit(tris, split)[0].sum() > len(tris) * (100 + split) // 100
+    bvh = build(tris, split_budget=split, **LAYOUTS[name])
+    rays = S.sphere_inward_rays(3000, 9)
+    h = check(bvh, rays, "watertight", many=True)
+    truth = orc.brute(tris, rays, leaf_test=1)
+    assert int((truth.prim >= 0).sum()) > 100
+    np.testing.assert_array_equal(h.prim.cpu().numpy(), truth.prim)
