@@ -1,5 +1,6 @@
-// Closest-hit and any-hit traversal of the binary layout. Traces walk its 4-wide nodes (quad_trace_kernel); counted
-// traces walk the binary FP32 nodes themselves, whose visits the counters report (trace_kernel, tail_kernel).
+// Closest-hit and any-hit traversal of the binary layout. Traces walk its 4-wide nodes (quad_trace_kernel,
+// quad_pool_kernel), or its binary FP32 nodes where the handle has none (binary_batch_kernel); counted traces walk the
+// binary nodes, whose visits the counters report (trace_kernel, tail_kernel).
 //
 // Replaces SBvh::Intersect / IntersectAny (src/acceleration/sbvh.cc:60-191) and the device brute force
 // DummyIntersect / DummyIntersectAny (src/gpu/renderer/gpu_renderer_util.h:29-94).

@@ -190,7 +190,9 @@ DIPL_API dipl_status dipl_bvh_trace_closest(const dipl_bvh* bvh, const dipl_ray*
 
 /* As dipl_bvh_trace_closest, also adding the node visits and triangle tests of the batch to
  * d_counters[0] and d_counters[1] (device, 2 x uint64). The counts mirror AccelerationStats'
- * traversal_count / intersection_count (src/stats/acceleration_stats.h:14-16) in 64 bits. */
+ * traversal_count / intersection_count (src/stats/acceleration_stats.h:14-16) in 64 bits. They count a traversal of
+ * the layout's own nodes (dipl_bvh_download_layout), one node or triangle at a time; the other entry points find the
+ * same records by other visits (binary layout: of 4-wide nodes). */
 DIPL_API dipl_status dipl_bvh_trace_closest_counted(const dipl_bvh* bvh, const dipl_ray* d_rays, int64_t n, dipl_hit* d_hits,
                                            int32_t leaf_test, uint32_t flags, uint64_t* d_counters, void* stream);
 
