@@ -116,3 +116,26 @@ def test_binary_nodes_without_the_4_wide_ones(limits, count, least):
             assert torch.equal(short.Intersect(A.Stats(), r, leaf_test=leaf_test).raw, want.raw)
             assert torch.equal(short.IntersectAny(A.Stats(), r, leaf_test=leaf_test), want.prim >= 0)
     short.check_errors()
+
+
+def test_a_captured_plan_without_the_4_wide_nodes(limits):
+    """A plan made where memory is short replays, and its handles are traced through the binary nodes."""
+    need, kw = NEEDS["hploc_emc"]
+    tris = torch.from_numpy(S.soup(20_000, seed=9)).cuda()
+    moved = tris * 0.5 + 0.25
+    whole, _ = make(moved, **kw)
+    gc.collect()
+    torch.cuda.synchronize()
+    limits(device_memory_bytes=L.get_limits()[1] + need)
+    plan = A.BuildPlan(A.AccelerationStructureConfig(kw["kind"]), [tris])
+    limits()
+    for mine, new in zip(plan.verts[0], A.soa_vertices(moved)):
+        mine.copy_(new)
+    plan.launch()
+    (short,) = plan.bvhs()
+    assert short.info().quad_nodes == 0 and whole.info().quad_nodes > 0
+    rays = torch.from_numpy(S.random_rays(50_000, seed=9)).cuda()
+    want = whole.Intersect(A.Stats(), rays)
+    assert torch.equal(short.Intersect(A.Stats(), rays).raw, want.raw)
+    assert torch.equal(short.IntersectAny(A.Stats(), rays), want.prim >= 0)
+    short.check_errors()
